@@ -6,7 +6,8 @@
 //   lab    : uint8_t[N]      per-node labels (leaf labels + band-top labels), rewritten
 //                            every checkpoint (include/utils.hpp:51-57 Label values)
 //   push   : 2 bits per node region-root flags set by each node's parent: 1 first-occurrence
-//                            root, 2 shifted-duplicate root (16 nodes per 32-bit word)
+//                            root, 2 shifted-duplicate root (16 nodes per 32-bit word; node x at
+//                            position x + 1, so every level starts on its own power of two)
 //   map    : cap+1 keys (16 B) then cap+1 values (8 B): open-addressing digest -> NodeID
 //            table, 24 B per slot (map.cuh)
 #pragma once
@@ -78,6 +79,12 @@ __host__ __device__ __forceinline__ uint32_t leftmost_leaf(uint32_t node, uint32
   leaf_range(node, num_nodes, lo, hi);
   return lo;
 }
+// The same range in closed form for a node of a tree of depth D (leaf_range's loop restated;
+// node_span(x) == leaf_range(x) for every node of every tree).
+struct NodeSpan {
+  uint32_t first, count;
+};
+__host__ __device__ __forceinline__ NodeSpan node_span(uint32_t node, uint32_t num_nodes, uint32_t depth);
 // level of a heap index: floor(log2(i+1))
 __host__ __device__ __forceinline__ uint32_t node_level(uint32_t i) {
 #ifdef __CUDA_ARCH__
@@ -85,6 +92,17 @@ __host__ __device__ __forceinline__ uint32_t node_level(uint32_t i) {
 #else
   return 31u - (uint32_t)__builtin_clz(i + 1u);
 #endif
+}
+
+__host__ __device__ __forceinline__ NodeSpan node_span(uint32_t node, uint32_t num_nodes, uint32_t depth) {
+  const uint64_t y = (uint64_t)node + 1u, end = (uint64_t)num_nodes + 1u;   // y: 1-based heap position
+  const uint32_t k = depth - node_level(node);
+  const uint64_t lo = y << k;   // first descendant's position on the deepest level
+  if (lo < end) {
+    const uint64_t full = 1ull << k;
+    return NodeSpan{(uint32_t)(lo - 1u), (uint32_t)(full < end - lo ? full : end - lo)};
+  }
+  return NodeSpan{(uint32_t)((y << (k - 1u)) - 1u), 1u << (k - 1u)};   // only the level above has leaves of it
 }
 
 __host__ __device__ __forceinline__ uint64_t ceil_div_u64(uint64_t a, uint64_t b) { return (a + b - 1) / b; }

@@ -182,7 +182,6 @@ struct b2d_dedup {
   uint32_t map_grows = 0;
   uint64_t map_size_host = 0;     // occupied slots after the last checkpoint
   DevBuf<unsigned long long> map_size;
-  DevBuf<uint32_t> tmp_first, tmp_shift, levels;
   DevBuf<uint32_t> first_list, shift_list, region_off, sprev, skey, hist, bucket_start, partial, partial2;
   DevBuf<uint8_t> diff;
   DevBuf<DevState> state;
@@ -297,8 +296,7 @@ uint64_t buf_bytes(const DevBuf<T>& b) {
 uint64_t handle_bytes(const b2d_dedup* d) {
   return buf_bytes(d->tree) + buf_bytes(d->lab) + buf_bytes(d->leaflab) + buf_bytes(d->push) +
          buf_bytes(d->dupflag) + (d->map_mem ? (d->map_cap + 1) * MAP_SLOT_BYTES : 0) +
-         buf_bytes(d->map_size) + buf_bytes(d->tmp_first) +
-         buf_bytes(d->tmp_shift) + buf_bytes(d->levels) + buf_bytes(d->first_list) + buf_bytes(d->shift_list) +
+         buf_bytes(d->map_size) + buf_bytes(d->first_list) + buf_bytes(d->shift_list) +
          buf_bytes(d->region_off) + buf_bytes(d->sprev) + buf_bytes(d->skey) + buf_bytes(d->hist) +
          buf_bytes(d->bucket_start) + buf_bytes(d->partial) + buf_bytes(d->partial2) + buf_bytes(d->diff) +
          buf_bytes(d->state) + buf_bytes(d->r_node_list) + buf_bytes(d->r_rep) + buf_bytes(d->r_dist) +
@@ -471,23 +469,22 @@ int prepare_checkpoint(b2d_dedup* d, const void* d_data, uint64_t len, bool make
     int rc = map_ensure(d);
     if (rc) return rc;
   }
-  // bucket capacity grows in powers of two so a buffer's graph survives many checkpoints
+  // one bucket per checkpoint since the baseline (the map holds no older entries); the capacity
+  // grows in powers of two so a buffer's graph survives many checkpoints
+  const uint32_t buckets = d->current_id - d->baseline_id + 1u;
   uint32_t bcap = d->bcap ? d->bcap : 64u;
-  while (bcap < d->current_id + 1u) bcap <<= 1;
+  while (bcap < buckets) bcap <<= 1;
   if (bcap > MAX_BUCKETS) bcap = MAX_BUCKETS;
   d->bcap = bcap;
   B2D_CU(d->first_list.reserve(d->n));
   B2D_CU(d->shift_list.reserve(d->n));
-  B2D_CU(d->tmp_first.reserve(d->n));
-  B2D_CU(d->tmp_shift.reserve(d->n));
-  B2D_CU(d->levels.reserve(68));
   B2D_CU(d->region_off.reserve(d->n));
   B2D_CU(d->sprev.reserve(d->n));
   B2D_CU(d->skey.reserve(d->n));
   B2D_CU(d->hist.reserve(bcap));
   B2D_CU(d->bucket_start.reserve(bcap));
   B2D_CU(d->partial.reserve((size_t)1184 * bcap));
-  B2D_CU(d->partial2.reserve(2 * COMPACT_GRID));
+  B2D_CU(d->partial2.reserve(3 * COMPACT_GRID));
   B2D_CU(d->diff.reserve(64 + 16ull * d->n + (uint64_t)d->n * d->chunk_size));
   B2D_CU(d->state.reserve(1));
   B2D_CU(d->state_h.reserve(1));
@@ -498,7 +495,7 @@ int prepare_checkpoint(b2d_dedup* d, const void* d_data, uint64_t len, bool make
   // the list approach applies one per-chunk rule to every checkpoint (src/list_approach.cpp:41-71):
   // the incremental leaf rule against a list that a baseline has zeroed
   r->baseline = (baseline && !d->list) ? 1u : 0u;
-  r->buckets = d->current_id + 1u;
+  r->buckets = buckets;
   map_view(d, r->map);
   return B2D_OK;
 }
@@ -509,8 +506,7 @@ void graph_key(const b2d_dedup* d, const RoundState* rs_dev, std::vector<uint64_
   k.assign({(uint64_t)d->data, d->data_len, d->chunk_size, (uint64_t)d->kind, (uint64_t)d->tree.p,
             (uint64_t)d->lab.p, (uint64_t)d->leaflab.p, (uint64_t)d->push.p, (uint64_t)d->dupflag.p,
             (uint64_t)d->first_list.p,
-            (uint64_t)d->shift_list.p, (uint64_t)d->tmp_first.p, (uint64_t)d->tmp_shift.p, (uint64_t)d->levels.p,
-            (uint64_t)d->region_off.p, (uint64_t)d->sprev.p, (uint64_t)d->skey.p, (uint64_t)d->hist.p,
+            (uint64_t)d->shift_list.p, (uint64_t)d->region_off.p, (uint64_t)d->sprev.p, (uint64_t)d->skey.p, (uint64_t)d->hist.p,
             (uint64_t)d->bucket_start.p, (uint64_t)d->partial.p, (uint64_t)d->partial2.p, (uint64_t)d->diff.p,
             (uint64_t)d->state.p, (uint64_t)d->state_h.p, (uint64_t)d->round_h.p, (uint64_t)rs_dev, d->bcap,
             (uint64_t)d->tune.allow_tma, (uint64_t)d->tune.stages, (uint64_t)d->tune.ctas_per_sm, (uint64_t)d->graph_timing,
@@ -527,9 +523,9 @@ DiffArgs diff_args(b2d_dedup* d, const RoundState* rs_dev) {
   map_view(d, m);
   DevState* ds = d->state.p;
   return DiffArgs{static_cast<const uint8_t*>(d->data), d->data_len, d->chunk_size, d->n, d->N, d->D, 0, 0,
-                  d->tree.p, d->push.p, m, &ds->status, &ds->meta, d->first_list.p, d->shift_list.p, d->tmp_first.p,
-                  d->tmp_shift.p, d->levels.p, d->region_off.p, d->sprev.p, d->skey.p, d->hist.p, d->bucket_start.p,
-                  d->partial.p, d->partial2.p, d->diff.p, rs_dev, 0u};
+                  d->tree.p, d->push.p, m, &ds->status, &ds->meta, d->first_list.p, d->shift_list.p, d->region_off.p,
+                  d->sprev.p, d->skey.p, d->hist.p, d->bucket_start.p, d->partial.p, d->partial2.p, d->diff.p, rs_dev,
+                  d->list ? d->n - 1u : 0u, d->list};
 }
 
 ForestArgs forest_args(b2d_dedup* d, const RoundState* rs_dev) {
@@ -574,22 +570,19 @@ int enqueue_checkpoint(b2d_dedup* d, cudaStream_t s, RoundState* rs_dev, bool up
   // chunk order, chunk indices in the diff); a batch may assemble all its handles' diffs in
   // shared launches
   if (!skip_diff) {
-    DiffArgs da = diff_args(d, rs_dev);
-    if (d->list) da.id_bias = d->n - 1u;
-    B2D_CU(launch_collect_diff(da, d->bcap, d->sm_count, s, d->list != 0));
+    B2D_CU(launch_collect_diff(diff_args(d, rs_dev), d->bcap, d->sm_count, s));
   }
   if (timing) B2D_CU(record_timing(d->ev[2], s));
   if (!managed) B2D_CU(cudaMemcpyAsync(d->state_h.p, d->state.p, sizeof(DevState), cudaMemcpyDeviceToHost, s));
-  // kernels only (memsets and copies are not counted): the diff assembly is 12 kernels, 10 in
-  // node order (no level reordering)
+  // kernels only (memsets and copies are not counted)
   if (d->list)
-    d->launches = (skip_leaves ? 0 : 1) + 1 + (skip_diff ? 0 : 10);
+    d->launches = (skip_leaves ? 0 : 1) + 1 + (skip_diff ? 0 : DIFF_LAUNCHES);
   else
     d->launches = (skip_leaves ? 0 : 1) +
                   (skip_forest ? 0 : forest_launch_count(d->n, d->D, 1, d->warp_bands) +
                                          forest_launch_count(d->n, d->D, 2, d->warp_bands) +
                                          (zero_probe_skipped ? 0 : 1)) +
-                  (skip_diff ? 0 : 12);
+                  (skip_diff ? 0 : DIFF_LAUNCHES);
   return B2D_OK;
 }
 
@@ -1135,8 +1128,8 @@ struct BatchLayout {
          total = 0;
 };
 // u32 tables of the shared diff assembly, each n (+1) long, in this order in the blob
-enum DiffTable { DT_G, DT_GS, DT_BCAP, DT_ONE, DT_BEG_G, DT_BEG_GL, DT_BEG_GP, DT_BEG_GS, DT_BEG_GATHER, DT_COUNT };
-constexpr int DIFF_TABLES = DT_BEG_GATHER + GATHER_VARIANTS;
+enum DiffTable { DT_GS, DT_BCAP, DT_BEG_G, DT_BEG_GC, DT_BEG_EMIT };
+constexpr int DIFF_TABLES = DT_BEG_EMIT + GATHER_VARIANTS;
 
 }  // namespace
 
@@ -1371,56 +1364,41 @@ int batch_launch(b2d_batch* b, b2d_dedup* const* hs, const void* const* data, co
   if (seg_diff) {
     auto tab = [&](int t) { return reinterpret_cast<uint32_t*>(H + L.dtab) + (size_t)t * tab_len; };
     auto dtab = [&](int t) { return reinterpret_cast<const uint32_t*>(B + L.dtab) + (size_t)t * tab_len; };
-    uint32_t tot_g = 0, tot_gl = 0, tot_gp = 0, tot_gs = 0, tot_one = 0, tot_v[GATHER_VARIANTS] = {0};
-    uint32_t max_bcap = 1;
+    uint32_t tot_g = 0, tot_gc = 0, tot_v[GATHER_VARIANTS] = {0};
+    uint32_t max_bcap = 1, max_smem = 0;
     for (uint32_t i = 0; i < count; i++) {
       b2d_dedup* d = hs[i];
       const DiffArgs da = diff_args(d, &d->state.p->round);
       std::memcpy(H + L.dargs + sizeof(DiffArgs) * i, &da, sizeof(da));
-      DiffGrids dg = diff_grids(da, b->sm_count);
-      if (d->list) dg.g = dg.gl = dg.gp = dg.gs = dg.gg = 0;   // its own branch assembles its diff
-      tab(DT_G)[i] = dg.g;
+      DiffGrids dg = diff_grids(da, d->bcap, b->sm_count);
+      if (d->list) dg.g = dg.gs = dg.gc = dg.ge = 0;   // its own branch assembles its diff
       tab(DT_GS)[i] = dg.gs;
       tab(DT_BCAP)[i] = d->bcap;
       max_bcap = std::max(max_bcap, d->bcap);
-      tab(DT_ONE)[i] = tot_one;
-      tot_one += d->list ? 0u : 1u;
+      max_smem = std::max(max_smem, diff_emit_smem(d->bcap));
       tab(DT_BEG_G)[i] = tot_g;
       tot_g += dg.g;
-      tab(DT_BEG_GL)[i] = tot_gl;
-      tot_gl += dg.gl;
-      tab(DT_BEG_GP)[i] = tot_gp;
-      tot_gp += dg.gp;
-      tab(DT_BEG_GS)[i] = tot_gs;
-      tot_gs += dg.gs;
+      tab(DT_BEG_GC)[i] = tot_gc;
+      tot_gc += dg.gc;
       for (int v = 0; v < GATHER_VARIANTS; v++) {
-        tab(DT_BEG_GATHER + v)[i] = tot_v[v];
-        if (v == dg.variant) tot_v[v] += dg.gg;
+        tab(DT_BEG_EMIT + v)[i] = tot_v[v];
+        if (v == dg.variant) tot_v[v] += dg.ge;
       }
     }
-    tab(DT_ONE)[count] = tot_one;
     tab(DT_BEG_G)[count] = tot_g;
-    tab(DT_BEG_GL)[count] = tot_gl;
-    tab(DT_BEG_GP)[count] = tot_gp;
-    tab(DT_BEG_GS)[count] = tot_gs;
-    for (int v = 0; v < GATHER_VARIANTS; v++) tab(DT_BEG_GATHER + v)[count] = tot_v[v];
-    dplan.base = SegGrid{reinterpret_cast<const DiffArgs*>(B + L.dargs), nullptr, dtab(DT_G), dtab(DT_GS),
-                         dtab(DT_BCAP), count};
-    dplan.beg_one = dtab(DT_ONE);
+    tab(DT_BEG_GC)[count] = tot_gc;
+    for (int v = 0; v < GATHER_VARIANTS; v++) tab(DT_BEG_EMIT + v)[count] = tot_v[v];
+    dplan.base = SegGrid{reinterpret_cast<const DiffArgs*>(B + L.dargs), nullptr, dtab(DT_GS), dtab(DT_BCAP), count};
     dplan.beg_g = dtab(DT_BEG_G);
-    dplan.beg_gl = dtab(DT_BEG_GL);
-    dplan.beg_gp = dtab(DT_BEG_GP);
-    dplan.beg_gs = dtab(DT_BEG_GS);
+    dplan.beg_gc = dtab(DT_BEG_GC);
     for (int v = 0; v < GATHER_VARIANTS; v++) {
-      dplan.beg_gather[v] = dtab(DT_BEG_GATHER + v);
-      dplan.tot_gather[v] = tot_v[v];
+      dplan.beg_emit[v] = dtab(DT_BEG_EMIT + v);
+      dplan.tot_emit[v] = tot_v[v];
     }
-    dplan.tot_one = tot_one;
     dplan.tot_g = tot_g;
-    dplan.tot_gl = tot_gl;
-    dplan.tot_gp = tot_gp;
-    dplan.tot_gs = tot_gs;
+    dplan.tot_gc = tot_gc;
     dplan.max_bcap = max_bcap;
+    dplan.max_emit_smem = max_smem;
   }
   // shared forest phases: ForestArgs and per-launch tables
   std::vector<ForestSeg> fseg(flaunch.size());
@@ -2057,8 +2035,8 @@ int b2d_estimate_memory(uint64_t len, uint32_t chunk_size, int map_max_load_pct,
   const uint64_t cap = map_capacity(2 * N, map_max_load_pct / 100.0, MAP_HEADROOM);
   uint64_t b = N * sizeof(Digest) + N + (n + 16) + ((N + 63) / 64 * 16 + 16) + n;   // tree, labels, flags
   b += (cap + 1) * MAP_SLOT_BYTES + 8;                                               // map
-  b += 8 * 4 * n + 68 * 4;                                                           // lists and keys
-  b += (uint64_t)64 * 4 * 2 + (uint64_t)1184 * 64 * 4 + 2 * COMPACT_GRID * 4;           // buckets, partials
+  b += 5 * 4 * n;                                                                    // lists and keys
+  b += (uint64_t)64 * 4 * 2 + (uint64_t)1184 * 64 * 4 + 3 * COMPACT_GRID * 4;           // buckets, partials
   b += 64 + 16 * n + n * chunk_size;                                                 // diff
   b += sizeof(DevState);
   *bytes = b;

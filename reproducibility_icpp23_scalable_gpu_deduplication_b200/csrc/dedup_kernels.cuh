@@ -28,7 +28,7 @@ struct RoundState {
   uint32_t cur;          // current_id
   uint32_t baseline_id;  // ref_id written into the header
   uint32_t baseline;     // 1: baseline checkpoint
-  uint32_t buckets;      // cur + 1: source-checkpoint buckets of the shift entries
+  uint32_t buckets;      // cur - baseline_id + 1: source-checkpoint buckets of the shift entries
   MapView map;           // the digest map (moves when it grows; graphs read it here)
 };
 
@@ -77,6 +77,8 @@ struct DevMeta {
   unsigned long long diff_len;      // bytes of the diff (header included)
   unsigned long long first_off, count_off, shift_off, data_off;  // byte offsets in the device diff buffer
   unsigned long long map_size;      // occupied map slots after this checkpoint
+  uint32_t done;         // CTAs of the shifted-root pass that have finished (the last lays the diff out)
+  uint32_t pad;
 };
 
 struct DiffArgs {
@@ -90,20 +92,19 @@ struct DiffArgs {
   DevMeta* meta;
   uint32_t* first_list;   // F node ids, canonical order
   uint32_t* shift_list;   // S node ids, canonical order
-  uint32_t* tmp_first;    // F node ids, node order
-  uint32_t* tmp_shift;    // S node ids, node order
-  uint32_t* levels;       // 2 x 34 level-run starts of the node-order lists
-  uint32_t* region_off;   // F exclusive chunk offsets, then T
+  uint32_t* region_off;   // F exclusive chunk offsets
   uint32_t* sprev;        // S source node ids
-  uint32_t* skey;         // S source checkpoint ids
-  uint32_t* hist;         // cur+1 per-checkpoint counts
-  uint32_t* bucket_start; // cur+1 exclusive offsets
-  uint32_t* partial;      // SCAN_GRID * max(2, cur+1) scratch
-  uint32_t* partial2;     // COMPACT_GRID * 2 scratch
+  uint32_t* skey;         // S source checkpoint ids, relative to baseline_id
+  uint32_t* hist;         // per-checkpoint counts (buckets)
+  uint32_t* bucket_start; // exclusive offsets (buckets)
+  uint32_t* partial;      // per-range counts, then positions, of each bucket
+  uint32_t* partial2;     // COMPACT_GRID * 3 scratch
   uint8_t* diff;          // device diff buffer
   const RoundState* rs;
   uint32_t id_bias;       // subtracted from every node id written into the diff (list approach:
                           // n - 1, so leaf heap indices become chunk indices; tree: 0)
+  int node_order;         // region lists in node order (the list approach, whose regions are single
+                          // leaves) instead of the tree's level-descending order
 };
 
 // Programmatic dependent launch (sm_90 and later).  The forest and diff-assembly kernels of one
@@ -228,10 +229,8 @@ cudaError_t launch_zero_exists_seg(const ForestArgs* args, uint32_t n, cudaStrea
 int forest_launch_count(uint32_t n, uint32_t D, int phase, int warp_mask = B2D_WARP_BANDS);
 cudaError_t launch_zero_exists(int* flag, const RoundState* rs, cudaStream_t stream);
 // bcap: bucket capacity the scratch was sized for (>= rs->buckets of every checkpoint run).
-// node_order: the region lists stay in node order (the list approach's order, whose regions
-// are single leaves) instead of the tree's level-descending order.
-cudaError_t launch_collect_diff(const DiffArgs& a, uint32_t bcap, int sm_count, cudaStream_t stream,
-                                bool node_order = false);
+cudaError_t launch_collect_diff(const DiffArgs& a, uint32_t bcap, int sm_count, cudaStream_t stream);
+constexpr int DIFF_LAUNCHES = 4;   // kernels of one launch_collect_diff
 // the list approach's labels: the lowest-index owner of a digest shared by several changed
 // chunks stays the first occurrence, the others become shifted duplicates; region flags are
 // set for both (src/list_approach.cpp:41-71)
@@ -243,32 +242,28 @@ cudaError_t launch_list_label(const ForestArgs& a, int sm_count, cudaStream_t st
 struct SegGrid {
   const DiffArgs* args;   // per handle
   const uint32_t* beg;    // n + 1 CTA offsets of the launch
-  const uint32_t* g;      // per handle: CTAs of its compaction and region launches
-  const uint32_t* gs;     // per handle: CTAs of its shift-entry launches
+  const uint32_t* gs;     // per handle: ranges of its shifted entries
   const uint32_t* bcap;   // per handle: bucket capacity of its scratch
   uint32_t n;
 };
-// grid sizes of one handle's diff assembly; variant = data-gather kernel (0: 16-byte
-// copies, 1: byte copies)
+// grid sizes of one handle's diff assembly (count and write passes, ranges of the shifted-root
+// pass and its CTAs with the first-root checks, emit pass); variant = emit kernel (0: 16-byte aligned sources, 1: any)
 struct DiffGrids {
-  uint32_t g, gs, gl, gp, gg;
+  uint32_t g, gs, gc, ge;
   int variant;
 };
 constexpr int GATHER_VARIANTS = 2;
-DiffGrids diff_grids(const DiffArgs& a, int sm_count);
+DiffGrids diff_grids(const DiffArgs& a, uint32_t bcap, int sm_count);
+uint32_t diff_emit_smem(uint32_t bcap);   // dynamic shared memory of the emit pass
 struct DiffBatch {
   SegGrid base;                     // beg unused
-  const uint32_t* beg_one;          // one CTA per handle that takes part (prefix table)
   const uint32_t* beg_g;
-  const uint32_t* beg_gl;
-  const uint32_t* beg_gp;
-  const uint32_t* beg_gs;
-  const uint32_t* beg_gather[GATHER_VARIANTS];
-  uint32_t tot_one;                 // handles with one CTA in the scan and layout launches
-  uint32_t tot_g, tot_gl, tot_gp, tot_gs, tot_gather[GATHER_VARIANTS];
-  uint32_t max_bcap;
+  const uint32_t* beg_gc;
+  const uint32_t* beg_emit[GATHER_VARIANTS];
+  uint32_t tot_g, tot_gc, tot_emit[GATHER_VARIANTS];
+  uint32_t max_bcap, max_emit_smem;
 };
-// launches (count returned in *launches); the handles' hist arrays are cleared here
+// launches (count returned in *launches)
 cudaError_t launch_collect_diff_batch(const DiffBatch& b, cudaStream_t stream, uint32_t* launches);
 
 }  // namespace b2d

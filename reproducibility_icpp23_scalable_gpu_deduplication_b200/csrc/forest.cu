@@ -51,9 +51,11 @@ constexpr uint8_t NONE_LABEL = 5;         // node index beyond the tree
 __device__ __forceinline__ uint8_t push_flag(uint8_t label) {
   return label == SHIFT_DUPL ? PUSH_SHIFT : (label == FIRST_OCUR ? PUSH_FIRST : PUSH_NONE);
 }
-// region-root flag of node x: 2 bits per node, 16 nodes per word (gather.cu reads them)
+// region-root flag of node x, at position x + 1: 2 bits per node, 16 nodes per word (gather.cu
+// reads them)
 __device__ __forceinline__ void push_set(uint8_t* push, uint64_t x, uint32_t flag) {
-  atomicOr(reinterpret_cast<uint32_t*>(push) + (x >> 4), flag << (2u * (uint32_t)(x & 15u)));
+  const uint64_t y = x + 1u;
+  atomicOr(reinterpret_cast<uint32_t*>(push) + (y >> 4), flag << (2u * (uint32_t)(y & 15u)));
 }
 
 // phase-1 parent insert, priority 1 + height (:133, :390).  The rare heavy paths (hashing,

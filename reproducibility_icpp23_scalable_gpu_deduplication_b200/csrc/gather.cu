@@ -3,12 +3,14 @@
 // Output order is the reference's sequential order (what its atomics produce with one
 // thread): region roots by (level descending, node ascending); the repeat table by
 // checkpoint id; shifted-duplicate entries stably bucketed by source checkpoint.
-//   1. compaction of the push flags in that canonical order (reduce-then-scan, 3 launches)
-//   2. first-occurrence region sizes -> exclusive chunk offsets (3 launches)
-//   3. shift entries: source NodeID lookup + per-CTA histograms (1 launch)
-//   4. layout: bucket starts, repeat table, header, byte offsets (1 launch, 1 CTA)
-//   5. stable bucket scatter of the shift entries (1 launch, one warp per range)
-//   6. first-occurrence metadata + 16-byte vectorised chunk gather (1 launch)
+//   1. diff_count  per CTA: region roots of each kind and the chunks under the first ones
+//   2. diff_write  the root lists in that order, with each first region's chunk offset
+//   3. diff_shift  source NodeID of every shifted root, per-range counts by source checkpoint;
+//                  the last CTA to finish lays the diff out (bucket starts, repeat table, header)
+//   4. diff_emit   stable bucket scatter of the shifted entries, the first-occurrence list and
+//                  the 16-byte vectorised data gather, side by side
+// Four launches: a checkpoint of a few MiB is bound by the chain of dependent launches, not by
+// their work (twelve launches took 36 us of a 1 MiB checkpoint's 130 us).
 // Diff layout (include/utils.hpp:29-37, src/tree_approach.cpp:777-780):
 //   [header 32 B][u32 first node x F][(u32 ckpt, u32 count) x P][(u32 node, u32 prev) x S][data]
 // It is placed `delta` bytes into the device buffer so the data section is 16-byte aligned.
@@ -33,129 +35,241 @@ __device__ __forceinline__ uint32_t seg_locate(const SegGrid& s, uint32_t& bid, 
   nb = s.beg[lo + 1] - s.beg[lo];
   return lo;
 }
-constexpr uint32_t SHIFT_GRID = 296;    // at most 2 x 148 ranges for the shift-entry passes
+constexpr uint32_t SHIFT_GRID = 296;    // at most 2 x 148 ranges for the shifted-entry passes
+constexpr uint32_t SHIFT_THREADS = 256;
+constexpr uint32_t EMIT_THREADS = 256;
 
 // Region roots are flagged in `push`: 2 bits per node (PUSH_FIRST = 1, PUSH_SHIFT = 2), 16 nodes
-// per 32-bit word, zero-padded to a multiple of 64 nodes, all-zero between checkpoints (a quarter
-// of the bytes of one flag byte per node, so the two passes below read 16 MB instead of 64 MB
-// for a 2^26-node tree).  Compaction runs in node order with 16-byte loads of 64 nodes; since the
-// canonical order is "level descending, node ascending" and node order is "level ascending,
-// node ascending", the canonical list is the node-order list with its per-level runs reversed,
-// which compact_permute_kernel applies after a per-level split of the node-order lists.
+// per 32-bit word, zero-padded to a multiple of 64 nodes, all-zero between checkpoints.  Node x
+// sits at position y = x + 1, so level L occupies [2^L, 2^(L+1)) and every 16-byte group of 64
+// flags from the second on lies within one level: walking the groups level by level from the
+// deepest, each level ascending, then the six levels of the first group, meets the roots in the
+// canonical order.  List diffs keep node order (their roots are single leaves), so their walk is
+// plainly ascending from the first leaf's group.
 constexpr uint32_t PUSH_GROUP = 64;   // nodes per 16-byte load
 __device__ __forceinline__ uint4 ld_push16(const uint8_t* push, uint64_t g) {
   return reinterpret_cast<const uint4*>(push)[g];
 }
+struct GroupWalk {
+  uint32_t total;   // groups walked
+  uint32_t first;   // node order: the first group; canonical order: 2^(level of the deepest group)
+  uint32_t deep;    // canonical order: groups of the deepest level
+  bool node_order;
+};
+__device__ __forceinline__ GroupWalk group_walk(const DiffArgs& a) {
+  GroupWalk w;
+  const uint32_t groups = (uint32_t)(((uint64_t)a.N >> 6) + 1u);   // positions 1 .. N
+  w.node_order = a.node_order != 0;
+  if (w.node_order) {
+    w.first = a.n >> 6;   // position of chunk 0's leaf: n
+    w.total = groups - w.first;
+    w.deep = 0;
+  } else {
+    w.total = groups;
+    w.first = groups > 1u ? 1u << (31u - __clz(groups - 1u)) : 0u;
+    w.deep = groups > 1u ? groups - w.first : 0u;
+  }
+  return w;
+}
+// group at step p of the walk
+__device__ __forceinline__ uint32_t walk_group(const GroupWalk& w, uint32_t p) {
+  if (w.node_order || p < w.deep) return w.first + p;
+  const uint32_t t = w.first - (p - w.deep);   // 2^L .. 1 over the levels above the deepest
+  if (t < 2u) return 0u;
+  return 3u * (1u << (31u - __clz(t - 1u))) - t;
+}
 // one bit (the low bit of each 2-bit field) per node flagged first / shifted
 __device__ __forceinline__ uint32_t push_first_bits(uint32_t w) { return w & ~(w >> 1) & 0x55555555u; }
 __device__ __forceinline__ uint32_t push_shift_bits(uint32_t w) { return (w >> 1) & ~w & 0x55555555u; }
-__device__ __forceinline__ void count64(uint4 v, uint32_t& cf, uint32_t& cs) {
-  cf += __popc(push_first_bits(v.x)) + __popc(push_first_bits(v.y)) + __popc(push_first_bits(v.z)) +
-        __popc(push_first_bits(v.w));
-  cs += __popc(push_shift_bits(v.x)) + __popc(push_shift_bits(v.y)) + __popc(push_shift_bits(v.z)) +
-        __popc(push_shift_bits(v.w));
+__device__ __forceinline__ uint32_t first_count(const uint4& v) {
+  return __popc(push_first_bits(v.x)) + __popc(push_first_bits(v.y)) + __popc(push_first_bits(v.z)) +
+         __popc(push_first_bits(v.w));
+}
+__device__ __forceinline__ uint32_t shift_count(const uint4& v) {
+  return __popc(push_shift_bits(v.x)) + __popc(push_shift_bits(v.y)) + __popc(push_shift_bits(v.z)) +
+         __popc(push_shift_bits(v.w));
+}
+// chunks under the first-occurrence roots of a group
+__device__ __forceinline__ uint32_t group_chunks(const DiffArgs& a, uint32_t g, const uint4& v, uint32_t cf) {
+  if (cf == 0) return 0u;
+  if (g > 0) {   // one level: full subtrees all hold 2^k chunks
+    const uint32_t k = a.D - (31u - __clz(g)) - 6u;
+    if ((((uint64_t)g + 1u) << (6u + k)) <= (uint64_t)a.N + 1u) return cf << k;
+  }
+  uint32_t c = 0;
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    for (uint32_t m = push_first_bits(w[k]); m; m &= m - 1u)
+      c += node_span(PUSH_GROUP * g + 16u * k + ((__ffs(m) - 1u) >> 1) - 1u, a.N, a.D).count;
+  return c;
 }
 
-__device__ __forceinline__ void compact_count_body(const DiffArgs& a, uint32_t bid, uint32_t nb) {
+__device__ __forceinline__ void diff_count_body(const DiffArgs& a, uint32_t bid, uint32_t nb, uint32_t bcap) {
   __shared__ uint32_t sh[COMPACT_THREADS / 32 + 1];
-  const uint64_t groups = ((uint64_t)a.N + PUSH_GROUP - 1u) / PUSH_GROUP;
+  const GroupWalk w = group_walk(a);
   uint64_t beg, end;
-  cta_range(groups, bid, nb, beg, end);
-  uint32_t cf = 0, cs = 0;
+  cta_range(w.total, bid, nb, beg, end);
+  uint32_t cf = 0, cs = 0, ct = 0;
   // two independent loads per thread per iteration
-  for (uint64_t g = beg + threadIdx.x; g < end; g += 2ull * blockDim.x) {
-    const uint4 v0 = ld_push16(a.push, g);
-    const uint4 v1 = g + blockDim.x < end ? ld_push16(a.push, g + blockDim.x) : make_uint4(0, 0, 0, 0);
-    if (v0.x | v0.y | v0.z | v0.w) count64(v0, cf, cs);
-    if (v1.x | v1.y | v1.z | v1.w) count64(v1, cf, cs);
+  for (uint64_t p = beg + threadIdx.x; p < end; p += 2ull * blockDim.x) {
+    const uint32_t g0 = walk_group(w, (uint32_t)p);
+    const bool two = p + blockDim.x < end;
+    const uint32_t g1 = two ? walk_group(w, (uint32_t)p + blockDim.x) : g0;
+    const uint4 v0 = ld_push16(a.push, g0);
+    const uint4 v1 = two ? ld_push16(a.push, g1) : make_uint4(0, 0, 0, 0);
+    if (v0.x | v0.y | v0.z | v0.w) {
+      const uint32_t f = first_count(v0);
+      cf += f;
+      cs += shift_count(v0);
+      ct += group_chunks(a, g0, v0, f);
+    }
+    if (v1.x | v1.y | v1.z | v1.w) {
+      const uint32_t f = first_count(v1);
+      cf += f;
+      cs += shift_count(v1);
+      ct += group_chunks(a, g1, v1, f);
+    }
   }
   const uint32_t tf = block_reduce_sum(cf, sh);
   const uint32_t ts = block_reduce_sum(cs, sh);
+  const uint32_t tt = block_reduce_sum(ct, sh);
   if (threadIdx.x == 0) {
-    a.partial2[2 * bid] = tf;
-    a.partial2[2 * bid + 1] = ts;
+    a.partial2[3 * bid] = tf;
+    a.partial2[3 * bid + 1] = ts;
+    a.partial2[3 * bid + 2] = tt;
   }
-}
-__global__ void __launch_bounds__(COMPACT_THREADS) compact_count_kernel(DiffArgs a0) {
-  griddep_enter();
-  compact_count_body(with_round(a0), blockIdx.x, gridDim.x);
-}
-__global__ void __launch_bounds__(COMPACT_THREADS) compact_count_seg(SegGrid s) {
-  uint32_t bid, nb;
-  const uint32_t h = seg_locate(s, bid, nb);
-  compact_count_body(with_round(s.args[h]), bid, nb);
-}
-
-__device__ __forceinline__ void compact_scan_body(const DiffArgs& a, uint32_t bid, uint32_t nb, uint32_t g) {
-  __shared__ uint32_t sh[33];
-  uint32_t tf, ts;
-  const uint32_t i = threadIdx.x;
-  const uint32_t vf = i < g ? a.partial2[2 * i] : 0u, vs = i < g ? a.partial2[2 * i + 1] : 0u;
-  const uint32_t ef = block_excl_scan(vf, sh, &tf);
-  const uint32_t es = block_excl_scan(vs, sh, &ts);
-  if (i < g) {
-    a.partial2[2 * i] = ef;
-    a.partial2[2 * i + 1] = es;
-  }
-  if (i == 0) {
-    a.meta->F = tf;
-    a.meta->S = ts;
-  }
-}
-__global__ void __launch_bounds__(1024) compact_scan_kernel(DiffArgs a0, uint32_t g, uint32_t bcap) {
-  griddep_enter();
-  compact_scan_body(with_round(a0), blockIdx.x, gridDim.x, g);
   // the per-checkpoint bucket counts start at zero
-  for (uint32_t t = threadIdx.x; t < bcap; t += blockDim.x) a0.hist[t] = 0u;
+  if (bid == 0)
+    for (uint32_t t = threadIdx.x; t < bcap; t += blockDim.x) a.hist[t] = 0u;
 }
-__global__ void __launch_bounds__(1024) compact_scan_seg(SegGrid s) {
+__global__ void __launch_bounds__(COMPACT_THREADS) diff_count_kernel(DiffArgs a0, uint32_t bcap) {
+  griddep_enter();
+  diff_count_body(with_round(a0), blockIdx.x, gridDim.x, bcap);
+}
+__global__ void __launch_bounds__(COMPACT_THREADS) diff_count_seg(SegGrid s) {
   uint32_t bid, nb;
   const uint32_t h = seg_locate(s, bid, nb);
-  compact_scan_body(with_round(s.args[h]), bid, nb, s.g[h]);
-  // the per-checkpoint bucket counts start at zero (the single-handle path memsets them)
-  for (uint32_t t = threadIdx.x; t < s.bcap[h]; t += blockDim.x) s.args[h].hist[t] = 0u;
+  diff_count_body(with_round(s.args[h]), bid, nb, s.bcap[h]);
 }
 
-// node-order lists of first / shift roots; clears the flags it consumed.  Each thread owns one
-// 64-node group of a tile, so one block scan covers COMPACT_THREADS * 64 = 32768 nodes, which
-// keeps both 16-bit halves of the packed counts exact.
-__device__ __forceinline__ void compact_write_body(const DiffArgs& a, uint32_t bid, uint32_t nb) {
+// Lists of first / shifted roots and the first regions' chunk offsets; clears the flags it
+// consumed.  Each CTA adds up the counts of the CTAs before it.  Each thread owns one 64-node
+// group of a tile, so one block scan covers COMPACT_THREADS * 64 = 32768 nodes, which keeps both
+// 16-bit halves of the packed counts exact.
+__device__ __forceinline__ void diff_write_body(const DiffArgs& a, uint32_t bid, uint32_t nb) {
   __shared__ uint32_t sh[COMPACT_THREADS / 32 + 1];
-  const uint64_t groups = ((uint64_t)a.N + PUSH_GROUP - 1u) / PUSH_GROUP;
+  const GroupWalk w = group_walk(a);
   uint64_t beg, end;
-  cta_range(groups, bid, nb, beg, end);
-  uint32_t bf = a.partial2[2 * bid], bs = a.partial2[2 * bid + 1];
+  cta_range(w.total, bid, nb, beg, end);
+  uint32_t bf = 0, bs = 0, bt = 0;
+  for (uint32_t i = threadIdx.x; i < bid; i += blockDim.x) {
+    bf += a.partial2[3 * i];
+    bs += a.partial2[3 * i + 1];
+    bt += a.partial2[3 * i + 2];
+  }
+  bf = block_reduce_sum(bf, sh);
+  bs = block_reduce_sum(bs, sh);
+  bt = block_reduce_sum(bt, sh);
+  if (bid == nb - 1u && threadIdx.x == 0) {
+    a.meta->F = bf + a.partial2[3 * bid];
+    a.meta->S = bs + a.partial2[3 * bid + 1];
+    a.meta->T = bt + a.partial2[3 * bid + 2];
+  }
   for (uint64_t t0 = beg; t0 < end; t0 += COMPACT_THREADS) {
-    const uint64_t g = t0 + threadIdx.x;
-    const uint4 v = g < end ? ld_push16(a.push, g) : make_uint4(0, 0, 0, 0);
+    const uint64_t p = t0 + threadIdx.x;
+    const uint32_t g = p < end ? walk_group(w, (uint32_t)p) : 0u;
+    const uint4 v = p < end ? ld_push16(a.push, g) : make_uint4(0, 0, 0, 0);
     const bool nz = (v.x | v.y | v.z | v.w) != 0u;
-    uint32_t cf = 0, cs = 0;
-    if (nz) count64(v, cf, cs);
-    uint32_t tot;
-    const uint32_t ex = block_excl_scan((cf << 16) | cs, sh, &tot);
+    uint32_t cf = 0, cs = 0, ct = 0;
     if (nz) {
-      uint32_t of = bf + (ex >> 16), os = bs + (ex & 0xffffu);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      cf = first_count(v);
+      cs = shift_count(v);
+      ct = group_chunks(a, g, v, cf);
+    }
+    if (!__syncthreads_or(nz)) continue;
+    uint32_t tot, tott;
+    const uint32_t ex = block_excl_scan((cf << 16) | cs, sh, &tot);
+    const uint32_t et = block_excl_scan(ct, sh, &tott);
+    // Groups with many roots of one level over full subtrees (runs of list chunks above all) are
+    // written by the whole warp, two nodes per lane, so stores cover whole sectors.
+    const uint32_t height = g > 0 ? a.D - (31u - __clz(g)) - 6u : 0u;
+    const bool dense = cf + cs >= 8u && g > 0 &&
+                       (w.node_order || (((uint64_t)g + 1u) << (6u + height)) <= (uint64_t)a.N + 1u);
+    for (uint32_t todo = __ballot_sync(0xffffffffu, dense); todo; todo &= todo - 1u) {
+      const uint32_t l = __ffs(todo) - 1u, lane = threadIdx.x & 31u;
+      const uint32_t ws[4] = {__shfl_sync(0xffffffffu, v.x, l), __shfl_sync(0xffffffffu, v.y, l),
+                              __shfl_sync(0xffffffffu, v.z, l), __shfl_sync(0xffffffffu, v.w, l)};
+      const uint32_t k = w.node_order ? 0u : __shfl_sync(0xffffffffu, height, l);
+      uint32_t of = bf + __shfl_sync(0xffffffffu, ex >> 16, l), os = bs + __shfl_sync(0xffffffffu, ex & 0xffffu, l);
+      uint32_t x = PUSH_GROUP * __shfl_sync(0xffffffffu, g, l) + 2u * lane - 1u;
+      const uint32_t ot = bt + __shfl_sync(0xffffffffu, et, l);
+      const uint32_t mine = lane >> 3, below = (1u << (4u * (lane & 7u))) - 1u;
+      uint32_t pf = 0, word = ws[0];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const uint32_t base = (uint32_t)(PUSH_GROUP * g) + 16u * k;
-        for (uint32_t m = push_first_bits(w[k]); m; m &= m - 1u) a.tmp_first[of++] = base + ((__ffs(m) - 1u) >> 1);
-        for (uint32_t m = push_shift_bits(w[k]); m; m &= m - 1u) a.tmp_shift[os++] = base + ((__ffs(m) - 1u) >> 1);
+      for (uint32_t q = 0; q < 4; q++) {
+        if (q == mine) word = ws[q];
+        const uint32_t m = q < mine ? ~0u : q == mine ? below : 0u;
+        pf += __popc(push_first_bits(ws[q]) & m);
+        os += __popc(push_shift_bits(ws[q]) & m);
+      }
+      of += pf;
+      uint32_t o = ot + (pf << k);
+#pragma unroll
+      for (uint32_t q = 0; q < 2; q++, x++) {
+        const uint32_t flag = word >> (4u * (lane & 7u) + 2u * q) & 3u;
+        if (flag == PUSH_FIRST) {
+          a.first_list[of] = x;
+          a.region_off[of] = o;
+          of++;
+          o += 1u << k;
+        } else if (flag == PUSH_SHIFT) {
+          a.shift_list[os++] = x;
+        }
+      }
+    }
+    if (dense) {
+      reinterpret_cast<uint4*>(a.push)[g] = make_uint4(0, 0, 0, 0);
+    } else if (nz) {
+      uint32_t of = bf + (ex >> 16), os = bs + (ex & 0xffffu), ot = bt + et;
+      auto emit = [&](uint32_t word, uint32_t base) {   // the roots of one 16-flag word, ascending
+        for (uint32_t m = push_first_bits(word); m; m &= m - 1u) {
+          const uint32_t x = base + ((__ffs(m) - 1u) >> 1);
+          a.first_list[of] = x;
+          a.region_off[of] = ot;
+          ot += node_span(x, a.N, a.D).count;
+          of++;
+        }
+        for (uint32_t m = push_shift_bits(word); m; m &= m - 1u) a.shift_list[os++] = base + ((__ffs(m) - 1u) >> 1);
+      };
+      const uint32_t ws[4] = {v.x, v.y, v.z, v.w};
+      if (g > 0 || w.node_order) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) emit(ws[k], PUSH_GROUP * g + 16u * k - 1u);
+      } else {   // positions 1 .. 63: levels 5 .. 0, each ascending
+        emit(ws[2], 31u);
+        emit(ws[3], 47u);
+        emit(ws[1], 15u);
+        emit(ws[0] & 0xffff0000u, ~0u);
+        emit(ws[0] & 0x0000ff00u, ~0u);
+        emit(ws[0] & 0x000000f0u, ~0u);
+        emit(ws[0] & 0x0000000cu, ~0u);
       }
       reinterpret_cast<uint4*>(a.push)[g] = make_uint4(0, 0, 0, 0);
     }
     bf += tot >> 16;
     bs += tot & 0xffffu;
+    bt += tott;
   }
 }
-__global__ void __launch_bounds__(COMPACT_THREADS) compact_write_kernel(DiffArgs a0) {
+__global__ void __launch_bounds__(COMPACT_THREADS) diff_write_kernel(DiffArgs a0) {
   griddep_enter();
-  compact_write_body(with_round(a0), blockIdx.x, gridDim.x);
+  diff_write_body(with_round(a0), blockIdx.x, gridDim.x);
 }
-__global__ void __launch_bounds__(COMPACT_THREADS) compact_write_seg(SegGrid s) {
+__global__ void __launch_bounds__(COMPACT_THREADS) diff_write_seg(SegGrid s) {
   uint32_t bid, nb;
   const uint32_t h = seg_locate(s, bid, nb);
-  compact_write_body(with_round(s.args[h]), bid, nb);
+  diff_write_body(with_round(s.args[h]), bid, nb);
 }
 
 // warp-parallel lower bound: first index of sorted v[0..cnt) with v[idx] >= key (32-ary search)
@@ -176,176 +290,17 @@ __device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t* v, uint32_t
   return lo + __popc(__ballot_sync(0xffffffffu, below));
 }
 
-// level runs of the node-order lists: levels[L] = start of level L in tmp_first,
-// levels[34 + L] in tmp_shift (L = 0..D+1); one warp per search
-__device__ __forceinline__ void compact_levels_body(const DiffArgs& a, uint32_t bid, uint32_t nb) {
-  const uint32_t gw = (bid * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t L = gw >> 1;
-  if (L > a.D + 1u) return;
-  const uint64_t key = (1ull << L) - 1ull;   // first node of level L
-  if ((gw & 1u) == 0) {
-    const uint32_t r = warp_lower_bound(a.tmp_first, a.meta->F, key);
-    if ((threadIdx.x & 31u) == 0) a.levels[L] = r;
-  } else {
-    const uint32_t r = warp_lower_bound(a.tmp_shift, a.meta->S, key);
-    if ((threadIdx.x & 31u) == 0) a.levels[34 + L] = r;
-  }
-}
-__global__ void compact_levels_kernel(DiffArgs a0) {
-  griddep_enter();
-  compact_levels_body(with_round(a0), blockIdx.x, gridDim.x);
-}
-__global__ void compact_levels_seg(SegGrid s) {
-  uint32_t bid, nb;
-  const uint32_t h = seg_locate(s, bid, nb);
-  compact_levels_body(with_round(s.args[h]), bid, nb);
+// ---------------------------------------------------------------- shifted duplicates, layout
+// Source checkpoints are counted in buckets relative to the last baseline, which emptied the
+// map: no entry is older, and a handle that has taken thousands of checkpoints sorts its entries
+// into as many buckets as its chain is long.
+__device__ __forceinline__ uint32_t bucket_count(const DiffArgs& a, uint32_t bcap) {
+  return a.rs->buckets <= bcap ? a.rs->buckets : bcap;
 }
 
-// canonical position of node-order entry i at level L: entries of deeper levels first
-__device__ __forceinline__ void compact_permute_body(const DiffArgs& a, uint32_t bid, uint32_t nb) {
-  const uint32_t F = a.meta->F, S = a.meta->S;
-  const uint64_t tot = (uint64_t)F + S;
-  for (uint64_t i = bid * (uint64_t)blockDim.x + threadIdx.x; i < tot; i += (uint64_t)nb * blockDim.x) {
-    const bool isf = i < F;
-    const uint32_t j = isf ? (uint32_t)i : (uint32_t)(i - F);
-    const uint32_t* lv = a.levels + (isf ? 0 : 34);
-    const uint32_t cnt = isf ? F : S;
-    const uint32_t node = isf ? a.tmp_first[j] : a.tmp_shift[j];
-    const uint32_t L = node_level(node);
-    // entries at levels deeper than L come first: cnt - (start of level L+1)
-    const uint32_t pos = (cnt - lv[L + 1]) + (j - lv[L]);
-    if (isf) a.first_list[pos] = node;
-    else a.shift_list[pos] = node;
-  }
-}
-__global__ void compact_permute_kernel(DiffArgs a0) {
-  griddep_enter();
-  compact_permute_body(with_round(a0), blockIdx.x, gridDim.x);
-}
-__global__ void compact_permute_seg(SegGrid s) {
-  uint32_t bid, nb;
-  const uint32_t h = seg_locate(s, bid, nb);
-  compact_permute_body(with_round(s.args[h]), bid, nb);
-}
-
-// ---------------------------------------------------------------- region sizes and offsets
-__device__ __forceinline__ void region_count_body(const DiffArgs& a, uint32_t bid, uint32_t nb) {
-  __shared__ uint32_t sh[COMPACT_THREADS / 32 + 1];
-  uint64_t beg, end;
-  cta_range(a.meta->F, bid, nb, beg, end);
-  uint32_t c = 0;
-  for (uint64_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
-    const uint32_t node = a.first_list[i];
-    c += num_leaf_descendents(node, a.N);
-    // collect_diff keeps a first-occurrence region only when the map names it as the
-    // owner of its digest (:548-556); the labelling guarantees it, so check it here
-    const uint64_t slot = map_find(a.map, a.tree[node]);
-    if (slot > a.map.cap || map_node(a.map, slot) != node || map_tree(a.map, slot) != a.cur)
-      set_error(a.st, DERR_INTERNAL, 20);
-  }
-  const uint32_t t = block_reduce_sum(c, sh);
-  if (threadIdx.x == 0) a.partial2[bid] = t;
-}
-__global__ void __launch_bounds__(COMPACT_THREADS) region_count_kernel(DiffArgs a0) {
-  griddep_enter();
-  region_count_body(with_round(a0), blockIdx.x, gridDim.x);
-}
-__global__ void __launch_bounds__(COMPACT_THREADS) region_count_seg(SegGrid s) {
-  uint32_t bid, nb;
-  const uint32_t h = seg_locate(s, bid, nb);
-  region_count_body(with_round(s.args[h]), bid, nb);
-}
-
-__device__ __forceinline__ void region_scan_body(const DiffArgs& a, uint32_t bid, uint32_t nb, uint32_t g) {
-  __shared__ uint32_t sh[33];
-  uint32_t tot;
-  const uint32_t i = threadIdx.x;
-  const uint32_t v = i < g ? a.partial2[i] : 0u;
-  const uint32_t e = block_excl_scan(v, sh, &tot);
-  if (i < g) a.partial2[i] = e;
-  if (i == 0) a.meta->T = tot;
-}
-__global__ void __launch_bounds__(1024) region_scan_kernel(DiffArgs a0, uint32_t g) {
-  griddep_enter();
-  region_scan_body(with_round(a0), blockIdx.x, gridDim.x, g);
-}
-__global__ void __launch_bounds__(1024) region_scan_seg(SegGrid s) {
-  uint32_t bid, nb;
-  const uint32_t h = seg_locate(s, bid, nb);
-  region_scan_body(with_round(s.args[h]), bid, nb, s.g[h]);
-}
-
-__device__ __forceinline__ void region_write_body(const DiffArgs& a, uint32_t bid, uint32_t nb) {
-  __shared__ uint32_t sh[COMPACT_THREADS / 32 + 1];
-  uint64_t beg, end;
-  cta_range(a.meta->F, bid, nb, beg, end);
-  uint32_t base = a.partial2[bid];
-  for (uint64_t t0 = beg; t0 < end; t0 += blockDim.x) {
-    const uint64_t i = t0 + threadIdx.x;
-    const uint32_t len = i < end ? num_leaf_descendents(a.first_list[i], a.N) : 0u;
-    uint32_t tot;
-    const uint32_t e = block_excl_scan(len, sh, &tot);
-    if (i < end) a.region_off[i] = base + e;
-    base += tot;
-  }
-}
-__global__ void __launch_bounds__(COMPACT_THREADS) region_write_kernel(DiffArgs a0) {
-  griddep_enter();
-  region_write_body(with_round(a0), blockIdx.x, gridDim.x);
-}
-__global__ void __launch_bounds__(COMPACT_THREADS) region_write_seg(SegGrid s) {
-  uint32_t bid, nb;
-  const uint32_t h = seg_locate(s, bid, nb);
-  region_write_body(with_round(s.args[h]), bid, nb);
-}
-
-// ---------------------------------------------------------------- shifted duplicates
-// source NodeID of each entry (:572-580, :672-674) and per-range histograms by checkpoint
-__device__ __forceinline__ void shift_prev_body(const DiffArgs& a, uint32_t bid, uint32_t nb, uint32_t bcap) {
-  const uint32_t B = a.rs->buckets <= bcap ? a.rs->buckets : bcap;
-  extern __shared__ uint32_t hs[];
-  uint64_t beg, end;
-  cta_range(a.meta->S, bid, nb, beg, end);
-  for (uint32_t t = threadIdx.x; t < B; t += blockDim.x) hs[t] = 0;
-  __syncthreads();
-  for (uint64_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
-    const uint32_t node = a.shift_list[i];
-    const uint64_t slot = map_find(a.map, a.tree[node]);
-    uint32_t pn = 0, pt = 0;
-    if (slot <= a.map.cap) {
-      pn = map_node(a.map, slot);
-      pt = map_tree(a.map, slot);
-    } else {
-      set_error(a.st, DERR_INTERNAL, 30);
-    }
-    if (pt >= B) {
-      set_error(a.st, DERR_INTERNAL, 31);
-      pt = 0;
-    }
-    a.sprev[i] = pn;
-    a.skey[i] = pt;
-    atomicAdd(&hs[pt], 1u);
-  }
-  __syncthreads();
-  for (uint32_t t = threadIdx.x; t < B; t += blockDim.x) {
-    const uint32_t v = hs[t];
-    a.partial[(uint64_t)t * nb + bid] = v;
-    if (v) atomicAdd(&a.hist[t], v);
-  }
-}
-__global__ void __launch_bounds__(128) shift_prev_kernel(DiffArgs a0, uint32_t bcap) {
-  griddep_enter();
-  shift_prev_body(with_round(a0), blockIdx.x, gridDim.x, bcap);
-}
-__global__ void __launch_bounds__(128) shift_prev_seg(SegGrid s) {
-  uint32_t bid, nb;
-  const uint32_t h = seg_locate(s, bid, nb);
-  shift_prev_body(with_round(s.args[h]), bid, nb, s.bcap[h]);
-}
-
-// one CTA: bucket starts, repeat table, per-range scatter bases, header, byte layout
-__device__ __forceinline__ void layout_body(const DiffArgs& a, uint32_t bid, uint32_t nb, uint32_t bcap, uint32_t g) {
-  const uint32_t B = a.rs->buckets <= bcap ? a.rs->buckets : bcap;
+// one CTA: bucket starts, repeat table, per-range scatter bases, header, byte layout.  The counts
+// come from other CTAs of the same launch, so they are read past L1.
+__device__ __forceinline__ void layout_body(const DiffArgs& a, uint32_t B, uint32_t g) {
   __shared__ uint32_t sh[33];
   __shared__ uint32_t carry_start, carry_rows;
   if (threadIdx.x == 0) { carry_start = 0; carry_rows = 0; }
@@ -354,15 +309,14 @@ __device__ __forceinline__ void layout_body(const DiffArgs& a, uint32_t bid, uin
   // count P first so the table position is known
   for (uint32_t t0 = 0; t0 < B; t0 += blockDim.x) {
     const uint32_t t = t0 + threadIdx.x;
-    const uint32_t h = t < B ? a.hist[t] : 0u;
-    uint32_t tot_h, tot_r;
+    const uint32_t h = t < B ? __ldcg(&a.hist[t]) : 0u;
+    uint32_t tot_h;
     const uint32_t eh = block_excl_scan(h, sh, &tot_h);
-    const uint32_t er = block_excl_scan(h ? 1u : 0u, sh, &tot_r);
+    const uint32_t tot_r = (uint32_t)__syncthreads_count(h != 0u);
     if (t < B) a.bucket_start[t] = carry_start + eh;
     __syncthreads();
     if (threadIdx.x == 0) { carry_start += tot_h; carry_rows += tot_r; }
     __syncthreads();
-    (void)er;
   }
   const uint32_t P = carry_rows;
   const uint64_t F = m0.F, S = m0.S, T = m0.T;
@@ -378,12 +332,12 @@ __device__ __forceinline__ void layout_body(const DiffArgs& a, uint32_t bid, uin
   __syncthreads();
   for (uint32_t t0 = 0; t0 < B; t0 += blockDim.x) {
     const uint32_t t = t0 + threadIdx.x;
-    const uint32_t h = t < B ? a.hist[t] : 0u;
+    const uint32_t h = t < B ? __ldcg(&a.hist[t]) : 0u;
     uint32_t tot_r;
     const uint32_t er = block_excl_scan(h ? 1u : 0u, sh, &tot_r);
     if (h) {
       uint32_t* row = reinterpret_cast<uint32_t*>(a.diff + count_off + 8ull * (row_carry + er));
-      row[0] = t;
+      row[0] = a.baseline_id + t;
       row[1] = h;
     }
     __syncthreads();
@@ -400,7 +354,7 @@ __device__ __forceinline__ void layout_body(const DiffArgs& a, uint32_t bid, uin
 #pragma unroll 4
       for (uint32_t j = 0; j < g; j += 32) {
         const uint32_t b = j + lane;
-        const uint32_t v = b < g ? row[b] : 0u;
+        const uint32_t v = b < g ? __ldcg(&row[b]) : 0u;
         const uint32_t inc = warp_incl_scan(v);
         if (b < g) row[b] = carry + inc - v;
         carry += __shfl_sync(0xffffffffu, inc, 31);
@@ -428,27 +382,84 @@ __device__ __forceinline__ void layout_body(const DiffArgs& a, uint32_t bid, uin
     m->map_size = *a.map.size;
   }
 }
-__global__ void __launch_bounds__(1024) layout_kernel(DiffArgs a0, uint32_t bcap, uint32_t g) {
-  griddep_enter();
-  layout_body(with_round(a0), blockIdx.x, gridDim.x, bcap, g);
+// Source NodeID of each shifted root (:572-580, :672-674) and per-range counts by checkpoint, one
+// range per CTA of the first `ranges`; the one of them that finishes last lays the diff out.
+// collect_diff keeps a first-occurrence region only when the map names it as the owner of its
+// digest (:548-556); the labelling guarantees it, so that is checked here by the other CTAs.
+__device__ __forceinline__ void diff_shift_body(const DiffArgs& a, uint32_t bid, uint32_t nb, uint32_t bcap,
+                                                uint32_t ranges) {
+  if (bid >= ranges) {
+    const uint32_t F = a.meta->F;
+    for (uint64_t i = (bid - ranges) * (uint64_t)blockDim.x + threadIdx.x; i < F;
+         i += (uint64_t)(nb - ranges) * blockDim.x) {
+      const uint32_t node = a.first_list[i];
+      const uint64_t slot = map_find(a.map, a.tree[node]);
+      if (slot > a.map.cap || map_node(a.map, slot) != node || map_tree(a.map, slot) != a.cur)
+        set_error(a.st, DERR_INTERNAL, 20);
+    }
+    return;
+  }
+  nb = ranges;
+  const uint32_t B = bucket_count(a, bcap);
+  extern __shared__ uint32_t hs[];
+  __shared__ uint32_t last;
+  uint64_t beg, end;
+  for (uint32_t t = threadIdx.x; t < B; t += blockDim.x) hs[t] = 0;
+  __syncthreads();
+  cta_range(a.meta->S, bid, nb, beg, end);
+  for (uint64_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
+    const uint32_t node = a.shift_list[i];
+    const uint64_t slot = map_find(a.map, a.tree[node]);
+    uint32_t pn = 0, pt = 0;
+    if (slot <= a.map.cap) {
+      pn = map_node(a.map, slot);
+      pt = map_tree(a.map, slot) - a.baseline_id;
+    } else {
+      set_error(a.st, DERR_INTERNAL, 30);
+    }
+    if (pt >= B) {
+      set_error(a.st, DERR_INTERNAL, 31);
+      pt = 0;
+    }
+    a.sprev[i] = pn;
+    a.skey[i] = pt;
+    atomicAdd(&hs[pt], 1u);
+  }
+  __syncthreads();
+  for (uint32_t t = threadIdx.x; t < B; t += blockDim.x) {
+    const uint32_t v = hs[t];
+    a.partial[(uint64_t)t * nb + bid] = v;
+    if (v) atomicAdd(&a.hist[t], v);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&a.meta->done, 1u) == nb - 1u;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  layout_body(a, B, nb);
 }
-__global__ void __launch_bounds__(1024) layout_seg(SegGrid s) {
+__global__ void __launch_bounds__(SHIFT_THREADS) diff_shift_kernel(DiffArgs a0, uint32_t bcap, uint32_t ranges) {
+  griddep_enter();
+  diff_shift_body(with_round(a0), blockIdx.x, gridDim.x, bcap, ranges);
+}
+__global__ void __launch_bounds__(SHIFT_THREADS) diff_shift_seg(SegGrid s) {
   uint32_t bid, nb;
   const uint32_t h = seg_locate(s, bid, nb);
-  layout_body(with_round(s.args[h]), bid, nb, s.bcap[h], s.gs[h]);
+  diff_shift_body(with_round(s.args[h]), bid, nb, s.bcap[h], s.gs[h]);
 }
 
-// stable scatter of shift entries: one warp walks its range in order
-__device__ __forceinline__ void shift_write_body(const DiffArgs& a, uint32_t bid, uint32_t nb, uint32_t bcap) {
-  const uint32_t B = a.rs->buckets <= bcap ? a.rs->buckets : bcap;
-  extern __shared__ uint32_t run[];
+// stable scatter of one range of the shifted entries: a warp walks it in order; run: B words of
+// the warp's own
+__device__ __forceinline__ void shift_write_range(const DiffArgs& a, uint32_t range, uint32_t ranges, uint32_t B,
+                                                  uint32_t* run) {
+  const uint32_t lane = threadIdx.x & 31u;
   uint64_t beg, end;
-  cta_range(a.meta->S, bid, nb, beg, end);
+  cta_range(a.meta->S, range, ranges, beg, end);
   if (beg >= end) return;
-  for (uint32_t t = threadIdx.x; t < B; t += 32) run[t] = a.partial[(uint64_t)t * nb + bid];
+  for (uint32_t t = lane; t < B; t += 32) run[t] = a.partial[(uint64_t)t * ranges + range];
   __syncwarp();
   const uint64_t shift_off = a.meta->shift_off;
-  const uint32_t lane = threadIdx.x;
   // UNR groups of 32 entries per pass: their loads are issued together (they do
   // not depend on the running bucket positions), then the groups are placed in order
   constexpr uint32_t UNR = 4;
@@ -480,39 +491,84 @@ __device__ __forceinline__ void shift_write_body(const DiffArgs& a, uint32_t bid
     }
   }
 }
-__global__ void __launch_bounds__(32) shift_write_kernel(DiffArgs a0, uint32_t bcap) {
-  griddep_enter();
-  shift_write_body(with_round(a0), blockIdx.x, gridDim.x, bcap);
-}
-__global__ void __launch_bounds__(32) shift_write_seg(SegGrid s) {
-  uint32_t bid, nb;
-  const uint32_t h = seg_locate(s, bid, nb);
-  shift_write_body(with_round(s.args[h]), bid, nb, s.bcap[h]);
-}
-
-// ---------------------------------------------------------------- metadata + data gather
-__device__ __forceinline__ uint32_t find_region(const uint32_t* off, uint32_t F, uint64_t k) {
-  uint32_t lo = 0, hi = F;   // largest i with off[i] <= k
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (off[mid] <= k) lo = mid; else hi = mid;
+// ---------------------------------------------------------------- data gather
+// 16 bytes of the buffer from byte s on (s + 16 <= len), whatever its alignment: two aligned
+// 16-byte loads and a byte shift, or byte loads where an aligned load would leave the buffer
+__device__ __forceinline__ uint4 load_unit(const uint8_t* data, uint64_t len, uint64_t s) {
+  const uint8_t* p = data + s;
+  const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 15u);
+  if (mis == 0) return __ldg(reinterpret_cast<const uint4*>(p));
+  uint4 r;
+  if (s < mis || len - s < 32u - mis) {
+    uint8_t t[16];
+#pragma unroll
+    for (int b = 0; b < 16; b++) t[b] = p[b];
+    memcpy(&r, t, 16);
+    return r;
   }
-  return lo;
+  const uint4* q = reinterpret_cast<const uint4*>(p - mis);
+  const uint4 lo = __ldg(q), hi = __ldg(q + 1);
+  uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+  if (mis & 8u) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) w[i] = w[i + 2];
+  }
+  if (mis & 4u) {
+#pragma unroll
+    for (int i = 0; i < 5; i++) w[i] = w[i + 1];
+  }
+  const uint32_t sh = 8u * (mis & 3u);
+  r.x = __funnelshift_r(w[0], w[1], sh);
+  r.y = __funnelshift_r(w[1], w[2], sh);
+  r.z = __funnelshift_r(w[2], w[3], sh);
+  r.w = __funnelshift_r(w[3], w[4], sh);
+  return r;
 }
 
-// Data section.  Each warp owns a contiguous range [k0, k1) of diff chunks (the same share for
-// every warp) and copies it with 16-byte vectors, lane after lane over consecutive 16-byte units
-// of the range, GATHER_UNROLL units per lane in flight (chunk size a multiple of 16, both sides
-// 16-byte aligned), whatever the region boundaries: many regions are a few chunks long.  A unit's
-// source follows from its chunk's region (start in the diff, root node).  The starts and roots
-// of 32 regions at a time are held one per lane, and each unit finds its region among them by a
-// five-step shuffle search, so no load waits on another: looked up in memory, each group of
-// chunks waited for two dependent loads before its data load could issue.  The short last chunk
-// is zero-padded (:643-645).
+// a 16-byte unit of the data section that a region ends in, or whose source reaches past the
+// buffer's end (zeros, :643-645): byte by byte, region r holding its first byte
+struct GatherBytes {
+  const uint8_t* data;
+  uint64_t len, cs, total;   // buffer length, chunk size, bytes of the data section
+  const uint32_t *region_off, *first_list;
+  uint32_t F, n, N, D;
+};
+__device__ __noinline__ void gather_unit_bytes(GatherBytes a, uint8_t* dst, uint64_t unit, uint32_t r) {
+  const uint64_t cs = a.cs;
+  uint64_t pos = 16ull * unit;
+  uint64_t shift = 0;   // source byte minus data-section byte, within region r
+  bool known = false;
+  for (int b = 0; b < 16 && pos < a.total; b++, pos++) {
+    while (r + 1u < a.F && (uint64_t)a.region_off[r + 1u] * cs <= pos) {
+      r++;
+      known = false;
+    }
+    if (!known) {
+      const uint64_t chunk = node_span(a.first_list[r], a.N, a.D).first - (a.n - 1u);
+      shift = chunk * cs - (uint64_t)a.region_off[r] * cs;
+      known = true;
+    }
+    const uint64_t s = pos + shift;
+    dst[pos] = s < a.len ? a.data[s] : 0u;
+  }
+}
+
+// Data section.  The chunks of a region lie one after another in the buffer, so the section is a
+// sequence of byte runs.  Each warp owns an equal share of the section's 16-byte units and copies
+// it lane after lane over consecutive units, GATHER_UNROLL per lane in flight, whatever the region
+// boundaries: many regions are a few chunks long.  The starts and sources of 32 regions at a time
+// are held one per lane, and each unit finds its region among them by a five-step shuffle search,
+// so no load waits on another.  Where one region covers a whole step of the warp the search is
+// left out and the warp streams to the region's end: a 4 GiB baseline, one region, was bound by
+// the search's instructions (2.40 ms, now 1.41 ms; a plain copy of the same bytes takes 1.35 ms).
+// Chunk sizes or buffers that are not 16-byte aligned take the same path with shifted loads
+// (load_unit): with one thread per chunk and byte copies, 1000 B chunks of a 150 MB buffer at an
+// 8-byte offset took 331 us per increment of 5 % and the whole series 2.40 ms, now 0.94 ms.
 #ifndef B2D_GATHER_UNROLL
 #define B2D_GATHER_UNROLL 4
 #endif
-__device__ __forceinline__ void gather_vec_body(const DiffArgs& a, uint32_t bid, uint32_t nb) {
+template <bool ALIGNED>
+__device__ __forceinline__ void gather_body(const DiffArgs& a, uint32_t bid, uint32_t nb) {
   constexpr uint32_t U = B2D_GATHER_UNROLL;
   const DevMeta m = *a.meta;
   uint8_t* dst_base = a.diff + m.data_off;
@@ -522,111 +578,141 @@ __device__ __forceinline__ void gather_vec_body(const DiffArgs& a, uint32_t bid,
   for (uint64_t i = gtid; i < m.F; i += nthr) first_meta[i] = a.first_list[i] - a.id_bias;
   if (m.T == 0) return;
   const uint32_t lane = threadIdx.x & 31u;
-  const uint64_t warp = gtid >> 5, nwarps = nthr >> 5;
-  uint64_t k0, k1;
-  cta_range(m.T, (uint32_t)warp, (uint32_t)nwarps, k0, k1);
-  if (k0 >= k1) return;
-  const uint64_t T = m.T;
+  const uint64_t total = m.T * a.cs;
   const uint32_t F = m.F;
-  const uint32_t units = a.cs / 16u;   // 16-byte units per chunk
-  const bool pow2 = (units & (units - 1u)) == 0u;
-  const uint32_t ush = __ffs(units) - 1u;
-  const uint64_t last = a.n - 1ull;
-  const bool short_last = (a.len % a.cs) != 0;
-  const uint4* src = reinterpret_cast<const uint4*>(a.data);
+  uint64_t u0, u1;
+  cta_range((total + 15u) / 16u, (uint32_t)(gtid >> 5), (uint32_t)(nthr >> 5), u0, u1);
+  if (u0 >= u1) return;
   uint4* dst = reinterpret_cast<uint4*>(dst_base);
-  // largest r with region_off[r] <= k0 (region_off[0] = 0)
-  uint32_t r = warp_lower_bound(a.region_off, F, k0 + 1u) - 1u;
-  uint64_t k = k0;
-  while (k < k1) {
-    // regions r .. r + 31, one per lane; chunks before `bend` lie in them
+  // largest r with region_off[r] <= the first unit's chunk (region_off[0] = 0)
+  uint32_t r = warp_lower_bound(a.region_off, F, 16ull * u0 / a.cs + 1u) - 1u;
+  uint64_t u = u0;
+  while (u < u1) {
+    // regions r .. r + 31, one per lane, as byte positions relative to unit u; a step covers at
+    // most 1 GiB, so positions fit 32 bits and a start beyond the step is never met
+    const uint64_t pos0 = 16ull * u;
     const uint32_t rl = r + lane;
-    const uint32_t off_l = rl < F ? a.region_off[rl] : (uint32_t)T;
-    const uint32_t node_l = rl < F ? a.first_list[rl] : 0u;
-    const uint64_t bend = r + 32u < F ? a.region_off[r + 32u] : T;
-    const uint64_t kend = bend < k1 ? bend : k1;
-    const uint64_t u_end = kend * units;
-    for (uint64_t base = k * units; base < u_end; base += 32ull * U) {
+    const bool has = rl < F;
+    const uint64_t off = has ? (uint64_t)a.region_off[rl] * a.cs : total;
+    uint64_t src0 = 0;   // buffer byte that data-section byte pos0 would come from
+    if (has) {
+      const NodeSpan sp = node_span(a.first_list[rl], a.N, a.D);
+      const uint64_t chunk = sp.first - (a.n - 1u);
+      if (chunk + sp.count > a.n) set_error(a.st, DERR_INTERNAL, 40);
+      src0 = chunk * a.cs - off + pos0;   // wraps where the region starts later: only sums are used
+    }
+    const uint64_t relw = off > pos0 ? off - pos0 : 0ull;
+    const uint32_t rel = relw > 0xfffffff0ull ? 0xfffffff0u : (uint32_t)relw;
+    const uint64_t bend = r + 32u < F ? (uint64_t)a.region_off[r + 32u] * a.cs : total;
+    const uint64_t brel = bend - pos0;
+    uint32_t next = __shfl_down_sync(0xffffffffu, rel, 1);   // where this lane's region ends
+    if (lane == 31u) next = brel > 0xfffffff0ull ? 0xfffffff0u : (uint32_t)brel;
+    uint64_t uend = (bend + 15u) / 16u;
+    if (uend > u1) uend = u1;
+    if (uend > u + (1u << 26)) uend = u + (1u << 26);
+    const uint32_t units = (uint32_t)(uend - u);
+    // regions that follow one another in the buffer too (a list's runs of chunks) are one run
+    const uint64_t src_first = __shfl_sync(0xffffffffu, src0, 0);   // by every lane: not inside the || below
+    if (__all_sync(0xffffffffu, !has || src0 == src_first))
+      next = brel > 0xfffffff0ull ? 0xfffffff0u : (uint32_t)brel;
+    auto region_of = [&](uint32_t pos) {   // largest j with region start j <= pos
+      uint32_t j = 0;
+#pragma unroll
+      for (uint32_t step = 16; step >= 1; step >>= 1) {
+        const uint32_t o = __shfl_sync(0xffffffffu, rel, j + step);
+        if (o <= pos) j += step;
+      }
+      return j;
+    };
+    for (uint32_t b = 0; b < units;) {
+      {   // one region over the warp's next whole steps: stream to its end
+        const uint32_t j = region_of(16u * b);
+        const uint32_t end = __shfl_sync(0xffffffffu, next, j);
+        uint64_t s = __shfl_sync(0xffffffffu, src0, j) + 16ull * b;
+        const uint64_t room = s < a.len ? (a.len - s) / 16u : 0ull;   // units before the buffer's end
+        uint32_t whole = (end / 16u < units ? end / 16u : units) - b;
+        if (whole > room) whole = (uint32_t)room;
+        if (whole >= 32u * U) {
+          s += 16ull * lane;
+          uint4* d = dst + u + b + lane;
+          b += whole / (32u * U) * (32u * U);
+          for (uint32_t left = whole / (32u * U); left; left--) {
+            uint4 v[U];
+#pragma unroll
+            for (uint32_t i = 0; i < U; i++)
+              v[i] = ALIGNED ? __ldg(reinterpret_cast<const uint4*>(a.data + s + 512u * i))
+                             : load_unit(a.data, a.len, s + 512u * i);
+#pragma unroll
+            for (uint32_t i = 0; i < U; i++) d[32u * i] = v[i];
+            s += 512u * U;
+            d += 32u * U;
+          }
+          continue;
+        }
+      }
       uint4 v[U];
-      uint32_t st = 0;   // bit i: unit i is this lane's to copy
+      uint32_t st = 0;   // bit i: unit i is this lane's to store
 #pragma unroll
       for (uint32_t i = 0; i < U; i++) {
-        const uint64_t g = base + lane + 32ull * i;
-        const bool act = g < u_end;
-        const uint64_t kk = act ? (pow2 ? g >> ush : g / units) : k;
-        uint32_t j = 0;   // largest j with region start j <= kk
-#pragma unroll
-        for (uint32_t step = 16; step >= 1; step >>= 1) {
-          const uint32_t o = __shfl_sync(0xffffffffu, off_l, j + step);
-          if (o <= kk) j += step;
-        }
-        const uint32_t off = __shfl_sync(0xffffffffu, off_l, j);
-        const uint32_t node = __shfl_sync(0xffffffffu, node_l, j);
+        const uint32_t g = b + lane + 32u * i;
+        const bool act = g < units;
+        const uint32_t pos = act ? 16u * g : 16u * b;
+        const uint32_t j = region_of(pos);
+        const uint32_t end = __shfl_sync(0xffffffffu, next, j);
+        const uint64_t s = __shfl_sync(0xffffffffu, src0, j) + pos;
         if (!act) continue;
-        const uint64_t chunk = (uint64_t)(leftmost_leaf(node, a.N) - (a.n - 1u)) + (kk - off);
-        const uint64_t su = chunk * units + (g - kk * units);
-        if (chunk > last) {
-          set_error(a.st, DERR_INTERNAL, 40);
-        } else if (short_last && chunk == last) {   // bytes past the buffer's end are zero
-          uint8_t tmp[16];
-          for (uint32_t b = 0; b < 16; b++) tmp[b] = 16ull * su + b < a.len ? a.data[16ull * su + b] : 0u;
-          uint4 w;
-          memcpy(&w, tmp, 16);
-          dst[g] = w;
-        } else {
+        if (pos + 16u <= end && s < a.len && a.len - s >= 16u) {
           st |= 1u << i;
-          v[i] = __ldg(src + su);
+          v[i] = ALIGNED ? __ldg(reinterpret_cast<const uint4*>(a.data + s)) : load_unit(a.data, a.len, s);
+        } else {
+          gather_unit_bytes(GatherBytes{a.data, a.len, a.cs, total, a.region_off, a.first_list, F, a.n, a.N, a.D},
+                            dst_base, u + g, r + j);
         }
       }
 #pragma unroll
       for (uint32_t i = 0; i < U; i++)
-        if ((st >> i) & 1u) dst[base + lane + 32ull * i] = v[i];
+        if ((st >> i) & 1u) dst[u + b + lane + 32u * i] = v[i];
+      b += 32u * U;
     }
-    k = kend;
-    r += 32u;
+    u = uend;
+    if (16ull * uend >= bend) r += 32u;   // else a step's limit: the same regions go on
   }
-}
-__global__ void __launch_bounds__(256) gather_vec_kernel(DiffArgs a0) {
-  griddep_enter();
-  gather_vec_body(with_round(a0), blockIdx.x, gridDim.x);
-}
-__global__ void __launch_bounds__(256) gather_vec_seg(SegGrid s) {
-  uint32_t bid, nb;
-  const uint32_t h = seg_locate(s, bid, nb);
-  gather_vec_body(with_round(s.args[h]), bid, nb);
 }
 
-// any chunk size / alignment: one thread per chunk, byte copies
-__device__ __forceinline__ void gather_bytes_body(const DiffArgs& a, uint32_t bid, uint32_t nb) {
-  const DevMeta m = *a.meta;
-  uint8_t* dst_base = a.diff + m.data_off;
-  uint8_t* first_meta = a.diff + m.first_off;
-  const uint64_t gtid = bid * (uint64_t)blockDim.x + threadIdx.x;
-  const uint64_t nthr = (uint64_t)nb * blockDim.x;
-  for (uint64_t i = gtid; i < m.F; i += nthr) {
-    const uint32_t v = a.first_list[i] - a.id_bias;
-    memcpy(first_meta + 4 * i, &v, 4);
-  }
-  for (uint64_t k = gtid; k < m.T; k += nthr) {
-    const uint32_t r = find_region(a.region_off, m.F, k);
-    const uint32_t node = a.first_list[r];
-    const uint64_t chunk = (uint64_t)(leftmost_leaf(node, a.N) - (a.n - 1u)) + (k - a.region_off[r]);
-    if (chunk >= a.n) { set_error(a.st, DERR_INTERNAL, 41); continue; }
-    const uint64_t src_off = chunk * a.cs;
-    const uint64_t avail = (chunk == a.n - 1u) ? a.len - src_off : a.cs;
-    uint8_t* d = dst_base + k * a.cs;
-    const uint8_t* s = a.data + src_off;
-    for (uint64_t b = 0; b < a.cs; b++) d[b] = b < avail ? s[b] : 0u;
-  }
+// ---------------------------------------------------------------- scatter and gather, one launch
+// CTAs below shift_ctas(ranges, B) scatter the shifted entries, one range per warp; the others
+// write the first-occurrence list and the data.  Both need only the layout.
+__host__ __device__ __forceinline__ uint32_t shift_warps(uint32_t bcap) {   // ranges per CTA: 8 KB of positions
+  const uint32_t w = 2048u / (bcap ? bcap : 1u);
+  return w < 1u ? 1u : (w > EMIT_THREADS / 32u ? EMIT_THREADS / 32u : w);
 }
-__global__ void __launch_bounds__(256) gather_bytes_kernel(DiffArgs a0) {
+__host__ __device__ __forceinline__ uint32_t shift_ctas(uint32_t ranges, uint32_t bcap) {
+  const uint32_t w = shift_warps(bcap);
+  return (ranges + w - 1u) / w;
+}
+template <bool ALIGNED>
+__device__ __forceinline__ void diff_emit_body(const DiffArgs& a, uint32_t bid, uint32_t nb, uint32_t bcap,
+                                               uint32_t ranges) {
+  extern __shared__ uint32_t run[];
+  const uint32_t nbs = shift_ctas(ranges, bcap);
+  if (bid >= nbs) {
+    gather_body<ALIGNED>(a, bid - nbs, nb - nbs);
+    return;
+  }
+  const uint32_t warp = threadIdx.x >> 5, warps = shift_warps(bcap);
+  const uint32_t range = bid * warps + warp;
+  if (warp < warps && range < ranges) shift_write_range(a, range, ranges, bucket_count(a, bcap), run + warp * bcap);
+}
+template <bool ALIGNED>
+__global__ void __launch_bounds__(EMIT_THREADS) diff_emit_kernel(DiffArgs a0, uint32_t bcap, uint32_t ranges) {
   griddep_enter();
-  gather_bytes_body(with_round(a0), blockIdx.x, gridDim.x);
+  diff_emit_body<ALIGNED>(with_round(a0), blockIdx.x, gridDim.x, bcap, ranges);
 }
-__global__ void __launch_bounds__(256) gather_bytes_seg(SegGrid s) {
+template <bool ALIGNED>
+__global__ void __launch_bounds__(EMIT_THREADS) diff_emit_seg(SegGrid s) {
   uint32_t bid, nb;
   const uint32_t h = seg_locate(s, bid, nb);
-  gather_bytes_body(with_round(s.args[h]), bid, nb);
+  diff_emit_body<ALIGNED>(with_round(s.args[h]), bid, nb, s.bcap[h], s.gs[h]);
 }
 
 static uint32_t grid_for(uint64_t units, uint64_t per_cta, uint32_t cap) {
@@ -636,87 +722,53 @@ static uint32_t grid_for(uint64_t units, uint64_t per_cta, uint32_t cap) {
 
 // grids follow the buffer size (host-known bounds: F, S <= n), so a small buffer is not charged
 // for hundreds of idle CTAs per launch; large buffers get the full grids
-DiffGrids diff_grids(const DiffArgs& a, int sm_count) {
+DiffGrids diff_grids(const DiffArgs& a, uint32_t bcap, int sm_count) {
   DiffGrids r;
-  r.g = grid_for(((uint64_t)a.N + 63u) / 64u, 512, COMPACT_GRID);   // ~1 64-node load per thread
-  // shift-entry ranges: the layout kernel scans every range's count per bucket in one CTA, so
-  // fewer, longer ranges (<= 296) keep it short; the scatter walks each range with one warp
+  r.g = grid_for(((uint64_t)a.N + 64u) / 64u, 512, COMPACT_GRID);   // ~1 64-node load per thread
+  // shifted-entry ranges: the layout scans every range's count per bucket in one CTA, so fewer,
+  // longer ranges (<= 296) keep it short; the scatter walks each range with one warp
   r.gs = grid_for(a.n, 8192, SHIFT_GRID);
-  r.gl = (2u * (a.D + 2u) * 32u + 255u) / 256u;
-  r.gp = grid_for(a.n, 2048, (uint32_t)sm_count * 2u);
-  r.gg = grid_for((uint64_t)a.n * a.cs, 32768, (uint32_t)sm_count * 4u);
-  const bool vec = (a.cs % 16u == 0) && ((reinterpret_cast<uintptr_t>(a.data) & 15u) == 0) &&
-                   ((reinterpret_cast<uintptr_t>(a.diff) & 15u) == 0);
-  r.variant = vec ? 0 : 1;
+  r.gc = r.gs + grid_for(a.n, 4096, (uint32_t)sm_count * 8u);
+  r.ge = shift_ctas(r.gs, bcap) + grid_for((uint64_t)a.n * a.cs, 32768, (uint32_t)sm_count * 8u);
+  // 16-byte aligned source units; both kinds write a 16-byte aligned data section
+  r.variant = (a.cs % 16u == 0) && ((reinterpret_cast<uintptr_t>(a.data) & 15u) == 0) ? 0 : 1;
   return r;
 }
+
+uint32_t diff_emit_smem(uint32_t bcap) { return (uint32_t)sizeof(uint32_t) * shift_warps(bcap) * bcap; }
 
 cudaError_t launch_collect_diff_batch(const DiffBatch& b, cudaStream_t stream, uint32_t* launches) {
   if (b.max_bcap > MAX_BUCKETS || b.base.n == 0) return cudaErrorInvalidValue;
   SegGrid s = b.base;
   uint32_t c = 0;
-  const size_t hsm = sizeof(uint32_t) * b.max_bcap;
-  s.beg = b.beg_g;   compact_count_seg<<<b.tot_g, COMPACT_THREADS, 0, stream>>>(s); c++;
-  s.beg = b.beg_one; compact_scan_seg<<<b.tot_one, 1024, 0, stream>>>(s); c++;
-  s.beg = b.beg_g;   compact_write_seg<<<b.tot_g, COMPACT_THREADS, 0, stream>>>(s); c++;
-  s.beg = b.beg_gl;  compact_levels_seg<<<b.tot_gl, 256, 0, stream>>>(s); c++;
-  s.beg = b.beg_gp;  compact_permute_seg<<<b.tot_gp, 256, 0, stream>>>(s); c++;
-  s.beg = b.beg_g;   region_count_seg<<<b.tot_g, COMPACT_THREADS, 0, stream>>>(s); c++;
-  s.beg = b.beg_one; region_scan_seg<<<b.tot_one, 1024, 0, stream>>>(s); c++;
-  s.beg = b.beg_g;   region_write_seg<<<b.tot_g, COMPACT_THREADS, 0, stream>>>(s); c++;
-  s.beg = b.beg_gs;  shift_prev_seg<<<b.tot_gs, 128, hsm, stream>>>(s); c++;
-  s.beg = b.beg_one; layout_seg<<<b.tot_one, 1024, 0, stream>>>(s); c++;
-  s.beg = b.beg_gs;  shift_write_seg<<<b.tot_gs, 32, hsm, stream>>>(s); c++;
+  s.beg = b.beg_g;   diff_count_seg<<<b.tot_g, COMPACT_THREADS, 0, stream>>>(s); c++;
+  s.beg = b.beg_g;   diff_write_seg<<<b.tot_g, COMPACT_THREADS, 0, stream>>>(s); c++;
+  s.beg = b.beg_gc;  diff_shift_seg<<<b.tot_gc, SHIFT_THREADS, sizeof(uint32_t) * b.max_bcap, stream>>>(s); c++;
   for (int v = 0; v < GATHER_VARIANTS; v++) {
-    if (!b.tot_gather[v]) continue;
-    s.beg = b.beg_gather[v];
-    if (v == 0) gather_vec_seg<<<b.tot_gather[v], 256, 0, stream>>>(s);
-    else gather_bytes_seg<<<b.tot_gather[v], 256, 0, stream>>>(s);
+    if (!b.tot_emit[v]) continue;
+    s.beg = b.beg_emit[v];
+    if (v == 0) diff_emit_seg<true><<<b.tot_emit[v], EMIT_THREADS, b.max_emit_smem, stream>>>(s);
+    else diff_emit_seg<false><<<b.tot_emit[v], EMIT_THREADS, b.max_emit_smem, stream>>>(s);
     c++;
   }
   if (launches) *launches = c;
   return cudaGetLastError();
 }
 
-cudaError_t launch_collect_diff(const DiffArgs& args, uint32_t bcap, int sm_count, cudaStream_t stream,
-                                bool node_order) {
-  DiffArgs a = args;
-  const DiffGrids dg = diff_grids(a, sm_count);
-  const uint32_t g = dg.g, gs = dg.gs;
-  const uint32_t B = bcap;   // capacity; each kernel reads the checkpoint's bucket count from rs
-  if (B > MAX_BUCKETS) return cudaErrorInvalidValue;
+cudaError_t launch_collect_diff(const DiffArgs& a, uint32_t bcap, int sm_count, cudaStream_t stream) {
+  const DiffGrids dg = diff_grids(a, bcap, sm_count);
+  // bcap is a capacity; each kernel reads the checkpoint's bucket count from rs
+  if (bcap > MAX_BUCKETS) return cudaErrorInvalidValue;
   // one kernel after another, each launched to overlap its start with its predecessor's end
-  // (launch_dependent); the scan kernel also clears the per-checkpoint bucket counts
-  cudaError_t e;
-#define B2D_LD(...)                                              \
-  if ((e = launch_dependent(__VA_ARGS__)) != cudaSuccess) return e;
-  B2D_LD(compact_count_kernel, g, COMPACT_THREADS, 0, stream, a)
-  B2D_LD(compact_scan_kernel, 1, 1024, 0, stream, a, g, B)
-  B2D_LD(compact_write_kernel, g, COMPACT_THREADS, 0, stream, a)
-  if (node_order) {
-    a.first_list = a.tmp_first;
-    a.shift_list = a.tmp_shift;
-  } else {
-    B2D_LD(compact_levels_kernel, dg.gl, 256, 0, stream, a)
-    B2D_LD(compact_permute_kernel, dg.gp, 256, 0, stream, a)
-  }
-  B2D_LD(region_count_kernel, g, COMPACT_THREADS, 0, stream, a)
-  B2D_LD(region_scan_kernel, 1, 1024, 0, stream, a, g)
-  B2D_LD(region_write_kernel, g, COMPACT_THREADS, 0, stream, a)
-  const size_t hsm = sizeof(uint32_t) * B;   // <= 32 KB for MAX_BUCKETS
-  B2D_LD(shift_prev_kernel, gs, 128, hsm, stream, a, B)
-  B2D_LD(layout_kernel, 1, 1024, 0, stream, a, B, gs)
-  B2D_LD(shift_write_kernel, gs, 32, hsm, stream, a, B)
-  const uint32_t gblocks = dg.gg;
-  const bool vec = (a.cs % 16u == 0) && ((reinterpret_cast<uintptr_t>(a.data) & 15u) == 0) &&
-                   ((reinterpret_cast<uintptr_t>(a.diff) & 15u) == 0);
-  if (vec) {
-    B2D_LD(gather_vec_kernel, gblocks, 256, 0, stream, a)
-  } else {
-    B2D_LD(gather_bytes_kernel, gblocks, 256, 0, stream, a)
-  }
-#undef B2D_LD
-  return cudaSuccess;
+  // (launch_dependent)
+  cudaError_t e = launch_dependent(diff_count_kernel, dg.g, COMPACT_THREADS, 0, stream, a, bcap);
+  if (e == cudaSuccess) e = launch_dependent(diff_write_kernel, dg.g, COMPACT_THREADS, 0, stream, a);
+  if (e == cudaSuccess)
+    e = launch_dependent(diff_shift_kernel, dg.gc, SHIFT_THREADS, sizeof(uint32_t) * bcap, stream, a, bcap, dg.gs);
+  if (e == cudaSuccess)
+    e = launch_dependent(dg.variant == 0 ? diff_emit_kernel<true> : diff_emit_kernel<false>, dg.ge, EMIT_THREADS,
+                         diff_emit_smem(bcap), stream, a, bcap, dg.gs);
+  return e;
 }
 
 }  // namespace b2d
