@@ -94,7 +94,7 @@ int b2d_set_stream(b2d_dedup* d, void* cuda_stream);
  *                       a power of two always use CTA bands
  *   "graph"             0 = launch a checkpoint's kernels one by one on the handle's stream
  *                       (default; measured faster), 1 = replay them as one CUDA graph, 2 = graph
- *                       without the phase-timing events (b2d_phase_times then reads 0) */
+ *                       that reports no phase times (b2d_phase_times then reads 0) */
 int b2d_set_param(b2d_dedup* d, const char* name, int64_t value);
 
 /* checkpoint(header_t&, uint8_t* data_ptr, size_t len, HostMirror& diff_h, bool make_baseline)
@@ -200,7 +200,7 @@ int b2d_timers(b2d_dedup* d, double out[4]);
 int b2d_restart_timers(b2d_dedup* d, double out[2]);
 /* datasizes: (data bytes incl. header, metadata bytes) of the last diff (:707-709) */
 int b2d_datasizes(b2d_dedup* d, uint64_t out[2]);
-/* Device time (seconds, CUDA events on the handle's stream) of the last checkpoint's three
+/* Device time (seconds, read from the global timer by its kernels) of the last checkpoint's three
  * stages: chunk hashing + labelling, Merkle forest, diff assembly.  *leaf_path (nullable) is 1
  * when the TMA-staged hashing kernel ran, 0 for the byte-granular one.  No reference
  * counterpart (the reference times whole phases on the host, src/tree_approach.cpp:1640-1688). */

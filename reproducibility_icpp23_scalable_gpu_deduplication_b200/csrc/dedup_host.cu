@@ -123,7 +123,22 @@ struct DevState {
   DevMeta meta;
   StraddleInfo straddle;
   RoundState round;
+  Stamps stamps;
 };
+static_assert(sizeof(DevState) % 4 == 0, "DevState is cleared and copied word by word");
+
+// The start of one checkpoint: a clear state and this checkpoint's RoundState, from `src` (pinned
+// host memory, read anew by every replay of a captured launch) or the launch's own argument.
+__global__ void round_init_kernel(DevState* ds, const RoundState* src, RoundState val) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  uint32_t* w = reinterpret_cast<uint32_t*>(ds);
+  for (uint32_t j = threadIdx.x; j < sizeof(DevState) / 4; j += blockDim.x) w[j] = 0u;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ds->round = src ? *src : val;
+    ds->stamps.begin = device_time_ns();
+  }
+}
 
 }  // namespace b2d
 
@@ -161,7 +176,7 @@ struct b2d_dedup {
   // replay each checkpoint's launches as one CUDA graph (off by default: on the 4 GiB series
   // the graph launch measured 0.15-0.2 ms slower per checkpoint than the 22 stream launches)
   bool use_graph = false;
-  bool graph_timing = true;       // phase timing events inside the graph
+  bool graph_timing = true;       // phase times are reported for graph replays
   double map_headroom = MAP_HEADROOM;   // baseline table size over its minimum (entries + N at max load)
   bool map_retune = false;              // resize an existing table to map_headroom at the next checkpoint
   int warp_bands = B2D_WARP_BANDS;      // forest phases that start with a warp band (bit 0: 1, bit 1: 2)
@@ -171,7 +186,6 @@ struct b2d_dedup {
   cudaStream_t stream = nullptr;
   int device = 0;
   int sm_count = 148;
-  cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
 
   DevBuf<Digest> tree;
   DevBuf<uint8_t> lab, leaflab, push, dupflag;
@@ -186,7 +200,7 @@ struct b2d_dedup {
   DevBuf<uint8_t> diff;
   DevBuf<DevState> state;
   PinnedBuf<DevState> state_h;
-  PinnedBuf<RoundState> round_h;   // this checkpoint's RoundState, uploaded by the graph
+  PinnedBuf<RoundState> round_h;   // this checkpoint's RoundState, read by a graph's first kernel
   const void* data = nullptr;      // buffer of the current checkpoint
   uint32_t bcap = 0;               // source-checkpoint bucket capacity of the scratch
   cudaGraphExec_t graph_exec = nullptr;
@@ -253,24 +267,12 @@ b2d_dedup::~b2d_dedup() {
       }
     }
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
-    for (auto& e : ev)
-      if (e) cudaEventDestroy(e);
     if (own_stream) cudaStreamDestroy(own_stream);
     if (cap_stream) cudaStreamDestroy(cap_stream);
   }
 }
 
 namespace {
-
-// A timing event inside a stream capture must be an external record node (a plain record only
-// joins streams there); outside a capture it is an ordinary record.
-cudaError_t record_timing(cudaEvent_t ev, cudaStream_t s) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  cudaError_t e = cudaStreamIsCapturing(s, &cs);
-  if (e != cudaSuccess) return e;
-  return cs == cudaStreamCaptureStatusActive ? cudaEventRecordWithFlags(ev, s, cudaEventRecordExternal)
-                                             : cudaEventRecord(ev, s);
-}
 
 // events that were never recorded (a failed launch) read as 0 and leave no error behind for
 // the next call's launch checks
@@ -409,7 +411,7 @@ LeafArgs leaf_args(const b2d_dedup* d, const RoundState* rs_dev) {
   const MapView m = map_at(d->map_mem, d->map_cap, d->map_size.p);
   return LeafArgs{static_cast<const uint8_t*>(d->data), d->data_len, d->chunk_size, d->n, d->kind, 0, 0,
                   d->tree.p, d->leaflab.p, d->dupflag.p, m, &d->state.p->status, rs_dev,
-                  (uint32_t)d->tune.wait_polls, 1u};
+                  (uint32_t)d->tune.wait_polls, 1u, &d->state.p->zero_exists};
 }
 
 // ------------------------------------------------------------------------------------------
@@ -514,10 +516,6 @@ void graph_key(const b2d_dedup* d, const RoundState* rs_dev, std::vector<uint64_
             (uint64_t)d->sm_count, (uint64_t)d->list, (uint64_t)d->warp_bands});
 }
 
-// Device work of one checkpoint on `s`.  `rs_dev` is where the kernels read this checkpoint's
-// RoundState; with `upload` the host copy (pinned) is copied there first.  `managed`: a batch
-// clears the DevState, writes the RoundState and reads the DevState back for all its handles
-// at once (and may have hashed the leaves already: `skip_leaves`).
 DiffArgs diff_args(b2d_dedup* d, const RoundState* rs_dev) {
   MapView m;
   map_view(d, m);
@@ -525,7 +523,7 @@ DiffArgs diff_args(b2d_dedup* d, const RoundState* rs_dev) {
   return DiffArgs{static_cast<const uint8_t*>(d->data), d->data_len, d->chunk_size, d->n, d->N, d->D, 0, 0,
                   d->tree.p, d->push.p, m, &ds->status, &ds->meta, d->first_list.p, d->shift_list.p, d->region_off.p,
                   d->sprev.p, d->skey.p, d->hist.p, d->bucket_start.p, d->partial.p, d->partial2.p, d->diff.p, rs_dev,
-                  d->list ? d->n - 1u : 0u, d->list};
+                  d->list ? d->n - 1u : 0u, d->list, &ds->stamps, nullptr, nullptr, 0u};
 }
 
 ForestArgs forest_args(b2d_dedup* d, const RoundState* rs_dev) {
@@ -533,18 +531,21 @@ ForestArgs forest_args(b2d_dedup* d, const RoundState* rs_dev) {
   map_view(d, m);
   DevState* ds = d->state.p;
   return ForestArgs{d->tree.p, d->lab.p, d->leaflab.p, d->push.p, m, &ds->status, &ds->zero_exists, d->dupflag.p,
-                    d->n, d->N, d->D, 0, d->kind, 0, rs_dev};
+                    d->n, d->N, d->D, 0, d->kind, 0, rs_dev, nullptr};
 }
 
-int enqueue_checkpoint(b2d_dedup* d, cudaStream_t s, RoundState* rs_dev, bool upload, bool timing, bool skip_leaves,
+// Device work of one checkpoint on `s`.  `rs_dev` is where the kernels read this checkpoint's
+// RoundState; `captured` launches take it from the pinned copy at every replay, others carry it as
+// a launch argument.  `managed`: a batch clears the DevState, writes the RoundState and reads the
+// DevState back for all its handles at once (and may have hashed the leaves already:
+// `skip_leaves`); else the last launch writes the DevState to the host.
+int enqueue_checkpoint(b2d_dedup* d, cudaStream_t s, RoundState* rs_dev, bool captured, bool skip_leaves,
                        bool managed = false, bool skip_diff = false, bool skip_forest = false) {
   DevState* ds = d->state.p;
-  bool zero_probe_skipped = false;
   if (!managed) {
-    B2D_CU(cudaMemsetAsync(ds, 0, sizeof(DevState), s));
-    if (upload) B2D_CU(cudaMemcpyAsync(rs_dev, d->round_h.p, sizeof(RoundState), cudaMemcpyHostToDevice, s));
+    round_init_kernel<<<1, 64, 0, s>>>(ds, captured ? d->round_h.p : nullptr, *d->round_h.p);
+    B2D_CU(cudaGetLastError());
   }
-  if (timing) B2D_CU(record_timing(d->ev[0], s));
   // dedup_data_baseline (:13-259) / dedup_data (:261-509)
   if (!skip_leaves) {
     const LeafArgs la = leaf_args(d, rs_dev);
@@ -552,51 +553,47 @@ int enqueue_checkpoint(b2d_dedup* d, cudaStream_t s, RoundState* rs_dev, bool up
     if (leaf_path < 0) return B2D_ERR_CUDA;
     d->leaf_tma = leaf_path == 1;
   }
-  if (timing) B2D_CU(record_timing(d->ev[3], s));
+  ForestArgs fa = forest_args(d, rs_dev);
+  fa.stamp = &ds->stamps.forest;
   if (d->list) {
     // list approach: no tree; per-chunk labels and region flags (src/list_approach.cpp:41-71)
-    B2D_CU(launch_list_label(forest_args(d, rs_dev), d->sm_count, s));
+    B2D_CU(launch_list_label(fa, d->sm_count, s));
   } else if (!skip_forest) {
-    const ForestArgs fa = forest_args(d, rs_dev);
     B2D_CU(launch_forest(fa, 1, s, d->sm_count, d->warp_bands));
-    // the zero-digest probe matters to baselines only; launches issued one by one for a single
-    // handle skip it otherwise (a captured graph or a batch keeps it: it serves both kinds)
-    if (managed || d->use_graph || d->round_h.p->baseline) B2D_CU(launch_zero_exists(&ds->zero_exists, rs_dev, s));
-    else zero_probe_skipped = true;
+    fa.stamp = nullptr;
     B2D_CU(launch_forest(fa, 2, s, d->sm_count, d->warp_bands));
   }
-  if (timing) B2D_CU(record_timing(d->ev[1], s));
   // collect_diff (:511-710; list approach src/list_approach.cpp:79-257, single-chunk regions in
   // chunk order, chunk indices in the diff); a batch may assemble all its handles' diffs in
   // shared launches
   if (!skip_diff) {
-    B2D_CU(launch_collect_diff(diff_args(d, rs_dev), d->bcap, d->sm_count, s));
+    DiffArgs da = diff_args(d, rs_dev);
+    if (!managed) {
+      da.state = reinterpret_cast<const uint32_t*>(ds);
+      da.state_host = reinterpret_cast<uint32_t*>(d->state_h.p);
+      da.state_words = sizeof(DevState) / 4;
+    }
+    B2D_CU(launch_collect_diff(da, d->bcap, d->sm_count, s));
   }
-  if (timing) B2D_CU(record_timing(d->ev[2], s));
-  if (!managed) B2D_CU(cudaMemcpyAsync(d->state_h.p, d->state.p, sizeof(DevState), cudaMemcpyDeviceToHost, s));
-  // kernels only (memsets and copies are not counted)
+  // kernels only
+  d->launches = (managed ? 0 : 1) + (skip_leaves ? 0 : 1) + (skip_diff ? 0 : DIFF_LAUNCHES);
   if (d->list)
-    d->launches = (skip_leaves ? 0 : 1) + 1 + (skip_diff ? 0 : DIFF_LAUNCHES);
-  else
-    d->launches = (skip_leaves ? 0 : 1) +
-                  (skip_forest ? 0 : forest_launch_count(d->n, d->D, 1, d->warp_bands) +
-                                         forest_launch_count(d->n, d->D, 2, d->warp_bands) +
-                                         (zero_probe_skipped ? 0 : 1)) +
-                  (skip_diff ? 0 : DIFF_LAUNCHES);
+    d->launches += 1;
+  else if (!skip_forest)
+    d->launches += forest_launch_count(d->n, d->D, 1, d->warp_bands) + forest_launch_count(d->n, d->D, 2, d->warp_bands);
   return B2D_OK;
 }
 
 int finish_checkpoint(b2d_dedup* d, bool advance, bool timing) {
   const DevState& st = *d->state_h.p;
   if (timing) {
-    const float ms_dedup = elapsed_ms(d->ev[0], d->ev[1]);
-    const float ms_gather = elapsed_ms(d->ev[1], d->ev[2]);
-    const float ms_leaf = elapsed_ms(d->ev[0], d->ev[3]);
-    d->phase[0] = ms_leaf * 1e-3;
-    d->phase[1] = (ms_dedup - ms_leaf) * 1e-3;
-    d->phase[2] = ms_gather * 1e-3;
-    d->timers[1] = ms_dedup * 1e-3;
-    d->timers[2] = ms_gather * 1e-3;
+    const Stamps& t = st.stamps;
+    const unsigned long long forest = t.forest ? t.forest : t.diff;   // one chunk: no forest launches
+    d->phase[0] = (double)(forest - t.begin) * 1e-9;
+    d->phase[1] = (double)(t.diff - forest) * 1e-9;
+    d->phase[2] = (double)(t.end - t.diff) * 1e-9;
+    d->timers[1] = (double)(t.diff - t.begin) * 1e-9;
+    d->timers[2] = d->phase[2];
   }
   d->timers[3] = 0;
   int rc = status_code(st.status);
@@ -631,12 +628,11 @@ int do_checkpoint(b2d_dedup* d, const void* d_data, uint64_t len, bool make_base
   RoundState* rs_dev = &d->state.p->round;
   if (!d->use_graph) {
     d->timers[0] = secs(t0, clk::now());
-    rc = enqueue_checkpoint(d, d->stream, rs_dev, true, true, false);
+    rc = enqueue_checkpoint(d, d->stream, rs_dev, false, false);
     if (rc) return rc;
     B2D_CU(cudaStreamSynchronize(d->stream));
     return finish_checkpoint(d, advance, true);
   }
-  // the round state lives in DevState, which the enqueue clears first: upload after the clear
   std::vector<uint64_t> key;
   graph_key(d, rs_dev, key);
   if (!d->graph_exec || key != d->graph_key) {
@@ -648,7 +644,7 @@ int do_checkpoint(b2d_dedup* d, const void* d_data, uint64_t len, bool make_base
     // cannot be captured) and launched on the caller's
     cudaGraph_t g = nullptr;
     B2D_CU(cudaStreamBeginCapture(d->cap_stream, cudaStreamCaptureModeThreadLocal));
-    rc = enqueue_checkpoint(d, d->cap_stream, rs_dev, true, d->graph_timing, false);
+    rc = enqueue_checkpoint(d, d->cap_stream, rs_dev, true, false);
     const cudaError_t ce = cudaStreamEndCapture(d->cap_stream, &g);
     if (rc) {
       if (g) cudaGraphDestroy(g);
@@ -1021,8 +1017,6 @@ int read_file(const std::string& path, std::vector<uint8_t>& out) {
 //   -> batch_collect_kernel + one read-back of every handle's DevState.
 // Each handle's output is what its own b2d_checkpoint_device would produce.
 // ------------------------------------------------------------------------------------------
-static_assert(sizeof(DevState) % 4 == 0, "DevState is cleared word by word");
-
 __global__ void batch_init_kernel(DevState* const* states, const RoundState* rounds, uint32_t count,
                                   unsigned int* queues, uint32_t ngroups, DevStatus* bst) {
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1501,8 +1495,8 @@ int batch_launch(b2d_batch* b, b2d_dedup* const* hs, const void* const* data, co
         // nothing of a tree handle runs in a branch when its leaves, forest and diff are all
         // shared; a list handle labels and assembles its diff here
         if (seg_forest && skip_leaves && !d->list) continue;
-        const int r = enqueue_checkpoint(d, s, &d->state.p->round, false, false, skip_leaves, true,
-                                         seg_diff && !d->list, seg_forest);
+        const int r = enqueue_checkpoint(d, s, &d->state.p->round, true, skip_leaves, true, seg_diff && !d->list,
+                                         seg_forest);
         if (r != B2D_OK) erc = r;
         launches += d->launches;
       }
@@ -1510,14 +1504,12 @@ int batch_launch(b2d_batch* b, b2d_dedup* const* hs, const void* const* data, co
       cap_err(cudaStreamWaitEvent(main, b->side_ev[j], 0));
     }
     if (seg_forest && erc == B2D_OK) {
-      // phase 1 steps, the zero-digest probe, phase 2 steps: each over every handle at once
+      // phase 1 steps, then phase 2 steps: each over every handle at once
       for (size_t q = 0; q < flaunch.size() && erc == B2D_OK; q++) {
         if (flaunch[q].phase != 1) continue;
         cap_err(launch_forest_seg(fseg[q], 1, flaunch[q].kind, flaunch[q].ctas, main));
         launches++;
       }
-      cap_err(launch_zero_exists_seg(reinterpret_cast<const ForestArgs*>(B + L.fargs), count, main));
-      launches++;
       for (size_t q = 0; q < flaunch.size() && erc == B2D_OK; q++) {
         if (flaunch[q].phase != 2) continue;
         cap_err(launch_forest_seg(fseg[q], 2, flaunch[q].kind, flaunch[q].ctas, main));
@@ -1681,8 +1673,6 @@ int b2d_create(uint32_t chunk_size, int hash_kind, b2d_dedup** out) {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&d->sm_count, cudaDevAttrMultiProcessorCount, d->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&d->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&d->cap_stream, cudaStreamNonBlocking);
-    for (auto& ev : d->ev)
-      if (e == cudaSuccess) e = cudaEventCreate(&ev);
     if (e != cudaSuccess) {
       delete d;
       return cuda_status(e);

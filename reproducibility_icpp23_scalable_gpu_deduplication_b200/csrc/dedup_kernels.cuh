@@ -49,6 +49,7 @@ struct LeafArgs {
   uint32_t wait_polls;   // 0: the barrier waits' normal bound; else give up after this many
                          // non-blocking polls (a test of the give-up path)
   uint32_t one;          // 1: the MD5 rounds' multiply-add factor (md5_pre_add)
+  int* zero_exists;      // baseline: set when a chunk's digest is all zero (it is then in the map)
 };
 
 struct ForestArgs {
@@ -58,13 +59,14 @@ struct ForestArgs {
   uint8_t* push;
   MapView map;
   DevStatus* st;
-  const int* zero_exists;   // baseline: does the all-zero digest exist in the map
+  int* zero_exists;         // baseline: does the all-zero digest exist in the map (phase 1 adds parents')
   uint8_t* dupflag;         // per chunk, set by the leaf stage, cleared by phase 1
   uint32_t n, N, D;         // chunks, nodes, deepest level
   uint32_t cur;
   int kind;
   int baseline;
   const RoundState* rs;
+  unsigned long long* stamp;   // where the launch's first thread records its start (null: nowhere)
 };
 
 // Per-checkpoint sizes, computed on the device so no host round trip is needed mid-checkpoint.
@@ -78,7 +80,14 @@ struct DevMeta {
   unsigned long long first_off, count_off, shift_off, data_off;  // byte offsets in the device diff buffer
   unsigned long long map_size;      // occupied map slots after this checkpoint
   uint32_t done;         // CTAs of the shifted-root pass that have finished (the last lays the diff out)
-  uint32_t pad;
+  uint32_t emitted;      // CTAs of the emit pass that have finished
+};
+
+// Global-timer readings (ns) of one checkpoint: after the state was cleared, at the start of the
+// forest (or list label) pass and of the diff assembly, and when the diff is complete.  Events
+// between the kernels kept each from starting while the one before it ends.
+struct Stamps {
+  unsigned long long begin, forest, diff, end;
 };
 
 struct DiffArgs {
@@ -105,6 +114,12 @@ struct DiffArgs {
                           // n - 1, so leaf heap indices become chunk indices; tree: 0)
   int node_order;         // region lists in node order (the list approach, whose regions are single
                           // leaves) instead of the tree's level-descending order
+  Stamps* stamps;         // diff and end are recorded here
+  // the emit pass's last CTA copies the checkpoint's device state to the host (pinned memory):
+  // `state_words` words from `state` to `state_host` (null: left to the caller)
+  const uint32_t* state;
+  uint32_t* state_host;
+  uint32_t state_words;
 };
 
 // Programmatic dependent launch (sm_90 and later).  The forest and diff-assembly kernels of one
@@ -115,6 +130,11 @@ struct DiffArgs {
 __device__ __forceinline__ void griddep_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ unsigned long long device_time_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
 }
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
@@ -225,9 +245,7 @@ struct ForestSeg {
   uint32_t n;
 };
 cudaError_t launch_forest_seg(const ForestSeg& s, int phase, int kind, uint32_t ctas, cudaStream_t stream);
-cudaError_t launch_zero_exists_seg(const ForestArgs* args, uint32_t n, cudaStream_t stream);
 int forest_launch_count(uint32_t n, uint32_t D, int phase, int warp_mask = B2D_WARP_BANDS);
-cudaError_t launch_zero_exists(int* flag, const RoundState* rs, cudaStream_t stream);
 // bcap: bucket capacity the scratch was sized for (>= rs->buckets of every checkpoint run).
 cudaError_t launch_collect_diff(const DiffArgs& a, uint32_t bcap, int sm_count, cudaStream_t stream);
 constexpr int DIFF_LAUNCHES = 4;   // kernels of one launch_collect_diff

@@ -51,6 +51,10 @@ constexpr uint8_t NONE_LABEL = 5;         // node index beyond the tree
 __device__ __forceinline__ uint8_t push_flag(uint8_t label) {
   return label == SHIFT_DUPL ? PUSH_SHIFT : (label == FIRST_OCUR ? PUSH_FIRST : PUSH_NONE);
 }
+// the start of the pass (dedup_kernels.cuh, Stamps), for the launch that is asked to record it
+__device__ __forceinline__ void stamp_start(const ForestArgs& a) {
+  if (a.stamp && blockIdx.x == 0 && threadIdx.x == 0) *a.stamp = device_time_ns();
+}
 // region-root flag of node x, at position x + 1: 2 bits per node, 16 nodes per word (gather.cu
 // reads them)
 __device__ __forceinline__ void push_set(uint8_t* push, uint64_t x, uint32_t flag) {
@@ -63,6 +67,7 @@ __device__ __forceinline__ void push_set(uint8_t* push, uint64_t x, uint32_t fla
 __device__ __noinline__ void insert_first_parent(const ForestArgs& a, uint32_t x, const Digest& d) {
   const uint32_t height = a.D - node_level(x);
   const unsigned long long v = ((unsigned long long)(1u + height) << 32) | x;
+  if (digest_zero(d)) *a.zero_exists = 1;
   const MapRef ref = map_insert(a.map, d, v, a.cur, a.st);
   if (ref.found && !ref.inserted) map_merge_current(a.map, ref.slot, v, a.cur);
 }
@@ -80,6 +85,9 @@ __device__ __noinline__ void insert_first_parent(const ForestArgs& a, uint32_t x
 constexpr int FF_GROUP = 2;
 __device__ __forceinline__ void insert_first_parents(const ForestArgs& a, const uint32_t (&x)[FF_GROUP],
                                                      const Digest (&d)[FF_GROUP], uint32_t cnt) {
+#pragma unroll
+  for (int j = 0; j < FF_GROUP; j++)
+    if ((uint32_t)j < cnt && digest_zero(d[j])) *a.zero_exists = 1;
 #if B2D_FF_GROUPED
   Key128 k[FF_GROUP];
   unsigned long long pv[FF_GROUP];
@@ -412,6 +420,7 @@ __device__ __forceinline__ void forest_first_body(const ForestArgs& a, uint32_t 
 __global__ void __launch_bounds__(FAST_THREADS, B2D_FF_MINB) forest_first_kernel(ForestArgs a0, uint32_t in,
                                                                                   uint32_t nbands) {
   griddep_enter();
+  stamp_start(a0);
   const ForestArgs a = with_round(a0);
   for (uint32_t bid = blockIdx.x; bid < nbands; bid += gridDim.x) {
     forest_first_body(a, bid, in);
@@ -788,6 +797,7 @@ static bool wq_fits(uint32_t ntasks, uint32_t grid) {
 __global__ void __launch_bounds__(WB_THREADS, B2D_WB1_MINB)
     forest_warp1_kernel(ForestArgs a0, uint32_t ntasks, uint32_t queue) {
   griddep_enter();
+  stamp_start(a0);
   B2D_WARP_INSERT_BUFFERS
   B2D_WARP_QUEUE_BUFFERS
   const ForestArgs a = with_round(a0);
@@ -944,6 +954,7 @@ __device__ __forceinline__ void forest_band_body(const ForestArgs& a, uint32_t b
 template <int PHASE>
 __global__ void __launch_bounds__(FOREST_THREADS) forest_band_kernel(ForestArgs a0, uint32_t top, uint32_t bot) {
   griddep_enter();
+  stamp_start(a0);
   forest_band_body<PHASE>(with_round(a0), blockIdx.x, top, bot);
 }
 template <int PHASE>
@@ -1005,10 +1016,11 @@ static uint32_t resident_ctas(K kernel) {
   return (uint32_t)nb;
 }
 
-cudaError_t launch_forest(const ForestArgs& a, int phase, cudaStream_t stream, int sm_count, int warp_mask) {
+cudaError_t launch_forest(const ForestArgs& args, int phase, cudaStream_t stream, int sm_count, int warp_mask) {
   static const uint32_t res_first = resident_ctas(forest_first_kernel);
   static const uint32_t res_fast = resident_ctas(forest_fast_kernel<2>);
   std::vector<ForestStep> steps;
+  ForestArgs a = args;
   if (warp_bands(a.n, a.D, phase, warp_mask)) {
     static const uint32_t res_w1 = resident_ctas(forest_warp1_kernel);
     static const uint32_t res_w2 = resident_ctas(forest_warp2_kernel);
@@ -1021,6 +1033,7 @@ cudaError_t launch_forest(const ForestArgs& a, int phase, cudaStream_t stream, i
     cudaError_t e = phase == 1 ? launch_dependent(forest_warp1_kernel, grid, WB_THREADS, 0, stream, a, ntasks, queue)
                                : launch_dependent(forest_warp2_kernel, grid, WB_THREADS, 0, stream, a, ntasks, queue);
     if (e != cudaSuccess) return e;
+    a.stamp = nullptr;
     forest_steps_from(a.D, a.D - levels, a.N, phase, steps);
   } else {
     forest_steps(a.D, a.N, phase, steps);
@@ -1038,6 +1051,7 @@ cudaError_t launch_forest(const ForestArgs& a, int phase, cudaStream_t stream, i
                      : launch_dependent(forest_band_kernel<2>, st.ctas, FOREST_THREADS, 0, stream, a, st.p0, st.p1);
     }
     if (e != cudaSuccess) return e;
+    a.stamp = nullptr;
   }
   return cudaSuccess;
 }
@@ -1067,32 +1081,6 @@ cudaError_t launch_forest_seg(const ForestSeg& s, int phase, int kind, uint32_t 
   return cudaGetLastError();
 }
 
-__device__ __forceinline__ void zero_exists_kernel_body(int* flag, const RoundState* rs) {
-  if (!rs->baseline) return;   // only the baseline tests the stale zero digest
-  Digest z;
-  z.w[0] = z.w[1] = z.w[2] = z.w[3] = 0u;
-  const MapView m = rs->map;
-  *flag = map_find(m, z) <= m.cap ? 1 : 0;
-}
-__global__ void zero_exists_kernel(int* flag, const RoundState* rs) {
-  griddep_enter();
-  zero_exists_kernel_body(flag, rs);
-}
-
-__global__ void zero_exists_seg(const ForestArgs* args, uint32_t n) {
-  const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-  if (h < n) zero_exists_kernel_body(const_cast<int*>(args[h].zero_exists), args[h].rs);   // the flag this step sets
-}
-
-cudaError_t launch_zero_exists_seg(const ForestArgs* args, uint32_t n, cudaStream_t stream) {
-  zero_exists_seg<<<(n + 127) / 128, 128, 0, stream>>>(args, n);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_zero_exists(int* flag, const RoundState* rs, cudaStream_t stream) {
-  return launch_dependent(zero_exists_kernel, 1, 1, 0, stream, flag, rs);
-}
-
 // List approach (src/list_approach.cpp:41-71): a changed chunk whose digest was new is a first
 // occurrence, one whose digest existed is a shifted duplicate.  The leaf stage labelled every
 // changed chunk of a digest shared within this checkpoint a first occurrence and flagged it;
@@ -1101,6 +1089,7 @@ cudaError_t launch_zero_exists(int* flag, const RoundState* rs, cudaStream_t str
 // region flags for the diff are set per chunk (its leaf), and the duplicate flags are cleared.
 __global__ void list_label_kernel(ForestArgs a0) {
   griddep_enter();
+  stamp_start(a0);
   const ForestArgs a = with_round(a0);
   for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < a.n; c += (uint64_t)gridDim.x * blockDim.x) {
     uint8_t lab = a.leaflab[c];

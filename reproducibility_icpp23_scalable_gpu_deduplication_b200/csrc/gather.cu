@@ -145,6 +145,7 @@ __device__ __forceinline__ void diff_count_body(const DiffArgs& a, uint32_t bid,
 }
 __global__ void __launch_bounds__(COMPACT_THREADS) diff_count_kernel(DiffArgs a0, uint32_t bcap) {
   griddep_enter();
+  if (blockIdx.x == 0 && threadIdx.x == 0) a0.stamps->diff = device_time_ns();
   diff_count_body(with_round(a0), blockIdx.x, gridDim.x, bcap);
 }
 __global__ void __launch_bounds__(COMPACT_THREADS) diff_count_seg(SegGrid s) {
@@ -707,6 +708,22 @@ template <bool ALIGNED>
 __global__ void __launch_bounds__(EMIT_THREADS) diff_emit_kernel(DiffArgs a0, uint32_t bcap, uint32_t ranges) {
   griddep_enter();
   diff_emit_body<ALIGNED>(with_round(a0), blockIdx.x, gridDim.x, bcap, ranges);
+  // the last CTA hands the checkpoint's state to the host: a copy enqueued behind this kernel
+  // took 10 us of a small checkpoint
+  if (a0.state_host == nullptr) return;
+  __shared__ uint32_t last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&a0.meta->emitted, 1u) == gridDim.x - 1u;
+    if (last) {
+      a0.stamps->end = device_time_ns();
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (last)
+    for (uint32_t i = threadIdx.x; i < a0.state_words; i += blockDim.x) a0.state_host[i] = __ldcg(a0.state + i);
 }
 template <bool ALIGNED>
 __global__ void __launch_bounds__(EMIT_THREADS) diff_emit_seg(SegGrid s) {

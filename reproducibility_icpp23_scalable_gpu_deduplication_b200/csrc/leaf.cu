@@ -51,7 +51,10 @@ __device__ __forceinline__ void leaf_finish(const LeafArgs& a, uint32_t chunk, c
   }
   if (fixed) {
     label = FIXED_DUPL;
-    if (a.baseline) a.tree[leaf] = d;
+    if (a.baseline) {
+      a.tree[leaf] = d;
+      *a.zero_exists = 1;
+    }
   }
   a.leaflab[chunk] = label;
 }
@@ -138,6 +141,7 @@ __device__ __forceinline__ void pipe_issue(const LeafArgs& a, LeafPipe& p, uint3
     leaf_finish(a, chunk, d, old);
     return;
   }
+  if (fixed) *a.zero_exists = 1;   // a baseline's zero digest
   p.c_on = true;
   p.c_fixed = fixed;
   p.c_chunk = chunk;
@@ -161,7 +165,7 @@ __device__ __forceinline__ Digest prior_digest(const LeafArgs& a, uint64_t chunk
 }
 
 __global__ void leaf_generic_kernel(LeafArgs a0, uint32_t c_begin, uint32_t c_end) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  griddep_enter();
   const LeafArgs a = with_round(a0);
   for (uint64_t c = (uint64_t)c_begin + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < c_end;
        c += (uint64_t)gridDim.x * blockDim.x) {
@@ -315,7 +319,7 @@ template <int U, int KIND>
 __global__ void __launch_bounds__((TMA_CONSUMER_WARPS + 1) * 32)
     leaf_tma_kernel(const __grid_constant__ CUtensorMap tmap, LeafArgs a0, uint32_t nfull, uint32_t S,
                     uint32_t stages) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  griddep_enter();
   const LeafArgs a = with_round(a0);
   constexpr uint32_t R = 32u * TMA_CONSUMER_WARPS;
   constexpr uint32_t STAGE_BYTES = R * U;
@@ -579,8 +583,7 @@ static cudaError_t launch_tma(const CUtensorMap& map, const LeafArgs& a, uint32_
   uint32_t grid = (uint32_t)sm_count * (uint32_t)(tune.ctas_per_sm > 0 ? tune.ctas_per_sm : (four ? 4 : 3));
   if (grid > ntiles) grid = ntiles;
   if (grid == 0) grid = 1;
-  kern<<<grid, (TMA_CONSUMER_WARPS + 1) * 32, smem, stream>>>(map, a, nfull, S, stages);
-  return cudaGetLastError();
+  return launch_dependent(kern, grid, (TMA_CONSUMER_WARPS + 1) * 32, smem, stream, map, a, nfull, S, stages);
 }
 
 static bool encode_map(const LeafArgs& a, int U, CUtensorMap& map) {
@@ -685,8 +688,7 @@ int launch_leaves(const LeafArgs& a, int sm_count, const LeafTuning& tune, cudaS
   const uint64_t cap = (uint64_t)sm_count * 16u;
   if (blocks > cap) blocks = cap;
   if (blocks == 0) blocks = 1;
-  leaf_generic_kernel<<<(uint32_t)blocks, threads, 0, stream>>>(a, 0u, a.n);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  return launch_dependent(leaf_generic_kernel, (uint32_t)blocks, threads, 0, stream, a, 0u, a.n) == cudaSuccess ? 0 : -1;
 }
 
 }  // namespace b2d
