@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "../../include/b200dedup.h"
+#include "bulk.cuh"
 #include "dedup_kernels.cuh"
 #include "hash.cuh"
 #include "map.cuh"
@@ -119,7 +120,7 @@ __global__ void hash_chunks_kernel(int kind, const uint8_t* data, uint64_t len, 
 struct DevState {
   DevStatus status;
   int zero_exists;
-  unsigned int pad;
+  int lost_any;
   DevMeta meta;
   StraddleInfo straddle;
   RoundState round;
@@ -203,6 +204,8 @@ struct b2d_dedup {
   PinnedBuf<RoundState> round_h;   // this checkpoint's RoundState, read by a graph's first kernel
   const void* data = nullptr;      // buffer of the current checkpoint
   uint32_t bcap = 0;               // source-checkpoint bucket capacity of the scratch
+  bool bulk = false;               // the current checkpoint is a baseline built in bulk (bulk.cu)
+  BulkPlan plan;
   cudaGraphExec_t graph_exec = nullptr;
   std::vector<uint64_t> graph_key;
   PinnedBuf<uint8_t> diff_h;
@@ -313,28 +316,31 @@ int map_view(b2d_dedup* d, MapView& m) {
 }
 
 // a fresh map of `cap` slots (+ the special slot) on the handle's stream
-int map_alloc(b2d_dedup* d, uint64_t cap, void** out) {
+int map_alloc(b2d_dedup* d, uint64_t cap, void** out, bool clear = true) {
   cudaMemPool_t pool = map_pool(d->device);
   if (!pool) return B2D_ERR_CUDA;
   const auto t0 = std::chrono::high_resolution_clock::now();
   B2D_CU(cudaMallocFromPoolAsync(out, MAP_SLOT_BYTES * (cap + 1), pool, d->stream));
   d->map_alloc_s += secs(t0, std::chrono::high_resolution_clock::now());
   // all keys EMPTY, all values all-ones (the extra slot: absent)
-  B2D_CU(cudaMemsetAsync(*out, 0xff, MAP_SLOT_BYTES * (cap + 1), d->stream));
+  if (clear) B2D_CU(cudaMemsetAsync(*out, 0xff, MAP_SLOT_BYTES * (cap + 1), d->stream));
   return B2D_OK;
 }
 
-int map_reset(b2d_dedup* d, uint64_t cap) {
+// an empty table; `clear` false: one whose slots a bulk build will write, all but the extra one
+int map_reset(b2d_dedup* d, uint64_t cap, bool clear = true) {
   if (!d->map_mem || d->map_cap != cap) {
     void* fresh = nullptr;
-    int rc = map_alloc(d, cap, &fresh);
+    int rc = map_alloc(d, cap, &fresh, clear);
     if (rc) return rc;
     if (d->map_mem) cudaFreeAsync(d->map_mem, d->stream);
     d->map_mem = fresh;
     d->map_cap = cap;
-  } else {
+  } else if (clear) {
     B2D_CU(cudaMemsetAsync(d->map_mem, 0xff, MAP_SLOT_BYTES * (cap + 1), d->stream));
   }
+  if (!clear)
+    B2D_CU(cudaMemsetAsync(static_cast<uint8_t*>(d->map_mem) + MAP_SLOT_BYTES * cap, 0xff, MAP_SLOT_BYTES, d->stream));
   B2D_CU(d->map_size.reserve(1));
   B2D_CU(cudaMemsetAsync(d->map_size.p, 0, sizeof(unsigned long long), d->stream));
   d->map_size_host = 0;
@@ -396,6 +402,8 @@ int map_ensure(b2d_dedup* d) {
   return B2D_OK;
 }
 
+uint64_t diff_capacity(const b2d_dedup* d) { return 64 + 16ull * d->n + (uint64_t)d->n * d->chunk_size; }
+
 int status_code(const DevStatus& st) {
   switch (st.error) {
     case DERR_NONE: return B2D_OK;
@@ -411,7 +419,7 @@ LeafArgs leaf_args(const b2d_dedup* d, const RoundState* rs_dev) {
   const MapView m = map_at(d->map_mem, d->map_cap, d->map_size.p);
   return LeafArgs{static_cast<const uint8_t*>(d->data), d->data_len, d->chunk_size, d->n, d->kind, 0, 0,
                   d->tree.p, d->leaflab.p, d->dupflag.p, m, &d->state.p->status, rs_dev,
-                  (uint32_t)d->tune.wait_polls, 1u, &d->state.p->zero_exists};
+                  (uint32_t)d->tune.wait_polls, 1u, &d->state.p->zero_exists, d->bulk};
 }
 
 // ------------------------------------------------------------------------------------------
@@ -432,7 +440,9 @@ int check_checkpoint(const b2d_dedup* d, const void* d_data, uint64_t len, bool 
   return B2D_OK;
 }
 
-int prepare_checkpoint(b2d_dedup* d, const void* d_data, uint64_t len, bool make_baseline) {
+// `own_launches`: the checkpoint's kernels are launched one by one for this handle alone (no
+// captured graph, which serves baselines and increments alike, and no batch)
+int prepare_checkpoint(b2d_dedup* d, const void* d_data, uint64_t len, bool make_baseline, bool own_launches) {
   const int vrc = check_checkpoint(d, d_data, len, make_baseline);
   if (vrc) return vrc;
   const uint64_t nc = (len + d->chunk_size - 1) / d->chunk_size;
@@ -462,12 +472,15 @@ int prepare_checkpoint(b2d_dedup* d, const void* d_data, uint64_t len, bool make
     B2D_CU(cudaMemsetAsync(d->push.p, 0, d->push.n, d->stream));
   }
   if (baseline) {
-    int rc = map_reset(d, map_capacity(2ull * d->N, d->map_max_load, d->map_headroom));
+    const uint64_t cap = map_capacity(2ull * d->N, d->map_max_load, d->map_headroom);
+    d->bulk = own_launches && bulk_plan(d->n, cap, d->list, diff_capacity(d), d->plan);
+    int rc = map_reset(d, cap, !d->bulk);
     if (rc) return rc;
     d->baseline_id = d->current_id;
     // the list approach starts a baseline from an all-zero digest list (src/list_approach.cpp:865-869)
-    if (d->list) B2D_CU(cudaMemsetAsync(d->tree.p + (d->n - 1u), 0, sizeof(Digest) * (size_t)d->n, d->stream));
+    if (d->list && !d->bulk) B2D_CU(cudaMemsetAsync(d->tree.p + (d->n - 1u), 0, sizeof(Digest) * (size_t)d->n, d->stream));
   } else {
+    d->bulk = false;
     int rc = map_ensure(d);
     if (rc) return rc;
   }
@@ -487,7 +500,7 @@ int prepare_checkpoint(b2d_dedup* d, const void* d_data, uint64_t len, bool make
   B2D_CU(d->bucket_start.reserve(bcap));
   B2D_CU(d->partial.reserve((size_t)1184 * bcap));
   B2D_CU(d->partial2.reserve(3 * COMPACT_GRID));
-  B2D_CU(d->diff.reserve(64 + 16ull * d->n + (uint64_t)d->n * d->chunk_size));
+  B2D_CU(d->diff.reserve(diff_capacity(d)));
   B2D_CU(d->state.reserve(1));
   B2D_CU(d->state_h.reserve(1));
   B2D_CU(d->round_h.reserve(1));
@@ -526,12 +539,51 @@ DiffArgs diff_args(b2d_dedup* d, const RoundState* rs_dev) {
                   d->list ? d->n - 1u : 0u, d->list, &ds->stamps, nullptr, nullptr, 0u};
 }
 
+// the bulk build's counters and marks lie in `sprev`, its overflow list in `skey`: both are free
+// until the diff is assembled, like the diff buffer, which holds its entries
+uint32_t* bulk_scratch(b2d_dedup* d, uint64_t off) { return d->sprev.p + off / 4; }
+BulkArgs bulk_args(b2d_dedup* d) {
+  BulkArgs b{};
+  DevState* ds = d->state.p;
+  const BulkPlan& p = d->plan;
+  b.tree = d->tree.p;
+  b.leaflab = d->leaflab.p;
+  map_view(d, b.map);
+  b.st = &ds->status;
+  b.n = d->n;
+  b.N = d->N;
+  b.D = d->D;
+  b.cur = d->current_id;
+  b.kind = d->kind;
+  b.list = d->list;
+  b.first_node = d->list ? d->n - 1u : 0u;
+  b.count = p.count;
+  b.ranges = p.ranges;
+  b.buckets = p.buckets;
+  b.start = bulk_scratch(d, p.start);
+  b.alloc = bulk_scratch(d, p.alloc);
+  b.alloc1 = bulk_scratch(d, p.alloc1);
+  b.tile_beg = bulk_scratch(d, p.tile_beg);
+  b.over_count = bulk_scratch(d, p.over_count);
+  b.lost = bulk_scratch(d, p.lost);
+  b.overflow = d->skey.p;
+  b.key1 = reinterpret_cast<Key128*>(d->diff.p + p.key1);
+  b.key2 = reinterpret_cast<Key128*>(d->diff.p + p.key2);
+  b.id1 = reinterpret_cast<uint32_t*>(d->diff.p + p.id1);
+  b.id2 = reinterpret_cast<uint32_t*>(d->diff.p + p.id2);
+  b.lost_any = &ds->lost_any;
+  b.zero_exists = &ds->zero_exists;
+  b.stamp = &ds->stamps.forest;
+  return b;
+}
+
 ForestArgs forest_args(b2d_dedup* d, const RoundState* rs_dev) {
   MapView m;
   map_view(d, m);
   DevState* ds = d->state.p;
   return ForestArgs{d->tree.p, d->lab.p, d->leaflab.p, d->push.p, m, &ds->status, &ds->zero_exists, d->dupflag.p,
-                    d->n, d->N, d->D, 0, d->kind, 0, rs_dev, nullptr};
+                    d->n, d->N, d->D, 0, d->kind, 0, rs_dev, nullptr,
+                    d->bulk ? bulk_scratch(d, d->plan.lost) : nullptr, &ds->lost_any, 0};
 }
 
 // Device work of one checkpoint on `s`.  `rs_dev` is where the kernels read this checkpoint's
@@ -542,6 +594,7 @@ ForestArgs forest_args(b2d_dedup* d, const RoundState* rs_dev) {
 int enqueue_checkpoint(b2d_dedup* d, cudaStream_t s, RoundState* rs_dev, bool captured, bool skip_leaves,
                        bool managed = false, bool skip_diff = false, bool skip_forest = false) {
   DevState* ds = d->state.p;
+  if (d->bulk) B2D_CU(cudaMemsetAsync(d->sprev.p, 0, d->plan.zeroed_bytes, s));
   if (!managed) {
     round_init_kernel<<<1, 64, 0, s>>>(ds, captured ? d->round_h.p : nullptr, *d->round_h.p);
     B2D_CU(cudaGetLastError());
@@ -555,11 +608,16 @@ int enqueue_checkpoint(b2d_dedup* d, cudaStream_t s, RoundState* rs_dev, bool ca
   }
   ForestArgs fa = forest_args(d, rs_dev);
   fa.stamp = &ds->stamps.forest;
+  uint32_t bulk_launches = 0;
+  if (d->bulk) {   // inner digests and the map; phase 1 has nothing left to do
+    B2D_CU(launch_bulk(bulk_args(d), d->sm_count, s, &bulk_launches));
+    fa.stamp = nullptr;
+  }
   if (d->list) {
     // list approach: no tree; per-chunk labels and region flags (src/list_approach.cpp:41-71)
     B2D_CU(launch_list_label(fa, d->sm_count, s));
   } else if (!skip_forest) {
-    B2D_CU(launch_forest(fa, 1, s, d->sm_count, d->warp_bands));
+    if (!d->bulk) B2D_CU(launch_forest(fa, 1, s, d->sm_count, d->warp_bands));
     fa.stamp = nullptr;
     B2D_CU(launch_forest(fa, 2, s, d->sm_count, d->warp_bands));
   }
@@ -577,10 +635,12 @@ int enqueue_checkpoint(b2d_dedup* d, cudaStream_t s, RoundState* rs_dev, bool ca
   }
   // kernels only
   d->launches = (managed ? 0 : 1) + (skip_leaves ? 0 : 1) + (skip_diff ? 0 : DIFF_LAUNCHES);
+  d->launches += bulk_launches;
   if (d->list)
     d->launches += 1;
   else if (!skip_forest)
-    d->launches += forest_launch_count(d->n, d->D, 1, d->warp_bands) + forest_launch_count(d->n, d->D, 2, d->warp_bands);
+    d->launches += (d->bulk ? 0 : forest_launch_count(d->n, d->D, 1, d->warp_bands)) +
+                   forest_launch_count(d->n, d->D, 2, d->warp_bands);
   return B2D_OK;
 }
 
@@ -623,7 +683,7 @@ int finish_checkpoint(b2d_dedup* d, bool advance, bool timing) {
 int do_checkpoint(b2d_dedup* d, const void* d_data, uint64_t len, bool make_baseline, bool advance) {
   using clk = std::chrono::high_resolution_clock;
   const auto t0 = clk::now();
-  int rc = prepare_checkpoint(d, d_data, len, make_baseline);
+  int rc = prepare_checkpoint(d, d_data, len, make_baseline, !d->use_graph);
   if (rc) return rc;
   RoundState* rs_dev = &d->state.p->round;
   if (!d->use_graph) {
@@ -1251,7 +1311,7 @@ int batch_launch(b2d_batch* b, b2d_dedup* const* hs, const void* const* data, co
     d->stream = b->stream;
     const bool mb = make_baseline && make_baseline[i];
     any_baseline = any_baseline || mb || d->current_id == 0;
-    rc = prepare_checkpoint(d, data[i], lens[i], mb);
+    rc = prepare_checkpoint(d, data[i], lens[i], mb, false);
     d->stream = keep;
     if (rc) {
       if (rcs) rcs[i] = rc;

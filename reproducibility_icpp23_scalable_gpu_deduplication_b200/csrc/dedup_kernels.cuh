@@ -50,6 +50,7 @@ struct LeafArgs {
                          // non-blocking polls (a test of the give-up path)
   uint32_t one;          // 1: the MD5 rounds' multiply-add factor (md5_pre_add)
   int* zero_exists;      // baseline: set when a chunk's digest is all zero (it is then in the map)
+  int bulk;              // a baseline built in bulk (bulk.cu): hash and label only, no map
 };
 
 struct ForestArgs {
@@ -67,6 +68,15 @@ struct ForestArgs {
   int baseline;
   const RoundState* rs;
   unsigned long long* stamp;   // where the launch's first thread records its start (null: nowhere)
+  // a baseline built in bulk (bulk.cu; null otherwise): bit per node that lost its map entry to
+  // another parent, and whether any did (read into lost_seen)
+  const uint32_t* lost;
+  const int* lost_any;
+  int lost_seen;
+  // the arguments as launched (kernel parameters or global memory).  The out-of-line paths take
+  // this pointer: handed a reference to the kernel's working copy, they forced that copy, and every
+  // use of it, into local memory.
+  const ForestArgs* self;
 };
 
 // Per-checkpoint sizes, computed on the device so no host round trip is needed mid-checkpoint.
@@ -165,6 +175,8 @@ __device__ __forceinline__ ForestArgs with_round(const ForestArgs& p) {
   a.cur = p.rs->cur;
   a.baseline = (int)p.rs->baseline;
   a.map = p.rs->map;
+  a.lost_seen = p.lost ? *p.lost_any : 0;
+  a.self = &p;
   return a;
 }
 __device__ __forceinline__ DiffArgs with_round(const DiffArgs& p) {

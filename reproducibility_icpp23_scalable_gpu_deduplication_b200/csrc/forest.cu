@@ -64,7 +64,8 @@ __device__ __forceinline__ void push_set(uint8_t* push, uint64_t x, uint32_t fla
 
 // phase-1 parent insert, priority 1 + height (:133, :390).  The rare heavy paths (hashing,
 // map probes) are kept out of line so the label folds stay small in the instruction cache.
-__device__ __noinline__ void insert_first_parent(const ForestArgs& a, uint32_t x, const Digest& d) {
+__device__ __noinline__ void insert_first_parent(const ForestArgs* self, uint32_t x, const Digest& d) {
+  const ForestArgs a = with_round(*self);
   const uint32_t height = a.D - node_level(x);
   const unsigned long long v = ((unsigned long long)(1u + height) << 32) | x;
   if (digest_zero(d)) *a.zero_exists = 1;
@@ -105,19 +106,21 @@ __device__ __forceinline__ void insert_first_parents(const ForestArgs& a, const 
 #else
 #pragma unroll
   for (int j = 0; j < FF_GROUP; j++)
-    if ((uint32_t)j < cnt) insert_first_parent(a, x[j], d[j]);
+    if ((uint32_t)j < cnt) insert_first_parent(a.self, x[j], d[j]);
 #endif
 }
 
-__device__ __noinline__ void hash_first_parent(const ForestArgs& a, uint32_t x) {
+__device__ __noinline__ void hash_first_parent(const ForestArgs* self, uint32_t x) {
+  const ForestArgs a = with_round(*self);
   const Digest d = hash_pair(a.kind, a.tree[2u * x + 1u], a.tree[2u * x + 2u]);
   a.tree[x] = d;
-  insert_first_parent(a, x, d);
+  insert_first_parent(self, x, d);
 }
 
 // two shifted children: the parent is a shifted duplicate only if its digest is already known;
 // the baseline tests the stale (zero) digest instead (:202 vs :459)
-__device__ __noinline__ uint8_t shift_pair(const ForestArgs& a, uint32_t x) {
+__device__ __noinline__ uint8_t shift_pair(const ForestArgs* self, uint32_t x) {
+  const ForestArgs a = with_round(*self);
   const uint32_t l = 2u * x + 1u, r = 2u * x + 2u;
   bool exists;
   if (a.baseline) {
@@ -136,7 +139,8 @@ __device__ __noinline__ uint8_t shift_pair(const ForestArgs& a, uint32_t x) {
 // baseline "Insert entries" (:218-224) for a parent that is not a first occurrence (those were
 // hashed and inserted by phase 1 with a lower priority, so re-inserting them changes nothing):
 // hash, insert with priority 64 + height
-__device__ __noinline__ void baseline_parent(const ForestArgs& a, uint32_t x) {
+__device__ __noinline__ void baseline_parent(const ForestArgs* self, uint32_t x) {
+  const ForestArgs a = with_round(*self);
   const Digest d = hash_pair(a.kind, a.tree[2u * x + 1u], a.tree[2u * x + 2u]);
   a.tree[x] = d;
   const uint32_t height = a.D - node_level(x);
@@ -145,11 +149,31 @@ __device__ __noinline__ void baseline_parent(const ForestArgs& a, uint32_t x) {
   if (ref.found && !ref.inserted) map_merge_current(a.map, ref.slot, v, a.cur);
 }
 
+// A parent of a baseline built in bulk (bulk.cu), whose digest is hashed and in the map already
+// under a first-occurrence parent's priority.  One that is no first occurrence and owns its entry
+// takes its real priority, 64 + height; a first occurrence that lost its entry to another parent
+// (a shallower or lower one of equal digest) becomes the owner.
+__device__ __noinline__ void bulk_settle(const ForestArgs* self, uint32_t x, bool first) {
+  const ForestArgs a = with_round(*self);
+  const uint64_t slot = map_find(a.map, a.tree[x]);
+  if (slot > a.map.cap) {
+    set_error(a.st, DERR_INTERNAL, 12);
+    return;
+  }
+  const uint32_t height = a.D - node_level(x);
+  const unsigned long long as_first = map_pack(((unsigned long long)(1u + height) << 32) | x, a.cur);
+  unsigned long long* v = map_val(a.map, slot);
+  if (!first)
+    atomicCAS(v, as_first, map_pack(((unsigned long long)(64u + height) << 32) | x, a.cur));
+  else if (map_node(a.map, slot) < a.n - 1u)
+    atomicExch(v, as_first);
+}
+
 template <int PHASE>
 __device__ __forceinline__ uint8_t forest_node(const ForestArgs& a, uint32_t x, uint8_t ll, uint8_t rl) {
   if constexpr (PHASE == 1) {
     if (ll == FIRST_OCUR && rl == FIRST_OCUR) {
-      hash_first_parent(a, x);
+      hash_first_parent(a.self, x);
       return FIRST_OCUR;
     }
     return DONE;
@@ -161,11 +185,18 @@ __device__ __forceinline__ uint8_t forest_node(const ForestArgs& a, uint32_t x, 
       if (pl) push_set(a.push, 2u * x + 1u, pl);
       if (pr) push_set(a.push, 2u * x + 2u, pr);
     } else if (ll == SHIFT_DUPL) {
-      out = shift_pair(a, x);
+      out = shift_pair(a.self, x);
     } else {
       out = ll;   // FIXED, FIRST or DONE pairs keep the label
     }
-    if (a.baseline && out != FIRST_OCUR) baseline_parent(a, x);
+    if (a.baseline) {
+      if (out != FIRST_OCUR) {
+        if (a.lost) bulk_settle(a.self, x, false);
+        else baseline_parent(a.self, x);
+      } else if (a.lost_seen && ((a.lost[x >> 5] >> (x & 31u)) & 1u)) {
+        bulk_settle(a.self, x, true);
+      }
+    }
     return out;
   }
 }
@@ -417,7 +448,7 @@ __device__ __forceinline__ void forest_first_body(const ForestArgs& a, uint32_t 
 #ifndef B2D_FOREST_PERSIST
 #define B2D_FOREST_PERSIST 1
 #endif
-__global__ void __launch_bounds__(FAST_THREADS, B2D_FF_MINB) forest_first_kernel(ForestArgs a0, uint32_t in,
+__global__ void __launch_bounds__(FAST_THREADS, B2D_FF_MINB) forest_first_kernel(const __grid_constant__ ForestArgs a0, uint32_t in,
                                                                                   uint32_t nbands) {
   griddep_enter();
   stamp_start(a0);
@@ -523,7 +554,7 @@ __device__ __forceinline__ void forest_fast_body(const ForestArgs& a, uint32_t b
   }
 }
 template <int PHASE>
-__global__ void __launch_bounds__(FAST_THREADS, B2D_FAST_MINB) forest_fast_kernel(ForestArgs a0, uint32_t in,
+__global__ void __launch_bounds__(FAST_THREADS, B2D_FAST_MINB) forest_fast_kernel(const __grid_constant__ ForestArgs a0, uint32_t in,
                                                                                   uint32_t nbands) {
   griddep_enter();
   const ForestArgs a = with_round(a0);
@@ -795,7 +826,7 @@ static bool wq_fits(uint32_t ntasks, uint32_t grid) {
 }
 
 __global__ void __launch_bounds__(WB_THREADS, B2D_WB1_MINB)
-    forest_warp1_kernel(ForestArgs a0, uint32_t ntasks, uint32_t queue) {
+    forest_warp1_kernel(const __grid_constant__ ForestArgs a0, uint32_t ntasks, uint32_t queue) {
   griddep_enter();
   stamp_start(a0);
   B2D_WARP_INSERT_BUFFERS
@@ -846,7 +877,7 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB1_MINB)
     warp1_task(a, t, lane, lab32[t * 32u + lane], wi);
 }
 __global__ void __launch_bounds__(WB_THREADS, B2D_WB2_MINB)
-    forest_warp2_kernel(ForestArgs a0, uint32_t ntasks, uint32_t queue) {
+    forest_warp2_kernel(const __grid_constant__ ForestArgs a0, uint32_t ntasks, uint32_t queue) {
   griddep_enter();
   B2D_WARP_QUEUE_BUFFERS
   const ForestArgs a = with_round(a0);
@@ -952,7 +983,7 @@ __device__ __forceinline__ void forest_band_body(const ForestArgs& a, uint32_t b
   }
 }
 template <int PHASE>
-__global__ void __launch_bounds__(FOREST_THREADS) forest_band_kernel(ForestArgs a0, uint32_t top, uint32_t bot) {
+__global__ void __launch_bounds__(FOREST_THREADS) forest_band_kernel(const __grid_constant__ ForestArgs a0, uint32_t top, uint32_t bot) {
   griddep_enter();
   stamp_start(a0);
   forest_band_body<PHASE>(with_round(a0), blockIdx.x, top, bot);
@@ -1087,7 +1118,7 @@ cudaError_t launch_forest_seg(const ForestSeg& s, int phase, int kind, uint32_t 
 // in the reference's sequential order the lowest chunk index inserts first, which is the map
 // entry's owner after the leaf stage's minimum, so the others become shifted duplicates.  The
 // region flags for the diff are set per chunk (its leaf), and the duplicate flags are cleared.
-__global__ void list_label_kernel(ForestArgs a0) {
+__global__ void list_label_kernel(const __grid_constant__ ForestArgs a0) {
   griddep_enter();
   stamp_start(a0);
   const ForestArgs a = with_round(a0);

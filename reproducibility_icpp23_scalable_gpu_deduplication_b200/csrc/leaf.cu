@@ -29,12 +29,32 @@ __device__ __forceinline__ void flag_shared(const LeafArgs& a, uint32_t chunk, u
   }
 }
 
+// A leaf of a baseline built in bulk (bulk.cu): its digest, and the label it has unless the build
+// finds it to be a copy.  `copy`: equal to the chunk before it, so a shifted duplicate at any rate.
+__device__ __forceinline__ void bulk_leaf(const LeafArgs& a, uint32_t chunk, const Digest& d, bool copy) {
+  const bool zero = digest_zero(d);
+  a.tree[a.n - 1u + chunk] = d;
+  a.leaflab[chunk] = zero ? FIXED_DUPL : copy ? SHIFT_DUPL : FIRST_OCUR;
+  if (zero) *a.zero_exists = 1;
+}
+// a warp's 32 consecutive chunks; all lanes call it
+__device__ __forceinline__ void bulk_finish(const LeafArgs& a, uint32_t chunk, bool valid, const Digest& d) {
+  Digest left;
+#pragma unroll
+  for (int q = 0; q < 4; q++) left.w[q] = __shfl_up_sync(0xffffffffu, d.w[q], 1);
+  if (valid) bulk_leaf(a, chunk, d, (threadIdx.x & 31u) != 0u && digest_eq(d, left));
+}
+
 // Per-leaf decision, same order of tests as the reference:
 //  baseline:    insert, then compare with the (fresh, all-zero) tree entry
 //  incremental: compare with the prior digest first; FIXED leaves skip the insert because
 //               their digest is already present from the checkpoint that stored it.
 __device__ __forceinline__ void leaf_finish(const LeafArgs& a, uint32_t chunk, const Digest& d, const Digest& old) {
   const uint32_t leaf = a.n - 1u + chunk;
+  if (a.bulk) {
+    bulk_leaf(a, chunk, d, false);
+    return;
+  }
   uint8_t label = DONE;
   const bool fixed = a.baseline ? digest_zero(d) : digest_eq(d, old);
   if (a.baseline || !fixed) {
@@ -161,7 +181,7 @@ __device__ __forceinline__ void pipe_drain(const LeafArgs& a, LeafPipe& p) {
 __device__ __forceinline__ Digest prior_digest(const LeafArgs& a, uint64_t chunk) {
   Digest z;
   z.w[0] = z.w[1] = z.w[2] = z.w[3] = 0u;
-  return a.baseline ? z : a.tree[a.n - 1u + chunk];
+  return a.baseline || a.bulk ? z : a.tree[a.n - 1u + chunk];
 }
 
 __global__ void leaf_generic_kernel(LeafArgs a0, uint32_t c_begin, uint32_t c_end) {
@@ -401,7 +421,9 @@ __global__ void __launch_bounds__((TMA_CONSUMER_WARPS + 1) * 32)
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);
     }
-    if (PIPE) {
+    if (a.bulk) {
+      bulk_finish(a, chunk, valid, finish_segments<KIND>(mm, md, a.cs));
+    } else if (PIPE) {
       pipe_flags(a, pipe);
       pipe_claim(a, pipe);
       if (valid) pipe_issue(a, pipe, chunk, finish_segments<KIND>(mm, md, a.cs), old);
@@ -409,7 +431,7 @@ __global__ void __launch_bounds__((TMA_CONSUMER_WARPS + 1) * 32)
       leaf_finish(a, chunk, finish_segments<KIND>(mm, md, a.cs), old);
     }
   }
-  if (PIPE) pipe_drain(a, pipe);
+  if (PIPE && !a.bulk) pipe_drain(a, pipe);
 }
 
 // Batched form: one persistent launch hashes the chunks of many buffers.  The producer lane
