@@ -16,9 +16,11 @@
 #include <cstring>
 #include <fstream>
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <new>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/b200dedup.h"
@@ -122,7 +124,6 @@ struct DevState {
   int zero_exists;
   int lost_any;
   DevMeta meta;
-  StraddleInfo straddle;
   RoundState round;
   Stamps stamps;
 };
@@ -151,6 +152,7 @@ using namespace b2d;
 // node: 2 bytes per byte of a 4 GiB buffer at 128-byte chunks), at load 0.25 after the
 // baseline, and the table grows only once its entries pass 2N (after about a hundred
 // checkpoints that each change 1% of the chunks).
+constexpr uint32_t STAGE_PIECES = 16;   // upload()'s ring
 constexpr double MAP_HEADROOM = 1.5;
 constexpr double MAP_GROWTH = 2.0;
 
@@ -220,7 +222,10 @@ struct b2d_dedup {
   DevBuf<uint32_t> r_offs, r_partial;      // r_offs: offsets, region starts, source starts, trees
   DevBuf<unsigned long long> r_cum, r_total;
   DevBuf<uint8_t> r_diff;
-  PinnedBuf<uint8_t> r_stage;
+  DevBuf<StraddleInfo> r_straddle;
+  PinnedBuf<uint8_t> r_hdr;                // headers of device diffs
+  PinnedBuf<uint8_t> r_stage;              // upload()'s ring, and when each piece's copy is done
+  cudaEvent_t stage_ev[STAGE_PIECES] = {};
 
   ~b2d_dedup();
 };
@@ -270,6 +275,8 @@ b2d_dedup::~b2d_dedup() {
       }
     }
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
+    for (auto& e : stage_ev)
+      if (e) cudaEventDestroy(e);
     if (own_stream) cudaStreamDestroy(own_stream);
     if (cap_stream) cudaStreamDestroy(cap_stream);
   }
@@ -307,7 +314,7 @@ uint64_t handle_bytes(const b2d_dedup* d) {
          buf_bytes(d->state) + buf_bytes(d->r_node_list) + buf_bytes(d->r_rep) + buf_bytes(d->r_dist) +
          buf_bytes(d->r_mflag) + buf_bytes(d->r_flag) +
          buf_bytes(d->r_offs) + buf_bytes(d->r_partial) + buf_bytes(d->r_cum) + buf_bytes(d->r_total) +
-         buf_bytes(d->r_diff);
+         buf_bytes(d->r_diff) + buf_bytes(d->r_straddle);
 }
 
 int map_view(b2d_dedup* d, MapView& m) {
@@ -841,38 +848,105 @@ bool parse_hdr(const uint8_t* b, uint64_t size, HostHdr& h) {
   return h.data_off <= size && h.cs > 0 && h.datalen > 0;
 }
 
+// Headers of device-resident diffs idx .. idx - count + 1, into hdr[0 .. count): one small kernel and
+// one wait for up to RESTART_HEADERS of them.
+int read_device_headers(b2d_dedup* d, const void* const* ddiffs, const uint64_t* sizes, int idx, int count,
+                        HostHdr* hdr) {
+  B2D_CU(d->r_hdr.reserve(32 * RESTART_HEADERS));
+  for (int k = 0; k < count;) {
+    RestartHeaders q{};
+    for (; q.count < RESTART_HEADERS && k + (int)q.count < count; q.count++) {
+      const int i = idx - k - (int)q.count;
+      if (!ddiffs[i] || sizes[i] < 32) return B2D_ERR_FORMAT;
+      q.diff[q.count] = static_cast<const uint8_t*>(ddiffs[i]);
+    }
+    B2D_CU(launch_restart_headers(q, d->r_hdr.p, d->stream));
+    B2D_CU(cudaStreamSynchronize(d->stream));
+    for (uint32_t j = 0; j < q.count; j++, k++)
+      if (!parse_hdr(d->r_hdr.p + 32 * j, sizes[idx - k], hdr[k])) return B2D_ERR_FORMAT;
+  }
+  return B2D_OK;
+}
+
+// Copies host memory to the device on the handle's stream.  Page-locked memory goes straight;
+// other memory passes through a ring of page-locked pieces that several threads fill while earlier
+// pieces are on their way.  One thread's memcpy (10 GB/s) held the copy to a fifth of what the bus
+// carries, and each diff was staged whole before its copy began.
+struct Upload {
+  uint8_t* dst;
+  const uint8_t* src;
+  uint64_t bytes;
+};
+constexpr uint64_t STAGE_PIECE = 2ull << 20;
+constexpr uint32_t STAGE_THREADS = 8;   // divides STAGE_PIECES
+static_assert(STAGE_PIECES % STAGE_THREADS == 0, "a ring slot belongs to one thread");
+int upload(b2d_dedup* d, const std::vector<Upload>& copies) {
+  std::vector<Upload> pieces;
+  for (const Upload& c : copies) {
+    cudaPointerAttributes pa;
+    const bool pinned = cudaPointerGetAttributes(&pa, c.src) == cudaSuccess && pa.type == cudaMemoryTypeHost;
+    if (!pinned) (void)cudaGetLastError();
+    if (pinned) {
+      B2D_CU(cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyHostToDevice, d->stream));
+    } else {
+      for (uint64_t o = 0; o < c.bytes; o += STAGE_PIECE)
+        pieces.push_back(Upload{c.dst + o, c.src + o, std::min(STAGE_PIECE, c.bytes - o)});
+    }
+  }
+  if (pieces.empty()) return B2D_OK;
+  B2D_CU(d->r_stage.reserve(STAGE_PIECE * std::min<uint64_t>(pieces.size(), STAGE_PIECES)));
+  for (auto& e : d->stage_ev)
+    if (!e) B2D_CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  // thread t of T (a power of two) fills pieces t, t + T, ...; piece p's ring slot is p modulo the
+  // ring, so a slot belongs to one thread.  The copies are enqueued by the threads, which the
+  // per-thread default stream, another stream in each, does not allow.
+  const uint32_t most = d->stream == cudaStreamPerThread
+                            ? 1u
+                            : std::min(STAGE_THREADS, std::max(1u, std::thread::hardware_concurrency()));
+  uint32_t T = 1;
+  while (2 * T <= std::min<uint64_t>(most, pieces.size())) T *= 2;
+  std::atomic<int> err{0};
+  auto work = [&](uint32_t t) {
+    cudaError_t e = cudaSetDevice(d->device);
+    for (size_t p = t; p < pieces.size() && e == cudaSuccess && err.load() == 0; p += T) {
+      const uint32_t slot = (uint32_t)(p % STAGE_PIECES);
+      uint8_t* s = d->r_stage.p + STAGE_PIECE * slot;
+      e = cudaEventSynchronize(d->stage_ev[slot]);   // the slot's last copy; at once if it had none
+      if (e != cudaSuccess) break;
+      std::memcpy(s, pieces[p].src, pieces[p].bytes);
+      e = cudaMemcpyAsync(pieces[p].dst, s, pieces[p].bytes, cudaMemcpyHostToDevice, d->stream);
+      if (e == cudaSuccess) e = cudaEventRecord(d->stage_ev[slot], d->stream);
+    }
+    if (e != cudaSuccess) err.store(cuda_status(e));
+  };
+  std::vector<std::thread> threads;
+  uint32_t started = 1;
+  try {
+    threads.reserve(T);
+    for (; started < T; started++) threads.emplace_back(work, started);
+  } catch (...) {   // no more threads: their pieces are filled here
+  }
+  work(0);
+  for (uint32_t t = started; t < T; t++) work(t);
+  for (auto& t : threads) t.join();
+  return err.load();
+}
+
+// One restart: the chain's headers, then the main diff and a window of older ones expanded together
+// and resolved by a walk, then further windows.  Device diffs are read where they lie; host diffs
+// are copied to the device a window at a time.
 int do_restart(b2d_dedup* d, void* d_out, uint64_t len, const uint8_t* const* diffs, const uint64_t* sizes,
                uint32_t count, uint32_t id, const void* const* ddiffs = nullptr) {
   using clk = std::chrono::high_resolution_clock;
   const auto t0 = clk::now();
   if (!d_out || (!diffs && !ddiffs) || !sizes || id >= count) return B2D_ERR_ARG;
-  // device-resident diffs: the host reads only their headers and repeat tables (small copies)
-  std::vector<std::vector<uint8_t>> hmeta;
-  std::vector<const uint8_t*> hptr;
-  if (ddiffs) {
-    hmeta.resize(count);
-    hptr.assign(count, nullptr);
-    // the same chain walk as below: from `id` down while the index is not below the last ref_id
-    for (int idx = (int)id; idx >= 0; idx--) {
-      if (!ddiffs[idx] || sizes[idx] < 32) return B2D_ERR_FORMAT;
-      uint8_t hdr[32];
-      B2D_CU(cudaMemcpy(hdr, ddiffs[idx], 32, cudaMemcpyDeviceToHost));
-      HostHdr hh;
-      if (!parse_hdr(hdr, sizes[idx], hh)) return B2D_ERR_FORMAT;
-      // header, then the repeat table right behind it (not at its offset in the diff: the
-      // first-occurrence list in between can be tens of megabytes)
-      auto& m = hmeta[idx];
-      m.resize(32 + 8ull * hh.P);
-      std::memcpy(m.data(), hdr, 32);
-      if (hh.P) B2D_CU(cudaMemcpy(m.data() + 32, static_cast<const uint8_t*>(ddiffs[idx]) + hh.count_off,
-                                  8ull * hh.P, cudaMemcpyDeviceToHost));
-      hptr[idx] = m.data();
-      if (idx - 1 < (int)hh.ref_id) break;
-    }
-    diffs = hptr.data();
-  }
   HostHdr h;
-  if (!parse_hdr(diffs[id], sizes[id], h)) return B2D_ERR_FORMAT;
+  if (ddiffs) {
+    const int hrc = read_device_headers(d, ddiffs, sizes, (int)id, 1, &h);
+    if (hrc) return hrc;
+  } else if (!parse_hdr(diffs[id], sizes[id], h)) {
+    return B2D_ERR_FORMAT;
+  }
   // every diff the checkpoint path writes has ref_id <= chkpt_id == its position in the list;
   // a list that breaks this names no chain to walk, so it is rejected before any device work
   if (h.ref_id > h.chkpt_id || h.chkpt_id != id) return B2D_ERR_FORMAT;
@@ -881,170 +955,186 @@ int do_restart(b2d_dedup* d, void* d_out, uint64_t len, const uint8_t* const* di
   if (nc > 0x7fffffffull) return B2D_ERR_FORMAT;
   const uint32_t n = (uint32_t)nc, N = 2u * n - 1u;
   // the chain, newest first: from `id` down while the index is not below the last ref_id
-  std::vector<int> chain;
-  std::vector<HostHdr> hdrs;
-  uint64_t max_size = 0, max_list = 0, max_ids = 0;
+  std::vector<HostHdr> hdrs{h};   // of diffs id, id - 1, ...
   {
+    std::vector<HostHdr> ahead;   // device headers read together, of diffs id - hdrs.size() on down
+    size_t used = 0;
     uint32_t ref = h.ref_id;
-    for (int idx = (int)id; idx >= 0 && idx >= (int)ref; idx--) {
+    for (int idx = (int)id - 1; idx >= 0 && idx >= (int)ref; idx--) {
       HostHdr hh;
-      if (!parse_hdr(diffs[idx], sizes[idx], hh)) return B2D_ERR_FORMAT;
-      if (idx != (int)id) ref = hh.ref_id;
-      chain.push_back(idx);
+      if (ddiffs) {
+        if (used == ahead.size()) {
+          ahead.resize((size_t)(idx - (int)ref + 1));
+          used = 0;
+          const int hrc = read_device_headers(d, ddiffs, sizes, idx, idx - (int)ref + 1, ahead.data());
+          if (hrc) return hrc;
+        }
+        hh = ahead[used++];
+      } else if (!parse_hdr(diffs[idx], sizes[idx], hh)) {
+        return B2D_ERR_FORMAT;
+      }
+      ref = hh.ref_id;
       hdrs.push_back(hh);
-      max_size = std::max<uint64_t>(max_size, sizes[idx]);
-      max_list = std::max<uint64_t>(max_list, std::max<uint64_t>(hh.F, hh.S));
-      max_ids = std::max<uint64_t>(max_ids, (uint64_t)hh.chkpt_id + 1);
     }
   }
-  // window slots: older diffs resolved per walk.  Device diffs are read where they lie, so a
-  // window holds several (bounded by the slots' memory); host diffs pass one at a time through
-  // one device copy.
-  const uint64_t older = chain.size() - 1;
-  uint32_t W = 1;
-  if (ddiffs && older > 1) {
-    const uint64_t per_slot = 13ull * n;   // dist u32 + rep uint2 + a flag byte per chunk
-    W = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(older, RESTART_WINDOW),
-                                     std::max<uint64_t>(1, RESTART_SLOT_BYTES / per_slot));
+  // Sets of diffs expanded together: the main diff with a window of older ones, then windows.  A
+  // window's diffs share a chunk size (the walk copies from all of them); its slots' memory and, for
+  // host diffs, their copies are bounded.
+  const uint64_t per_slot = 13ull * n;   // dist u32 + rep uint2 + a flag byte per chunk
+  const uint64_t window = std::min<uint64_t>(RESTART_WINDOW, std::max<uint64_t>(1, RESTART_SLOT_BYTES / per_slot));
+  struct Set {
+    size_t beg, end;   // of hdrs
+  };
+  std::vector<Set> sets;
+  uint64_t max_bytes = 0, max_lists = 0, max_cum = 0, max_count = 0;
+  auto room = [&](size_t k) { return (sizes[id - k] + 31u) / 16u * 16u; };   // a diff's device copy
+  auto plan = [&](uint64_t win, uint64_t byte_limit) {
+    sets.clear();
+    max_bytes = max_lists = max_cum = max_count = 0;
+    for (size_t k = 0; k < hdrs.size();) {
+      Set q{k, k};
+      uint64_t bytes = 0, lists = 0, cums = 0;
+      const size_t older0 = k == 0 ? 1 : k;
+      while (q.end < hdrs.size()) {
+        const size_t j = q.end;
+        if (j > older0 && (j - older0 >= win || hdrs[j].cs != hdrs[older0].cs)) break;
+        if (j > q.beg && bytes + room(j) > byte_limit) break;
+        bytes += room(j);
+        lists += 2ull * hdrs[j].F + 4ull * hdrs[j].S;
+        cums += (uint64_t)hdrs[j].chkpt_id + 1u;
+        q.end++;
+      }
+      max_bytes = std::max(max_bytes, bytes);
+      max_lists = std::max(max_lists, lists);
+      max_cum = std::max(max_cum, cums);
+      max_count = std::max<uint64_t>(max_count, q.end - q.beg);
+      sets.push_back(q);
+      k = q.end;
+    }
+  };
+  plan(window, ddiffs ? ~0ull : RESTART_SLOT_BYTES);
+  if (!ddiffs && d->r_diff.reserve(max_bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    plan(1, 0);   // one diff at a time
+    B2D_CU(d->r_diff.reserve(max_bytes));
   }
   B2D_CU(d->r_node_list.reserve(n));
   B2D_CU(d->r_mflag.reserve(n));
-  B2D_CU(d->r_dist.reserve((uint64_t)n * W));
-  B2D_CU(d->r_rep.reserve((uint64_t)n * W));
-  B2D_CU(d->r_flag.reserve((uint64_t)n * W));
-  B2D_CU(d->r_offs.reserve(4 * std::max<uint64_t>(max_list, 1)));
-  B2D_CU(d->r_partial.reserve(SCAN_GRID));
-  B2D_CU(d->r_cum.reserve(max_ids));
-  B2D_CU(d->r_total.reserve(1));
-  if (!ddiffs) B2D_CU(d->r_diff.reserve(max_size + 16));   // device diffs are read where they lie
+  B2D_CU(d->r_dist.reserve((uint64_t)n * max_count));
+  B2D_CU(d->r_rep.reserve((uint64_t)n * max_count));
+  B2D_CU(d->r_flag.reserve((uint64_t)n * max_count));
+  B2D_CU(d->r_offs.reserve(std::max<uint64_t>(max_lists, 1)));
+  B2D_CU(d->r_partial.reserve(2 * SCAN_GRID * max_count));
+  B2D_CU(d->r_cum.reserve(max_cum));
+  B2D_CU(d->r_total.reserve(2 * max_count));
+  B2D_CU(d->r_straddle.reserve(max_count));
   B2D_CU(d->state.reserve(1));
   B2D_CU(d->state_h.reserve(1));
-  if (!ddiffs) B2D_CU(d->r_stage.grow(max_size + 16 + 8 * max_ids));
   B2D_CU(cudaMemsetAsync(d->state.p, 0, sizeof(DevState), d->stream));
   d->launches = 0;
   double copy_time = 0;
-  auto slot = [&](uint32_t k) {
-    RestartSlot sl;
-    sl.dist = d->r_dist.p + (uint64_t)n * k;
-    sl.rep = d->r_rep.p + (uint64_t)n * k;
-    sl.flag = d->r_flag.p + (uint64_t)n * k;
-    return sl;
-  };
 
-  RestartArgs a{};
-  a.n = n;
-  a.N = N;
-  a.out = static_cast<uint8_t*>(d_out);
-  a.out_len = h.datalen;
-  a.node_list = d->r_node_list.p;
-  a.mflag = d->r_mflag.p;
-  const uint64_t lcap = std::max<uint64_t>(max_list, 1);
-  a.offs = d->r_offs.p;
-  a.rstart = d->r_offs.p + lcap;
-  a.pstart = d->r_offs.p + 2 * lcap;
-  a.rtree = d->r_offs.p + 3 * lcap;
-  a.partial = d->r_partial.p;
-  a.total = d->r_total.p;
-  a.st = &d->state.p->status;
-  // list diffs name chunks; the restart kernels work on leaf heap indices (leaf of chunk c = n-1+c)
-  a.id_bias = d->list ? n - 1u : 0u;
   RestartWalk w{};
   w.main_cur = h.chkpt_id;
   w.n = n;
   w.N = N;
-  w.out = a.out;
+  w.out = static_cast<uint8_t*>(d_out);
   w.out_len = h.datalen;
-  w.node_list = a.node_list;
-  w.mflag = a.mflag;
-  w.st = a.st;
-  uint32_t wcount = 0;
-  auto flush = [&](bool last) -> cudaError_t {
-    if (wcount == 0) return cudaSuccess;
-    w.count = wcount;
-    w.last = last;
-    cudaError_t e = launch_restart_walk(w, d->sm_count, d->stream);
-    d->launches += 1;
-    w.dense = 1;   // a walk that is not the last wrote every chunk's NodeID
-    wcount = 0;
-    return e;
-  };
-
-  for (size_t k = 0; k < chain.size(); k++) {
-    const int idx = chain[k];
-    const HostHdr& hh = hdrs[k];
-    const bool is_main = k == 0;
-    // host diffs: one copy into the device scratch, placed so the data section is 16-byte
-    // aligned; pinned (page-locked) host diffs are copied straight from where they are, others
-    // go through the handle's pinned staging buffer.  The repeat table's running counts are
-    // uploaded beside them.
-    const uint32_t delta = (uint32_t)((16u - (hh.data_off & 15u)) & 15u);
-    const uint64_t ncum = (uint64_t)hh.chkpt_id + 1;
-    bool pinned = ddiffs != nullptr;
-    if (!ddiffs) {
-      cudaPointerAttributes pa;
-      pinned = cudaPointerGetAttributes(&pa, diffs[idx]) == cudaSuccess && pa.type == cudaMemoryTypeHost;
-      if (!pinned) (void)cudaGetLastError();
-    }
-    if (!pinned) B2D_CU(cudaStreamSynchronize(d->stream));
+  w.node_list = d->r_node_list.p;
+  w.mflag = d->r_mflag.p;
+  w.st = &d->state.p->status;
+  for (const Set& q : sets) {
+    const bool first = q.beg == 0, last = q.end == hdrs.size();
+    const uint32_t members = (uint32_t)(q.end - q.beg);
+    RestartSet rs{};
+    rs.count = members;
+    uint32_t* lists = d->r_offs.p;
+    unsigned long long* cum = d->r_cum.p;
+    uint64_t at = 0;   // in r_diff
     const auto c0 = clk::now();
-    const uint8_t* src = ddiffs ? static_cast<const uint8_t*>(ddiffs[idx]) : diffs[idx];
-    if (!pinned) {
-      memcpy(d->r_stage.p + delta, diffs[idx], sizes[idx]);
-      src = d->r_stage.p + delta;
+    std::vector<Upload> copies;
+    for (uint32_t m = 0; m < members; m++) {
+      const HostHdr& hh = hdrs[q.beg + m];
+      const size_t idx = id - (q.beg + m);
+      RestartArgs& a = rs.a[m];
+      if (ddiffs) {
+        a.diff = static_cast<const uint8_t*>(ddiffs[idx]);
+      } else {
+        // placed so that the data section is 16-byte aligned
+        uint8_t* dst = d->r_diff.p + at + (16u - (hh.data_off & 15u)) % 16u;
+        copies.push_back(Upload{dst, diffs[idx], sizes[idx]});
+        a.diff = dst;
+        at += room(q.beg + m);
+      }
+      a.diff_size = sizes[idx];
+      a.first_off = hh.first_off;
+      a.count_off = hh.count_off;
+      a.shift_off = hh.shift_off;
+      a.data_off = hh.data_off;
+      a.F = hh.F;
+      a.P = hh.P;
+      a.S = hh.S;
+      a.cur_id = hh.chkpt_id;
+      a.datalen = hh.datalen;
+      a.cs = hh.cs;
+      a.n = n;
+      a.N = N;
+      a.is_main = first && m == 0;
+      a.out = w.out;
+      a.out_len = h.datalen;
+      a.node_list = d->r_node_list.p;
+      a.mflag = d->r_mflag.p;
+      a.slot.dist = d->r_dist.p + (uint64_t)n * m;
+      a.slot.rep = d->r_rep.p + (uint64_t)n * m;
+      a.slot.flag = d->r_flag.p + (uint64_t)n * m;
+      a.cum = cum;
+      a.ncum = hh.chkpt_id + 1u;
+      cum += a.ncum;
+      auto take = [&](uint32_t entries) {
+        uint32_t* p = lists;
+        lists += entries;
+        return p;
+      };
+      a.offs[0] = take(hh.F);
+      a.rstart[0] = take(hh.F);
+      a.offs[1] = take(hh.S);
+      a.rstart[1] = take(hh.S);
+      a.pstart = take(hh.S);
+      a.rtree = take(hh.S);
+      for (uint32_t l = 0; l < 2; l++) {
+        a.partial[l] = d->r_partial.p + SCAN_GRID * (2 * m + l);
+        a.total[l] = d->r_total.p + 2 * m + l;
+      }
+      a.st = w.st;
+      // list diffs name chunks; the restart kernels work on leaf heap indices (leaf of chunk c = n-1+c)
+      a.id_bias = d->list ? n - 1u : 0u;
     }
-    std::vector<unsigned long long> cum(ncum, 0ull);
-    bool bad_row = false;
-    const uint8_t* ctab = ddiffs ? diffs[idx] + 32 : diffs[idx] + hh.count_off;   // repeat table on the host
-    for (uint32_t i = 0; i < hh.P; i++) {
-      uint32_t ck, cnt;
-      memcpy(&ck, ctab + 8ull * i, 4);
-      memcpy(&cnt, ctab + 8ull * i + 4, 4);
-      if (ck < ncum) cum[ck] = cnt; else bad_row = true;
-    }
-    for (uint64_t t = 1; t < ncum; t++) cum[t] += cum[t - 1];
-    if (!ddiffs)
-      B2D_CU(cudaMemcpyAsync(d->r_diff.p + delta, src, sizes[idx], cudaMemcpyHostToDevice, d->stream));
-    B2D_CU(cudaMemcpyAsync(d->r_cum.p, cum.data(), sizeof(unsigned long long) * ncum, cudaMemcpyHostToDevice,
-                           d->stream));
-    if (is_main && !ddiffs) {
+    if (!ddiffs) {
+      const int urc = upload(d, copies);
       B2D_CU(cudaStreamSynchronize(d->stream));
-      copy_time = secs(c0, clk::now());
+      if (urc) return urc;
+      copy_time += secs(c0, clk::now());
     }
-    a.diff = ddiffs ? src : d->r_diff.p + delta;
-    a.diff_size = sizes[idx];
-    a.first_off = hh.first_off;
-    a.count_off = hh.count_off;
-    a.shift_off = hh.shift_off;
-    a.data_off = hh.data_off;
-    a.F = hh.F;
-    a.P = hh.P;
-    a.S = hh.S;
-    a.cur_id = hh.chkpt_id;
-    a.datalen = hh.datalen;
-    a.cs = hh.cs;
-    a.is_main = is_main;
-    a.cum = d->r_cum.p;
-    a.ncum = (uint32_t)ncum;
-    a.slot = slot(is_main ? 0 : wcount);
-    B2D_CU(launch_restart_diff(a, &d->state.p->straddle, d->sm_count, d->stream));
-    d->launches += restart_diff_launches(n, d->list != 0);
-    if (!is_main) {
-      // the window's walk copies from every diff in it, which share one chunk size
-      if (wcount == 0) w.cs = hh.cs;
-      w.data[wcount] = a.diff + hh.data_off;
-      w.data_len[wcount] = sizes[idx] - hh.data_off;
-      w.datalen[wcount] = hh.datalen;
-      w.cur[wcount] = hh.chkpt_id;
-      w.slot[wcount] = a.slot;
-      wcount++;
-      const bool end = k + 1 == chain.size();
-      if (bad_row || end || wcount == W || hdrs[k + 1].cs != hh.cs) B2D_CU(flush(bad_row || end));
+    B2D_CU(cudaMemsetAsync(d->r_flag.p, 0, (uint64_t)n * members, d->stream));
+    if (first) B2D_CU(cudaMemsetAsync(d->r_mflag.p, 0, n, d->stream));
+    B2D_CU(launch_restart_diffs(rs, d->r_straddle.p, d->sm_count, d->stream));
+    d->launches += restart_diffs_launches(n, d->list != 0);
+    w.count = 0;
+    for (uint32_t m = first ? 1 : 0; m < members; m++) {
+      const RestartArgs& a = rs.a[m];
+      w.cs = a.cs;
+      w.data[w.count] = a.diff + a.data_off;
+      w.data_len[w.count] = a.diff_size - a.data_off;
+      w.datalen[w.count] = a.datalen;
+      w.cur[w.count] = a.cur_id;
+      w.slot[w.count] = a.slot;
+      w.count++;
     }
-    if (bad_row) {
-      B2D_CU(cudaStreamSynchronize(d->stream));
-      d->restart_timers[0] = copy_time;
-      d->restart_timers[1] = secs(t0, clk::now());
-      return B2D_ERR_RESTART_RANGE;
+    if (w.count) {
+      w.last = last;
+      B2D_CU(launch_restart_walk(w, d->sm_count, d->stream));
+      d->launches += 1;
+      w.dense = 1;   // a walk that is not the last wrote every chunk's NodeID
     }
   }
   B2D_CU(cudaMemcpyAsync(d->state_h.p, d->state.p, sizeof(DevState), cudaMemcpyDeviceToHost, d->stream));

@@ -172,7 +172,7 @@ __device__ __forceinline__ uint32_t entry_len(const RestartArgs& a, uint64_t i, 
   if (which == 0) {
     uint32_t lo, hi;
     leaf_range(rd_node(a, a.diff + a.first_off + 4 * i), a.N, lo, hi);
-    if (want_meta) a.rstart[i] = lo;
+    if (want_meta) a.rstart[0][i] = lo;
     return hi - lo + 1u;
   }
   const uint32_t node = rd_node(a, a.diff + a.shift_off + 8 * i);
@@ -181,7 +181,7 @@ __device__ __forceinline__ uint32_t entry_len(const RestartArgs& a, uint64_t i, 
   leaf_range(node, a.N, nlo, nhi);
   leaf_range(prev, a.N, plo, phi);
   if (want_meta) {
-    a.rstart[i] = nlo;
+    a.rstart[1][i] = nlo;
     a.pstart[i] = plo;
     a.rtree[i] = shift_tree(a, i);
   }
@@ -190,39 +190,58 @@ __device__ __forceinline__ uint32_t entry_len(const RestartArgs& a, uint64_t i, 
   return a.is_main ? phi - plo + 1u : nhi - nlo + 1u;
 }
 
-__global__ void __launch_bounds__(R_THREADS) r_count_kernel(RestartArgs a, int which) {
+// Every step below is a body for one diff on a virtual grid (bid of nb CTAs), with a launcher for
+// one diff and one for all diffs of a RestartSet (blockIdx.y: the diff, or diff and list).
+__device__ __forceinline__ void count_body(const RestartArgs& a, int which, uint32_t bid, uint32_t nb) {
   __shared__ uint32_t sh[R_THREADS / 32 + 1];
   uint64_t beg, end;
-  cta_range(which == 0 ? a.F : a.S, blockIdx.x, gridDim.x, beg, end);
+  cta_range(which == 0 ? a.F : a.S, bid, nb, beg, end);
   uint32_t c = 0;
   for (uint64_t i = beg + threadIdx.x; i < end; i += blockDim.x) c += entry_len(a, i, which, false);
   const uint32_t t = block_reduce_sum(c, sh);
-  if (threadIdx.x == 0) a.partial[blockIdx.x] = t;
+  if (threadIdx.x == 0) a.partial[which][bid] = t;
 }
-
-__global__ void __launch_bounds__(1024) r_scan_kernel(RestartArgs a, uint32_t g) {
+__device__ __forceinline__ void scan_body(const RestartArgs& a, int which, uint32_t g) {
   __shared__ uint32_t sh[33];
   uint32_t tot;
   const uint32_t i = threadIdx.x;
-  const uint32_t v = i < g ? a.partial[i] : 0u;
+  const uint32_t v = i < g ? a.partial[which][i] : 0u;
   const uint32_t e = block_excl_scan(v, sh, &tot);
-  if (i < g) a.partial[i] = e;
-  if (i == 0) *a.total = tot;
+  if (i < g) a.partial[which][i] = e;
+  if (i == 0) *a.total[which] = tot;
 }
-
-__global__ void __launch_bounds__(R_THREADS) r_write_kernel(RestartArgs a, int which) {
+__device__ __forceinline__ void write_body(const RestartArgs& a, int which, uint32_t bid, uint32_t nb) {
   __shared__ uint32_t sh[R_THREADS / 32 + 1];
   uint64_t beg, end;
-  cta_range(which == 0 ? a.F : a.S, blockIdx.x, gridDim.x, beg, end);
-  uint32_t base = a.partial[blockIdx.x];
+  cta_range(which == 0 ? a.F : a.S, bid, nb, beg, end);
+  uint32_t base = a.partial[which][bid];
   for (uint64_t t0 = beg; t0 < end; t0 += blockDim.x) {
     const uint64_t i = t0 + threadIdx.x;
     const uint32_t len = i < end ? entry_len(a, i, which, true) : 0u;
     uint32_t tot;
     const uint32_t e = block_excl_scan(len, sh, &tot);
-    if (i < end) a.offs[i] = base + e;
+    if (i < end) a.offs[which][i] = base + e;
     base += tot;
   }
+}
+__global__ void __launch_bounds__(R_THREADS) r_count_kernel(RestartArgs a, int which) {
+  count_body(a, which, blockIdx.x, gridDim.x);
+}
+__global__ void __launch_bounds__(1024) r_scan_kernel(RestartArgs a, int which, uint32_t g) { scan_body(a, which, g); }
+__global__ void __launch_bounds__(R_THREADS) r_write_kernel(RestartArgs a, int which) {
+  write_body(a, which, blockIdx.x, gridDim.x);
+}
+__global__ void __launch_bounds__(R_THREADS) r_count_set(const __grid_constant__ RestartSet s) {
+  griddep_enter();
+  count_body(s.a[blockIdx.y >> 1], (int)(blockIdx.y & 1u), blockIdx.x, gridDim.x);
+}
+__global__ void __launch_bounds__(1024) r_scan_set(const __grid_constant__ RestartSet s, uint32_t g) {
+  griddep_enter();
+  scan_body(s.a[blockIdx.x >> 1], (int)(blockIdx.x & 1u), g);
+}
+__global__ void __launch_bounds__(R_THREADS) r_write_set(const __grid_constant__ RestartSet s) {
+  griddep_enter();
+  write_body(s.a[blockIdx.y >> 1], (int)(blockIdx.y & 1u), blockIdx.x, gridDim.x);
 }
 
 // largest i in [lo, hi) with off[i] <= k (off[lo] <= k)
@@ -243,8 +262,8 @@ __device__ __forceinline__ uint32_t find_entry(const uint32_t* off, uint32_t lo,
 // With a.id_bias (list diffs) every entry is one chunk: position k is entry k, no search.
 #define R_EXPAND_LOOP(base, count, off, cnt)                                                      \
   const uint32_t lane = threadIdx.x & 31u;                                                        \
-  const uint64_t w0_ = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;                    \
-  const uint64_t nw_ = ((uint64_t)gridDim.x * blockDim.x) >> 5;                                   \
+  const uint64_t w0_ = (bid * (uint64_t)blockDim.x + threadIdx.x) >> 5;                           \
+  const uint64_t nw_ = ((uint64_t)nb_ctas * blockDim.x) >> 5;                                     \
   const uint64_t per_ = ((count) + nw_ * 32u - 1u) / (nw_ * 32u) * 32u;                           \
   const uint64_t beg_ = w0_ * per_;                                                               \
   const uint64_t end_ = beg_ + per_ < (count) ? beg_ + per_ : (count);                            \
@@ -263,11 +282,11 @@ __device__ __forceinline__ uint32_t window_entry(const uint32_t* off, uint32_t i
 
 // first-occurrence regions: dist for every leaf; the main diff also fills node_list and copies
 // the chunk (:822-865 main, :1005-1030 older)
-__global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_first_kernel(RestartArgs a) {
-  const uint64_t T = a.id_bias ? (uint64_t)a.F : *a.total;
+__device__ __forceinline__ void expand_first_body(const RestartArgs& a, uint32_t bid, uint32_t nb_ctas) {
+  const uint64_t T = a.id_bias ? (uint64_t)a.F : *a.total[0];
   const uint8_t* data = a.diff + a.data_off;
   const uint64_t data_len = a.diff_size - a.data_off;
-  R_EXPAND_LOOP(kb, T, a.offs, a.F) {
+  R_EXPAND_LOOP(kb, T, a.offs[0], a.F) {
     const uint64_t k = kb + lane;
     uint64_t dst = 0, nb = 0;
     const uint8_t* src = nullptr;
@@ -280,9 +299,9 @@ __global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_first_ke
         j = 0;
         off0 = (uint32_t)k;
       } else {
-        i = R_WINDOW_ENTRY(a.offs, a.F, k);
-        start = a.rstart[i];
-        off0 = a.offs[i];
+        i = R_WINDOW_ENTRY(a.offs[0], a.F, k);
+        start = a.rstart[0][i];
+        off0 = a.offs[0][i];
         j = (uint32_t)(k - off0);
       }
       const uint64_t c = (uint64_t)start - (a.n - 1u) + j;
@@ -306,6 +325,16 @@ __global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_first_ke
   }
 }
 
+__global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_first_kernel(
+    const __grid_constant__ RestartArgs a) {
+  expand_first_body(a, blockIdx.x, gridDim.x);
+}
+__global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_first_set(
+    const __grid_constant__ RestartSet s) {
+  griddep_enter();
+  expand_first_body(s.a[blockIdx.y], blockIdx.x, gridDim.x);
+}
+
 // Leaves on the shallower level under a region root that spans two depths (only possible
 // when the chunk count is not a power of two): the reference inserts them with an offset
 // computed in wrapping u32 arithmetic (:844-846, :1016-1018).  Reproduced so later lookups
@@ -327,7 +356,7 @@ StraddleQuery straddle_query(uint32_t n) {
   return q;
 }
 
-__global__ void r_straddle_find_kernel(RestartArgs a, StraddleQuery q, StraddleInfo* sd) {
+__device__ __forceinline__ void straddle_find_body(const RestartArgs& a, const StraddleQuery& q, StraddleInfo* sd) {
   const uint32_t D = node_level(a.N - 1u);
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < a.F; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t node = rd_u32(a.diff + a.first_off + 4 * i);
@@ -343,7 +372,7 @@ __global__ void r_straddle_find_kernel(RestartArgs a, StraddleQuery q, StraddleI
     const uint64_t hi = hi_all < lvl_end ? hi_all : lvl_end;
     if (lo <= hi) {
       sd->root = node;
-      sd->region_off = a.offs[i];
+      sd->region_off = a.offs[0][i];
       sd->lo = (uint32_t)lo;
       sd->hi = (uint32_t)hi;
       __threadfence();
@@ -352,7 +381,7 @@ __global__ void r_straddle_find_kernel(RestartArgs a, StraddleQuery q, StraddleI
   }
 }
 
-__global__ void r_straddle_kernel(RestartArgs a, const StraddleInfo* sd) {
+__device__ __forceinline__ void straddle_body(const RestartArgs& a, const StraddleInfo* sd) {
   if (!sd->present) return;
   const uint32_t root = sd->root, region_off = sd->region_off, lo = sd->lo, hi = sd->hi;
   const uint32_t start = leftmost_leaf(root, a.N);
@@ -365,12 +394,25 @@ __global__ void r_straddle_kernel(RestartArgs a, const StraddleInfo* sd) {
   }
 }
 
+__global__ void r_straddle_find_kernel(RestartArgs a, StraddleQuery q, StraddleInfo* sd) {
+  straddle_find_body(a, q, sd);
+}
+__global__ void r_straddle_kernel(RestartArgs a, const StraddleInfo* sd) { straddle_body(a, sd); }
+__global__ void r_straddle_find_set(const __grid_constant__ RestartSet s, StraddleQuery q, StraddleInfo* sd) {
+  griddep_enter();
+  straddle_find_body(s.a[blockIdx.y], q, sd + blockIdx.y);
+}
+__global__ void r_straddle_set(const __grid_constant__ RestartSet s, const StraddleInfo* sd) {
+  griddep_enter();
+  straddle_body(s.a[blockIdx.y], sd + blockIdx.y);
+}
+
 // shifted-duplicate entries (:888-927 main, :1049-1075 older)
-__global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_shift_kernel(RestartArgs a) {
-  const uint64_t T = a.id_bias ? (uint64_t)a.S : *a.total;
+__device__ __forceinline__ void expand_shift_body(const RestartArgs& a, uint32_t bid, uint32_t nb_ctas) {
+  const uint64_t T = a.id_bias ? (uint64_t)a.S : *a.total[1];
   const uint8_t* data = a.diff + a.data_off;
   const uint64_t data_len = a.diff_size - a.data_off;
-  R_EXPAND_LOOP(kb, T, a.offs, a.S) {
+  R_EXPAND_LOOP(kb, T, a.offs[1], a.S) {
     const uint64_t k = kb + lane;
     uint64_t dst = 0, nb = 0;
     const uint8_t* src = nullptr;
@@ -384,9 +426,9 @@ __global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_shift_ke
         prev_start = rd_node(a, a.diff + a.shift_off + 8ull * k + 4);
         tree = shift_tree(a, k);
       } else {
-        i = R_WINDOW_ENTRY(a.offs, a.S, k);
-        j = (uint32_t)(k - a.offs[i]);
-        node_start = a.rstart[i];
+        i = R_WINDOW_ENTRY(a.offs[1], a.S, k);
+        j = (uint32_t)(k - a.offs[1][i]);
+        node_start = a.rstart[1][i];
         prev_start = a.pstart[i];
         tree = a.rtree[i];
       }
@@ -416,6 +458,16 @@ __global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_shift_ke
   }
 }
 
+__global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_shift_kernel(
+    const __grid_constant__ RestartArgs a) {
+  expand_shift_body(a, blockIdx.x, gridDim.x);
+}
+__global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_shift_set(
+    const __grid_constant__ RestartSet s) {
+  griddep_enter();
+  expand_shift_body(s.a[blockIdx.y], blockIdx.x, gridDim.x);
+}
+
 // Every chunk through the window's diffs, newest first (:1083-1118 per diff): a diff acts on a
 // chunk whose NodeID names it -- copy from its data when the leaf is a first occurrence there
 // (or a shifted copy of one in the same diff), follow a shifted leaf to its source NodeID, or
@@ -423,7 +475,8 @@ __global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_shift_ke
 // (their leaf, main id - 1), as the reference's node_list does (:933-939).  A chunk's NodeID
 // usually stays its own leaf all the way down, so that leaf's flags in every slot are loaded up
 // front, side by side; another leaf's flags are loaded when the walk reaches it.
-__global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_walk_kernel(RestartWalk w) {
+__global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_walk_kernel(const __grid_constant__ RestartWalk w) {
+  griddep_enter();
   R_WARP_LOOP(cb, w.n) {
     const uint64_t c = cb + lane;
     const uint64_t dst = c * w.cs;
@@ -494,23 +547,54 @@ __global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_walk_kernel(Res
 // running shift counts per checkpoint id from a device-resident diff's (ckpt, count) table:
 // the last row for an id wins, then an inclusive scan over ids (:871-885); rows naming an id
 // beyond the diff's own are outside the reference's array and are reported
-__global__ void r_cum_kernel(RestartArgs a) {
+__device__ __forceinline__ void cum_body(const RestartArgs& a) {
+  __shared__ uint32_t sh[33];
   unsigned long long* cum = const_cast<unsigned long long*>(a.cum);
   for (uint32_t t = threadIdx.x; t < a.ncum; t += blockDim.x) cum[t] = 0;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (uint32_t i = 0; i < a.P; i++) {
-      const uint32_t ck = rd_u32(a.diff + a.count_off + 8ull * i);
-      const uint32_t cnt = rd_u32(a.diff + a.count_off + 8ull * i + 4);
-      if (ck < a.ncum) cum[ck] = cnt;
+  auto id = [&](uint32_t i) { return rd_u32(a.diff + a.count_off + 8ull * i); };
+  auto cnt = [&](uint32_t i) { return rd_u32(a.diff + a.count_off + 8ull * i + 4); };
+  // ascending ids (every table a checkpoint writes) go in side by side; others row by row
+  bool bad = false;
+  for (uint32_t i = threadIdx.x; i + 1u < a.P; i += blockDim.x) bad |= id(i) >= id(i + 1u);
+  if (__syncthreads_or(bad)) {
+    if (threadIdx.x == 0)
+      for (uint32_t i = 0; i < a.P; i++) {
+        if (id(i) < a.ncum) cum[id(i)] = cnt(i);
+        else set_error(a.st, DERR_RESTART_RANGE, 5);
+      }
+  } else {
+    for (uint32_t i = threadIdx.x; i < a.P; i += blockDim.x) {
+      if (id(i) < a.ncum) cum[id(i)] = cnt(i);
       else set_error(a.st, DERR_RESTART_RANGE, 5);
     }
-    unsigned long long run = 0;
-    for (uint32_t t = 0; t < a.ncum; t++) {
-      run += cum[t];
-      cum[t] = run;
-    }
   }
+  __syncthreads();
+  // inclusive scan; 64-bit sums (each count is a u32), so the block scan runs on the two halves of
+  // the counts: 16 bits of 256 counts add up within 32
+  unsigned long long carry = 0;
+  for (uint32_t t0 = 0; t0 < a.ncum; t0 += blockDim.x) {
+    const uint32_t t = t0 + threadIdx.x;
+    const uint32_t v = t < a.ncum ? (uint32_t)cum[t] : 0u;
+    uint32_t tl, th;
+    const uint32_t el = block_excl_scan(v & 0xffffu, sh, &tl);
+    const uint32_t eh = block_excl_scan(v >> 16, sh, &th);
+    if (t < a.ncum) cum[t] = carry + el + ((unsigned long long)eh << 16) + v;
+    carry += tl + ((unsigned long long)th << 16);
+  }
+}
+__global__ void __launch_bounds__(256) r_cum_kernel(RestartArgs a) { cum_body(a); }
+__global__ void __launch_bounds__(256) r_cum_set(const __grid_constant__ RestartSet s) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  cum_body(s.a[blockIdx.x]);
+}
+
+__global__ void __launch_bounds__(32) r_headers_kernel(const __grid_constant__ RestartHeaders h, uint8_t* out) {
+  out[32u * blockIdx.x + threadIdx.x] = h.diff[blockIdx.x][threadIdx.x];
+}
+cudaError_t launch_restart_headers(const RestartHeaders& h, uint8_t* out, cudaStream_t s) {
+  if (h.count == 0 || h.count > RESTART_HEADERS) return cudaErrorInvalidValue;
+  r_headers_kernel<<<h.count, 32, 0, s>>>(h, out);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_restart_cum(const RestartArgs& a, cudaStream_t s) {
@@ -553,7 +637,7 @@ cudaError_t launch_restart_diff(const RestartArgs& args, StraddleInfo* sd, int s
   // first-occurrence regions
   if (scan) {
     r_count_kernel<<<g, R_THREADS, 0, s>>>(a, 0);
-    r_scan_kernel<<<1, 1024, 0, s>>>(a, g);
+    r_scan_kernel<<<1, 1024, 0, s>>>(a, 0, g);
     r_write_kernel<<<g, R_THREADS, 0, s>>>(a, 0);
   }
   r_expand_first_kernel<<<grid_for(a.n, sm_count), R_THREADS, 0, s>>>(a);
@@ -567,11 +651,54 @@ cudaError_t launch_restart_diff(const RestartArgs& args, StraddleInfo* sd, int s
   // shifted duplicates
   if (scan) {
     r_count_kernel<<<g, R_THREADS, 0, s>>>(a, 1);
-    r_scan_kernel<<<1, 1024, 0, s>>>(a, g);
+    r_scan_kernel<<<1, 1024, 0, s>>>(a, 1, g);
     r_write_kernel<<<g, R_THREADS, 0, s>>>(a, 1);
   }
   r_expand_shift_kernel<<<grid_for(a.n, sm_count), R_THREADS, 0, s>>>(a);
   return cudaGetLastError();
+}
+
+int restart_diffs_launches(uint32_t n, bool list) { return list ? 3 : 6 + (straddle_query(n).count ? 2 : 0); }
+
+cudaError_t launch_restart_diffs(const RestartSet& set, StraddleInfo* sd, int sm_count, cudaStream_t s) {
+  RestartSet q = set;
+  if (q.count == 0 || q.count > RESTART_WINDOW + 1u) return cudaErrorInvalidValue;
+  uint64_t most[2] = {1, 1};   // longest list of each kind
+  for (uint32_t k = 0; k < q.count; k++) {
+    RestartArgs& a = q.a[k];
+    copy_width((uint64_t)(uintptr_t)a.out, (uint64_t)(uintptr_t)(a.diff + a.data_off), a.cs, a.width, a.per,
+               a.per_log2);
+    if (a.F > most[0]) most[0] = a.F;
+    if (a.S > most[1]) most[1] = a.S;
+  }
+  const uint32_t n = q.a[0].n;
+  const bool scan = !q.a[0].id_bias;   // list entries are single chunks: offsets are the entry indices
+  const StraddleQuery st = scan ? straddle_query(n) : StraddleQuery{};
+  cudaError_t e = cudaSuccess;
+  if (st.count) e = cudaMemsetAsync(sd, 0, sizeof(StraddleInfo) * q.count, s);
+  if (e != cudaSuccess) return e;
+  r_cum_set<<<q.count, 256, 0, s>>>(q);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+#define R_LD(...)                                                \
+  if ((e = launch_dependent(__VA_ARGS__)) != cudaSuccess) return e;
+  if (scan) {
+    // about four entries per thread; short lists take few CTAs
+    const uint64_t longest = most[0] > most[1] ? most[0] : most[1];
+    const uint64_t want = (longest + 4u * R_THREADS - 1u) / (4u * R_THREADS);
+    const uint32_t g = want < SCAN_GRID ? (uint32_t)want : SCAN_GRID;
+    R_LD(r_count_set, dim3(g, 2u * q.count), R_THREADS, 0, s, q)
+    R_LD(r_scan_set, 2u * q.count, 1024, 0, s, q, g)
+    R_LD(r_write_set, dim3(g, 2u * q.count), R_THREADS, 0, s, q)
+  }
+  const uint32_t gx = grid_for(n, sm_count);
+  R_LD(r_expand_first_set, dim3(gx, q.count), R_THREADS, 0, s, q)
+  if (st.count) {
+    R_LD(r_straddle_find_set, dim3(grid_for(most[0], sm_count), q.count), R_THREADS, 0, s, q, st, sd)
+    R_LD(r_straddle_set, dim3((uint32_t)sm_count, q.count), R_THREADS, 0, s, q, sd)
+  }
+  R_LD(r_expand_shift_set, dim3(gx, q.count), R_THREADS, 0, s, q)
+#undef R_LD
+  return cudaSuccess;
 }
 
 cudaError_t launch_restart_walk(const RestartWalk& walk, int sm_count, cudaStream_t s) {
@@ -580,8 +707,7 @@ cudaError_t launch_restart_walk(const RestartWalk& walk, int sm_count, cudaStrea
   uint64_t src_al = 0;
   for (uint32_t k = 0; k < w.count; k++) src_al |= (uint64_t)(uintptr_t)w.data[k];
   copy_width((uint64_t)(uintptr_t)w.out, src_al, w.cs, w.width, w.per, w.per_log2);
-  r_walk_kernel<<<grid_for(w.n, sm_count), R_THREADS, 0, s>>>(w);
-  return cudaGetLastError();
+  return launch_dependent(r_walk_kernel, grid_for(w.n, sm_count), R_THREADS, 0, s, w);
 }
 
 }  // namespace b2d

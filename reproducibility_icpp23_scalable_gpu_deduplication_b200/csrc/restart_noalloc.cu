@@ -132,13 +132,14 @@ extern "C" int b2d_restart_noalloc(void* d_out, uint64_t len, const void* const*
   a.slot.dist = reinterpret_cast<uint32_t*>(base + NA_DIST);
   a.slot.rep = reinterpret_cast<uint2*>(base + NA_REP);
   a.slot.flag = base + NA_FLAG;
-  a.offs = reinterpret_cast<uint32_t*>(base + NA_OFFS);
-  a.rstart = a.offs + NOALLOC_MAX_CHUNKS;
-  a.pstart = a.offs + 2 * NOALLOC_MAX_CHUNKS;
-  a.rtree = a.offs + 3 * NOALLOC_MAX_CHUNKS;
+  // both lists in one place: the first is expanded before the second is scanned
+  a.offs[0] = a.offs[1] = reinterpret_cast<uint32_t*>(base + NA_OFFS);
+  a.rstart[0] = a.rstart[1] = a.offs[0] + NOALLOC_MAX_CHUNKS;
+  a.pstart = a.offs[0] + 2 * NOALLOC_MAX_CHUNKS;
+  a.rtree = a.offs[0] + 3 * NOALLOC_MAX_CHUNKS;
   a.cum = reinterpret_cast<unsigned long long*>(base + NA_CUM);
-  a.partial = reinterpret_cast<uint32_t*>(base + NA_PARTIAL);
-  a.total = reinterpret_cast<unsigned long long*>(base + NA_TOTAL);
+  a.partial[0] = a.partial[1] = reinterpret_cast<uint32_t*>(base + NA_PARTIAL);
+  a.total[0] = a.total[1] = reinterpret_cast<unsigned long long*>(base + NA_TOTAL);
   a.st = reinterpret_cast<DevStatus*>(base + NA_STATUS);
   StraddleInfo* sd = reinterpret_cast<StraddleInfo*>(base + NA_STRADDLE);
   if (cudaMemsetAsync(a.st, 0, sizeof(DevStatus), s) != cudaSuccess) return B2D_ERR_CUDA;
