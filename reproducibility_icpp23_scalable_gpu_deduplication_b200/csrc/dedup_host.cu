@@ -422,10 +422,16 @@ int status_code(const DevStatus& st) {
 }
 
 
+// Labels and duplicate flags start so many bytes into their buffers that the first leaf of the
+// deepest level is 16-byte aligned (forest.cu, LeafSlots).
+uint32_t leaf_pad(const b2d_dedup* d) { return (16u - ((uint32_t)((1ull << d->D) - d->n) & 15u)) & 15u; }
+uint8_t* leaf_labels(const b2d_dedup* d) { return d->leaflab.p + leaf_pad(d); }
+uint8_t* dup_flags(const b2d_dedup* d) { return d->dupflag.p + leaf_pad(d); }
+
 LeafArgs leaf_args(const b2d_dedup* d, const RoundState* rs_dev) {
   const MapView m = map_at(d->map_mem, d->map_cap, d->map_size.p);
   return LeafArgs{static_cast<const uint8_t*>(d->data), d->data_len, d->chunk_size, d->n, d->kind, 0, 0,
-                  d->tree.p, d->leaflab.p, d->dupflag.p, m, &d->state.p->status, rs_dev,
+                  d->tree.p, leaf_labels(d), dup_flags(d), m, &d->state.p->status, rs_dev,
                   (uint32_t)d->tune.wait_polls, 1u, &d->state.p->zero_exists, d->bulk};
 }
 
@@ -467,9 +473,9 @@ int prepare_checkpoint(b2d_dedup* d, const void* d_data, uint64_t len, bool make
   B2D_CU(d->tree.reserve(d->N));
   B2D_CU(d->lab.reserve(d->N));
   B2D_CU(d->leaflab.reserve((uint64_t)d->n + 16u));
-  if (d->dupflag.n < d->n || !d->dupflag.p) {
+  if (d->dupflag.n < (uint64_t)d->n + 16u || !d->dupflag.p) {
     // duplicate flags stay all-zero between checkpoints (phase 1 clears what it reads)
-    B2D_CU(d->dupflag.reserve(d->n));
+    B2D_CU(d->dupflag.reserve((uint64_t)d->n + 16u));
     B2D_CU(cudaMemsetAsync(d->dupflag.p, 0, d->dupflag.n, d->stream));
   }
   const uint64_t push_bytes = ((uint64_t)d->N + 63ull) / 64ull * 16ull + 16ull;   // 2 bits per node
@@ -554,7 +560,7 @@ BulkArgs bulk_args(b2d_dedup* d) {
   DevState* ds = d->state.p;
   const BulkPlan& p = d->plan;
   b.tree = d->tree.p;
-  b.leaflab = d->leaflab.p;
+  b.leaflab = leaf_labels(d);
   map_view(d, b.map);
   b.st = &ds->status;
   b.n = d->n;
@@ -588,7 +594,7 @@ ForestArgs forest_args(b2d_dedup* d, const RoundState* rs_dev) {
   MapView m;
   map_view(d, m);
   DevState* ds = d->state.p;
-  return ForestArgs{d->tree.p, d->lab.p, d->leaflab.p, d->push.p, m, &ds->status, &ds->zero_exists, d->dupflag.p,
+  return ForestArgs{d->tree.p, d->lab.p, leaf_labels(d), d->push.p, m, &ds->status, &ds->zero_exists, dup_flags(d),
                     d->n, d->N, d->D, 0, d->kind, 0, rs_dev, nullptr,
                     d->bulk ? bulk_scratch(d, d->plan.lost) : nullptr, &ds->lost_any, 0};
 }
@@ -2096,7 +2102,7 @@ int b2d_debug_tree(b2d_dedup* d, void* dst, uint64_t nodes) {
 }
 int b2d_debug_labels(b2d_dedup* d, void* dst, uint64_t leaves) {
   if (!d || !dst || leaves > d->n || !d->leaflab.p) return B2D_ERR_ARG;
-  B2D_CU(cudaMemcpyAsync(dst, d->leaflab.p, leaves, cudaMemcpyDeviceToHost, d->stream));
+  B2D_CU(cudaMemcpyAsync(dst, leaf_labels(d), leaves, cudaMemcpyDeviceToHost, d->stream));
   B2D_CU(cudaStreamSynchronize(d->stream));
   return B2D_OK;
 }
@@ -2173,7 +2179,7 @@ int b2d_estimate_memory(uint64_t len, uint32_t chunk_size, int map_max_load_pct,
   // the allocations prepare_checkpoint makes for a buffer of `len` bytes (checkpoint side)
   const uint64_t n = (len + chunk_size - 1) / chunk_size, N = 2 * n - 1;
   const uint64_t cap = map_capacity(2 * N, map_max_load_pct / 100.0, MAP_HEADROOM);
-  uint64_t b = N * sizeof(Digest) + N + (n + 16) + ((N + 63) / 64 * 16 + 16) + n;   // tree, labels, flags
+  uint64_t b = N * sizeof(Digest) + N + (n + 16) + ((N + 63) / 64 * 16 + 16) + (n + 16);   // tree, labels, flags
   b += (cap + 1) * MAP_SLOT_BYTES + 8;                                               // map
   b += 5 * 4 * n;                                                                    // lists and keys
   b += (uint64_t)64 * 4 * 2 + (uint64_t)1184 * 64 * 4 + 3 * COMPACT_GRID * 4;           // buckets, partials

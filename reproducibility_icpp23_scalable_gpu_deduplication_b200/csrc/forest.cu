@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(FAST_THREADS, B2D_FAST_MINB) forest_fast_seg(F
   forest_fast_body<PHASE>(with_round(s.args[h]), bid, s.p0[h]);
 }
 
-// Warp bands: the first band of each phase of a tree whose chunk count is a power of two, as
+// Warp bands: the first band of each phase, as
 // independent warp tasks (no CTA barrier).  A CTA band stalls all its warps on three barriers
 // per band and a CTA takes its bands one after another, so most of a band's time was load and
 // barrier latency; a warp task folds its leaves in registers and by shuffles only, and each
@@ -597,8 +597,35 @@ constexpr uint32_t WB_THREADS = 256;
 #endif
 
 static bool warp_bands(uint32_t n, uint32_t D, int phase, int mask) {
-  return (mask & (phase == 1 ? 1 : 2)) && n >= 2u && (n & (n - 1u)) == 0 &&
-         D >= (phase == 1 ? WB1_LEVELS : WB2_LEVELS);
+  return (mask & (phase == 1 ? 1 : 2)) && n >= 2u && D >= (phase == 1 ? WB1_LEVELS : WB2_LEVELS);
+}
+
+// Leaf labels by slot of the deepest level.  Slot s < deep is the leaf at position s of level D;
+// the slots from there on (chunk counts that are not powers of two; deep is even) stand in pairs
+// for the leaves of level D-1, whose label both slots of a pair carry.  The host places `leaflab`
+// and `dupflag` so that slot 0 is 16-byte aligned: a lane whose slots are all on level D loads
+// them at once.
+struct LeafSlots {
+  uint32_t full;   // slots
+  uint32_t deep;   // leaves on level D
+};
+__device__ __forceinline__ LeafSlots leaf_slots(const ForestArgs& a) {
+  const uint32_t full = 1u << a.D;
+  return LeafSlots{full, 2u * a.n - full};
+}
+// the labels of slots s, s + 1 (s even), in the low 16 bits
+__device__ __forceinline__ uint32_t slot_pair(const ForestArgs& a, const LeafSlots& q, uint32_t s) {
+  if (s < q.deep) return *reinterpret_cast<const uint16_t*>(a.leaflab + (q.full - a.n) + s);
+  return 0x0101u * a.leaflab[(q.full + s) / 2u - a.n];
+}
+__device__ __forceinline__ uint32_t slot_labels4(const ForestArgs& a, const LeafSlots& q, uint32_t s) {
+  if (s + 4u <= q.deep) return *reinterpret_cast<const uint32_t*>(a.leaflab + (q.full - a.n) + s);
+  return slot_pair(a, q, s) | slot_pair(a, q, s + 2u) << 16;
+}
+__device__ __forceinline__ uint4 slot_labels16(const ForestArgs& a, const LeafSlots& q, uint32_t s) {
+  if (s + 16u <= q.deep) return *reinterpret_cast<const uint4*>(a.leaflab + (q.full - a.n) + s);
+  return make_uint4(slot_labels4(a, q, s), slot_labels4(a, q, s + 4u), slot_labels4(a, q, s + 8u),
+                    slot_labels4(a, q, s + 12u));
 }
 
 // Parents a phase-1 warp task created, inserted into the map together once the task's hashing is
@@ -642,8 +669,10 @@ __device__ __forceinline__ void wi_flush(const ForestArgs& a, const WarpInserts&
 __device__ __forceinline__ void warp1_task(const ForestArgs& a, uint32_t task, uint32_t lane, uint32_t w,
                                            const WarpInserts& wi) {
   const uint64_t root = ((1ull << (a.D - WB1_LEVELS)) - 1ull) + task;
-  const uint32_t c0 = task * 128u + 4u * lane;          // first chunk of this lane
-  const uint64_t x0 = (uint64_t)(a.n - 1u) + c0;        // its leaf (a left child)
+  const uint32_t s0 = task * 128u + 4u * lane;          // first slot of this lane
+  const uint64_t x0 = (1ull << a.D) - 1ull + s0;        // its node (a left child)
+  const uint64_t p0 = (x0 - 1ull) >> 1;                 // the two nodes above
+  const uint32_t leaves = (uint32_t)(p0 >= a.n - 1u) | (uint32_t)(p0 + 1u >= a.n - 1u) << 1;   // of those
   const uint32_t z = ~(((w & 0x7f7f7f7fu) + 0x7f7f7f7fu) | w | 0x7f7f7f7fu);   // exact: byte == FIRST (0)
   uint32_t m0 = ((z >> 7) & 1u) | ((z >> 14) & 2u) | ((z >> 21) & 4u) | ((z >> 28) & 8u);
   if (!__any_sync(0xffffffffu, m0 != 0u)) {
@@ -656,33 +685,44 @@ __device__ __forceinline__ void warp1_task(const ForestArgs& a, uint32_t task, u
 #pragma unroll
   for (int j = 0; j < 4; j++) lv[j].w[0] = lv[j].w[1] = lv[j].w[2] = lv[j].w[3] = 0u;
   if (m0) {
-    const uint32_t df = *reinterpret_cast<const uint32_t*>(a.dupflag + c0);
+    const uint32_t df =
+        leaves ? 1u : *reinterpret_cast<const uint32_t*>(a.dupflag + ((1u << a.D) - a.n) + s0);
 #pragma unroll
     for (int j = 0; j < 2; j++)
       if (((m0 >> (2 * j)) & 3u) == 3u) {
-        lv[2 * j] = a.tree[x0 + 2 * j];
-        lv[2 * j + 1] = a.tree[x0 + 2 * j + 1];
+        if ((leaves >> j) & 1u) {
+          lv[2 * j] = a.tree[p0 + j];
+        } else {
+          lv[2 * j] = a.tree[x0 + 2 * j];
+          lv[2 * j + 1] = a.tree[x0 + 2 * j + 1];
+        }
       }
     if (df) {
       // lowest-index relabel of the first occurrences the leaf stage flagged as sharing a digest
 #pragma unroll
-      for (int j = 0; j < 4; j++)
-        if ((m0 >> j) & 1u)
-          if (leaf_view<1>(a, (uint32_t)(x0 + j), FIRST_OCUR) != FIRST_OCUR) m0 &= ~(1u << j);
+      for (int j = 0; j < 4; j++) {
+        const bool leaf = (leaves >> (j / 2)) & 1u;   // the pair is one leaf of level D-1
+        if (((m0 >> j) & 1u) && !(leaf && (j & 1)))
+          if (leaf_view<1>(a, (uint32_t)(leaf ? p0 + j / 2 : x0 + j), FIRST_OCUR) != FIRST_OCUR)
+            m0 &= ~((leaf ? 3u : 1u) << j);
+      }
     }
   }
   // height 1: nodes p0, p0 + 1; height 2: node y
-  const uint64_t p0 = (x0 - 1ull) >> 1;
   Digest d1[2];
   uint32_t m1 = 0;
 #pragma unroll
   for (int j = 0; j < 2; j++) {
     d1[j].w[0] = d1[j].w[1] = d1[j].w[2] = d1[j].w[3] = 0u;
     if (((m0 >> (2 * j)) & 3u) == 3u) {
+      m1 |= 1u << j;
+      if ((leaves >> j) & 1u) {
+        d1[j] = lv[2 * j];
+        continue;
+      }
       d1[j] = hash_pair(a.kind, lv[2 * j], lv[2 * j + 1]);
       a.tree[p0 + j] = d1[j];
       wi_add(wi, (uint32_t)(p0 + j), d1[j]);
-      m1 |= 1u << j;
     }
   }
   uint64_t y = (p0 - 1ull) >> 1;
@@ -729,8 +769,7 @@ __device__ __forceinline__ uint8_t fixed_or_node(const ForestArgs& a, uint32_t x
 
 __device__ __forceinline__ void warp2_task(const ForestArgs& a, uint32_t task, uint32_t lane, const uint4& w) {
   const uint64_t root = ((1ull << (a.D - WB2_LEVELS)) - 1ull) + task;
-  const uint32_t c0 = task * 512u + 16u * lane;
-  const uint64_t x0 = (uint64_t)(a.n - 1u) + c0;
+  const uint64_t x0 = (1ull << a.D) - 1ull + task * 512u + 16u * lane;
   bool fast = !a.baseline && w.x == 0x01010101u && w.y == 0x01010101u && w.z == 0x01010101u &&
               w.w == 0x01010101u;   // all 16 leaves FIXED
   if (__all_sync(0xffffffffu, fast)) {
@@ -748,7 +787,10 @@ __device__ __forceinline__ void warp2_task(const ForestArgs& a, uint32_t task, u
     for (int width = 8; width >= 1; width >>= 1) {
       first = (first - 1ull) >> 1;
 #pragma unroll
-      for (int j = 0; j < width; j++) v[j] = fixed_or_node(a, (uint32_t)(first + j), v[2 * j], v[2 * j + 1]);
+      for (int j = 0; j < width; j++) {
+        if (width == 8 && first + j >= a.n - 1u) v[j] = v[2 * j];   // a leaf of level D-1
+        else v[j] = fixed_or_node(a, (uint32_t)(first + j), v[2 * j], v[2 * j + 1]);
+      }
     }
     lab = v[0];
   }
@@ -835,12 +877,13 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB1_MINB)
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t G = (gridDim.x * WB_THREADS) >> 5;
   const uint32_t w0 = (blockIdx.x * WB_THREADS + threadIdx.x) >> 5;
-  const uint32_t* lab32 = reinterpret_cast<const uint32_t*>(a.leaflab);
+  const LeafSlots q = leaf_slots(a);
+  auto labels = [&](uint32_t task) { return slot_labels4(a, q, task * 128u + 4u * lane); };
   if (!queue) {
-    uint32_t w = w0 < ntasks ? lab32[w0 * 32u + lane] : 0u;
+    uint32_t w = w0 < ntasks ? labels(w0) : 0u;
     for (uint32_t task = w0; task < ntasks; task += G) {
       const uint32_t next = task + G;
-      const uint32_t wn = next < ntasks ? lab32[next * 32u + lane] : 0u;
+      const uint32_t wn = next < ntasks ? labels(next) : 0u;
       warp1_task(a, task, lane, w, wi);
       w = wn;
     }
@@ -851,7 +894,7 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB1_MINB)
 #pragma unroll
   for (uint32_t k = 0; k < WB_SCAN; k++) {
     const uint32_t t = w0 + k * G;
-    wn[k] = t < ntasks ? lab32[t * 32u + lane] : 0x01010101u;
+    wn[k] = t < ntasks ? labels(t) : 0x01010101u;
   }
   for (uint32_t t0 = w0; t0 < ntasks; t0 += WB_SCAN * G) {
     uint32_t work = 0;   // bit k: task t0 + kG holds a first occurrence
@@ -861,7 +904,7 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB1_MINB)
 #pragma unroll
     for (uint32_t k = 0; k < WB_SCAN; k++) {
       const uint32_t t = t0 + (WB_SCAN + k) * G;
-      wn[k] = t < ntasks ? lab32[t * 32u + lane] : 0x01010101u;
+      wn[k] = t < ntasks ? labels(t) : 0x01010101u;
     }
 #pragma unroll
     for (uint32_t k = 0; k < WB_SCAN; k++) {
@@ -874,7 +917,7 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB1_MINB)
   __syncthreads();
   const uint32_t qn = wq_n_;
   for (uint32_t t = wq_pop(wq_, &wq_h_, qn, lane); t != ~0u; t = wq_pop(wq_, &wq_h_, qn, lane))
-    warp1_task(a, t, lane, lab32[t * 32u + lane], wi);
+    warp1_task(a, t, lane, labels(t), wi);
 }
 __global__ void __launch_bounds__(WB_THREADS, B2D_WB2_MINB)
     forest_warp2_kernel(const __grid_constant__ ForestArgs a0, uint32_t ntasks, uint32_t queue) {
@@ -884,12 +927,13 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB2_MINB)
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t G = (gridDim.x * WB_THREADS) >> 5;
   const uint32_t w0 = (blockIdx.x * WB_THREADS + threadIdx.x) >> 5;
-  const uint4* lab128 = reinterpret_cast<const uint4*>(a.leaflab);
+  const LeafSlots q = leaf_slots(a);
+  auto labels = [&](uint32_t task) { return slot_labels16(a, q, task * 512u + 16u * lane); };
   if (!queue) {
-    uint4 w = w0 < ntasks ? lab128[w0 * 32u + lane] : make_uint4(0, 0, 0, 0);
+    uint4 w = w0 < ntasks ? labels(w0) : make_uint4(0, 0, 0, 0);
     for (uint32_t task = w0; task < ntasks; task += G) {
       const uint32_t next = task + G;
-      const uint4 wn = next < ntasks ? lab128[next * 32u + lane] : make_uint4(0, 0, 0, 0);
+      const uint4 wn = next < ntasks ? labels(next) : make_uint4(0, 0, 0, 0);
       warp2_task(a, task, lane, w);
       w = wn;
     }
@@ -901,7 +945,7 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB2_MINB)
 #pragma unroll
   for (uint32_t k = 0; k < WB_SCAN; k++) {
     const uint32_t t = w0 + k * G;
-    wn[k] = t < ntasks ? lab128[t * 32u + lane] : fixed4;
+    wn[k] = t < ntasks ? labels(t) : fixed4;
   }
   for (uint32_t t0 = w0; t0 < ntasks; t0 += WB_SCAN * G) {
     uint32_t work = 0;   // bit k: task t0 + kG has a leaf that is not FIXED (every task of a baseline)
@@ -914,7 +958,7 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB2_MINB)
 #pragma unroll
     for (uint32_t k = 0; k < WB_SCAN; k++) {
       const uint32_t t = t0 + (WB_SCAN + k) * G;
-      wn[k] = t < ntasks ? lab128[t * 32u + lane] : fixed4;
+      wn[k] = t < ntasks ? labels(t) : fixed4;
     }
 #pragma unroll
     for (uint32_t k = 0; k < WB_SCAN; k++) {
@@ -927,7 +971,7 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB2_MINB)
   __syncthreads();
   const uint32_t qn = wq_n_;
   for (uint32_t t = wq_pop(wq_, &wq_h_, qn, lane); t != ~0u; t = wq_pop(wq_, &wq_h_, qn, lane))
-    warp2_task(a, t, lane, lab128[t * 32u + lane]);
+    warp2_task(a, t, lane, labels(t));
 }
 
 // Segmented warp bands (batched form): CTA b of a handle's range holds its tasks 8b .. 8b+7,
@@ -938,18 +982,18 @@ __global__ void __launch_bounds__(WB_THREADS) forest_warp1_seg(ForestSeg s) {
   const uint32_t h = seg_find(s.beg, s.n, bid, nb);
   const ForestArgs a = with_round(s.args[h]);
   const uint32_t task = bid * (WB_THREADS / 32u) + (threadIdx.x >> 5);
-  if (task >= (a.n >> WB1_LEVELS)) return;
+  if (task >= (1u << (a.D - WB1_LEVELS))) return;
   const uint32_t lane = threadIdx.x & 31u;
-  warp1_task(a, task, lane, reinterpret_cast<const uint32_t*>(a.leaflab)[task * 32u + lane], wi);
+  warp1_task(a, task, lane, slot_labels4(a, leaf_slots(a), task * 128u + 4u * lane), wi);
 }
 __global__ void __launch_bounds__(WB_THREADS) forest_warp2_seg(ForestSeg s) {
   uint32_t bid, nb;
   const uint32_t h = seg_find(s.beg, s.n, bid, nb);
   const ForestArgs a = with_round(s.args[h]);
   const uint32_t task = bid * (WB_THREADS / 32u) + (threadIdx.x >> 5);
-  if (task >= (a.n >> WB2_LEVELS)) return;
+  if (task >= (1u << (a.D - WB2_LEVELS))) return;
   const uint32_t lane = threadIdx.x & 31u;
-  warp2_task(a, task, lane, reinterpret_cast<const uint4*>(a.leaflab)[task * 32u + lane]);
+  warp2_task(a, task, lane, slot_labels16(a, leaf_slots(a), task * 512u + 16u * lane));
 }
 
 // General band: levels [top, bot] (top <= bot <= D), level by level through shared memory.
@@ -1032,7 +1076,7 @@ void forest_steps_batch(uint32_t n, uint32_t D, uint64_t N, int phase, std::vect
   std::vector<ForestStep> rest;
   forest_steps_from(D, D - levels, N, phase, rest);
   out.clear();
-  out.push_back(ForestStep{2, D, 0, ((n >> levels) + WB_THREADS / 32u - 1u) / (WB_THREADS / 32u)});
+  out.push_back(ForestStep{2, D, 0, ((1u << (D - levels)) + WB_THREADS / 32u - 1u) / (WB_THREADS / 32u)});
   out.insert(out.end(), rest.begin(), rest.end());
 }
 
@@ -1056,11 +1100,12 @@ cudaError_t launch_forest(const ForestArgs& args, int phase, cudaStream_t stream
     static const uint32_t res_w1 = resident_ctas(forest_warp1_kernel);
     static const uint32_t res_w2 = resident_ctas(forest_warp2_kernel);
     const uint32_t levels = phase == 1 ? WB1_LEVELS : WB2_LEVELS;
-    const uint32_t ntasks = a.n >> levels;
+    const uint32_t ntasks = 1u << (a.D - levels);
     const uint32_t want = (ntasks + WB_THREADS / 32u - 1u) / (WB_THREADS / 32u);
     const uint32_t cap = (phase == 1 ? res_w1 : res_w2) * (uint32_t)(sm_count > 0 ? sm_count : 1);
     const uint32_t grid = want < cap ? want : cap;
-    const uint32_t queue = wq_fits(ntasks, grid) ? 1u : 0u;
+    // one task per warp at most: nothing to spread, and the queue's barrier and atomics only delay it
+    const uint32_t queue = ntasks > grid * (WB_THREADS / 32u) && wq_fits(ntasks, grid) ? 1u : 0u;
     cudaError_t e = phase == 1 ? launch_dependent(forest_warp1_kernel, grid, WB_THREADS, 0, stream, a, ntasks, queue)
                                : launch_dependent(forest_warp2_kernel, grid, WB_THREADS, 0, stream, a, ntasks, queue);
     if (e != cudaSuccess) return e;

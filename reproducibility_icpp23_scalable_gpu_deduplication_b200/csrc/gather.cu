@@ -14,6 +14,7 @@
 // Diff layout (include/utils.hpp:29-37, src/tree_approach.cpp:777-780):
 //   [header 32 B][u32 first node x F][(u32 ckpt, u32 count) x P][(u32 node, u32 prev) x S][data]
 // It is placed `delta` bytes into the device buffer so the data section is 16-byte aligned.
+#include "copy.cuh"
 #include "dedup_kernels.cuh"
 #include "map.cuh"
 #include "scan.cuh"
@@ -273,24 +274,6 @@ __global__ void __launch_bounds__(COMPACT_THREADS) diff_write_seg(SegGrid s) {
   diff_write_body(with_round(s.args[h]), bid, nb);
 }
 
-// warp-parallel lower bound: first index of sorted v[0..cnt) with v[idx] >= key (32-ary search)
-__device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t* v, uint32_t cnt, uint64_t key) {
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t lo = 0, hi = cnt;
-  while (hi - lo > 32u) {
-    const uint32_t step = (hi - lo + 31u) / 32u;
-    const uint32_t probe = lo + lane * step;
-    const bool below = probe < hi && v[probe] < key;
-    const uint32_t c = __popc(__ballot_sync(0xffffffffu, below));
-    const uint32_t nlo = c ? lo + (c - 1u) * step + 1u : lo;
-    const uint32_t nhi = (c < 32u && lo + c * step < hi) ? lo + c * step : hi;
-    lo = nlo;
-    hi = nhi;
-  }
-  const bool below = lo + lane < hi && v[lo + lane] < key;
-  return lo + __popc(__ballot_sync(0xffffffffu, below));
-}
-
 // ---------------------------------------------------------------- shifted duplicates, layout
 // Source checkpoints are counted in buckets relative to the last baseline, which emptied the
 // map: no entry is older, and a handle that has taken thousands of checkpoints sorts its entries
@@ -493,39 +476,6 @@ __device__ __forceinline__ void shift_write_range(const DiffArgs& a, uint32_t ra
   }
 }
 // ---------------------------------------------------------------- data gather
-// 16 bytes of the buffer from byte s on (s + 16 <= len), whatever its alignment: two aligned
-// 16-byte loads and a byte shift, or byte loads where an aligned load would leave the buffer
-__device__ __forceinline__ uint4 load_unit(const uint8_t* data, uint64_t len, uint64_t s) {
-  const uint8_t* p = data + s;
-  const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 15u);
-  if (mis == 0) return __ldg(reinterpret_cast<const uint4*>(p));
-  uint4 r;
-  if (s < mis || len - s < 32u - mis) {
-    uint8_t t[16];
-#pragma unroll
-    for (int b = 0; b < 16; b++) t[b] = p[b];
-    memcpy(&r, t, 16);
-    return r;
-  }
-  const uint4* q = reinterpret_cast<const uint4*>(p - mis);
-  const uint4 lo = __ldg(q), hi = __ldg(q + 1);
-  uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-  if (mis & 8u) {
-#pragma unroll
-    for (int i = 0; i < 6; i++) w[i] = w[i + 2];
-  }
-  if (mis & 4u) {
-#pragma unroll
-    for (int i = 0; i < 5; i++) w[i] = w[i + 1];
-  }
-  const uint32_t sh = 8u * (mis & 3u);
-  r.x = __funnelshift_r(w[0], w[1], sh);
-  r.y = __funnelshift_r(w[1], w[2], sh);
-  r.z = __funnelshift_r(w[2], w[3], sh);
-  r.w = __funnelshift_r(w[3], w[4], sh);
-  return r;
-}
-
 // a 16-byte unit of the data section that a region ends in, or whose source reaches past the
 // buffer's end (zeros, :643-645): byte by byte, region r holding its first byte
 struct GatherBytes {

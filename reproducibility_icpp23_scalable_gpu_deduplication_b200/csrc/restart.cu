@@ -267,15 +267,23 @@ __device__ __forceinline__ uint32_t find_entry(const uint32_t* off, uint32_t lo,
   const uint64_t per_ = ((count) + nw_ * 32u - 1u) / (nw_ * 32u) * 32u;                           \
   const uint64_t beg_ = w0_ * per_;                                                               \
   const uint64_t end_ = beg_ + per_ < (count) ? beg_ + per_ : (count);                            \
-  uint32_t ib_ = (!a.id_bias && beg_ < end_) ? find_entry((off), 0u, (cnt), beg_) : 0u;          \
+  uint32_t ib_ = (!a.id_bias && beg_ < end_) ? warp_lower_bound((off), (cnt), beg_ + 1u) - 1u : 0u; \
   for (uint64_t base = beg_; base < end_; base += 32u)
 
-// entry of position k of the current window, whose first position lies in entry ib; an entry
-// covering no position (only a malformed diff has one) sends the search past the window
+// entry of position k of the current window, whose first position lies in entry ib: the offsets of
+// the 32 entries from ib on are held one per lane and searched by shuffles (all lanes call it).  An
+// entry covering no position (only a malformed diff has one) sends the search past the window.
 __device__ __forceinline__ uint32_t window_entry(const uint32_t* off, uint32_t ib, uint32_t cnt, uint64_t k) {
-  const uint32_t hi = ib + 32u < cnt ? ib + 32u : cnt;
-  uint32_t i = find_entry(off, ib, hi, k);
-  if (i + 1u == hi && hi < cnt && off[hi] <= k) i = find_entry(off, hi, cnt, k);
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t o = ib + lane < cnt ? off[ib + lane] : 0xffffffffu;
+  uint32_t j = 0;
+#pragma unroll
+  for (uint32_t step = 16; step >= 1; step >>= 1) {
+    const uint32_t t = __shfl_sync(R_FULL, o, j + step);
+    if (ib + j + step < cnt && t <= k) j += step;
+  }
+  uint32_t i = ib + j;
+  if (j == 31u && i + 1u < cnt && off[i + 1u] <= k) i = find_entry(off, i, cnt, k);
   return i;
 }
 #define R_WINDOW_ENTRY(off, cnt, k) window_entry((off), ib_, (cnt), (k))
@@ -290,7 +298,7 @@ __device__ __forceinline__ void expand_first_body(const RestartArgs& a, uint32_t
     const uint64_t k = kb + lane;
     uint64_t dst = 0, nb = 0;
     const uint8_t* src = nullptr;
-    uint32_t i = ib_;
+    uint32_t i = a.id_bias ? ib_ : R_WINDOW_ENTRY(a.offs[0], a.F, k);
     if (k < end_) {
       uint32_t start, j, off0;
       if (a.id_bias) {   // one chunk per entry, at data offset k (src/list_approach.cpp:331-351)
@@ -299,7 +307,6 @@ __device__ __forceinline__ void expand_first_body(const RestartArgs& a, uint32_t
         j = 0;
         off0 = (uint32_t)k;
       } else {
-        i = R_WINDOW_ENTRY(a.offs[0], a.F, k);
         start = a.rstart[0][i];
         off0 = a.offs[0][i];
         j = (uint32_t)(k - off0);
@@ -416,7 +423,7 @@ __device__ __forceinline__ void expand_shift_body(const RestartArgs& a, uint32_t
     const uint64_t k = kb + lane;
     uint64_t dst = 0, nb = 0;
     const uint8_t* src = nullptr;
-    uint32_t i = ib_;
+    uint32_t i = a.id_bias ? ib_ : R_WINDOW_ENTRY(a.offs[1], a.S, k);
     if (k < end_) {
       uint32_t j, node_start, prev_start, tree;
       if (a.id_bias) {   // one chunk per entry (src/list_approach.cpp:371-408, :501-513)
@@ -426,7 +433,6 @@ __device__ __forceinline__ void expand_shift_body(const RestartArgs& a, uint32_t
         prev_start = rd_node(a, a.diff + a.shift_off + 8ull * k + 4);
         tree = shift_tree(a, k);
       } else {
-        i = R_WINDOW_ENTRY(a.offs[1], a.S, k);
         j = (uint32_t)(k - a.offs[1][i]);
         node_start = a.rstart[1][i];
         prev_start = a.pstart[i];

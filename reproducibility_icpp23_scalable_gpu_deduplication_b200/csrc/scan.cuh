@@ -42,6 +42,24 @@ __device__ __forceinline__ uint32_t block_reduce_sum(uint32_t v, uint32_t* sh) {
   return tot;
 }
 
+// warp-parallel lower bound: first index of sorted v[0..cnt) with v[idx] >= key (32-ary search)
+__device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t* v, uint32_t cnt, uint64_t key) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t lo = 0, hi = cnt;
+  while (hi - lo > 32u) {
+    const uint32_t step = (hi - lo + 31u) / 32u;
+    const uint32_t probe = lo + lane * step;
+    const bool below = probe < hi && v[probe] < key;
+    const uint32_t c = __popc(__ballot_sync(0xffffffffu, below));
+    const uint32_t nlo = c ? lo + (c - 1u) * step + 1u : lo;
+    const uint32_t nhi = (c < 32u && lo + c * step < hi) ? lo + c * step : hi;
+    lo = nlo;
+    hi = nhi;
+  }
+  const bool below = lo + lane < hi && v[lo + lane] < key;
+  return lo + __popc(__ballot_sync(0xffffffffu, below));
+}
+
 // contiguous range [beg, end) of `count` items owned by CTA b out of g
 __device__ __forceinline__ void cta_range(uint64_t count, uint32_t b, uint32_t g, uint64_t& beg, uint64_t& end) {
   const uint64_t per = (count + g - 1) / g;
