@@ -62,59 +62,21 @@ __device__ __forceinline__ void push_set(uint8_t* push, uint64_t x, uint32_t fla
   atomicOr(reinterpret_cast<uint32_t*>(push) + (y >> 4), flag << (2u * (uint32_t)(y & 15u)));
 }
 
-// phase-1 parent insert, priority 1 + height (:133, :390).  The rare heavy paths (hashing,
-// map probes) are kept out of line so the label folds stay small in the instruction cache.
-__device__ __noinline__ void insert_first_parent(const ForestArgs* self, uint32_t x, const Digest& d) {
-  const ForestArgs a = with_round(*self);
-  const uint32_t height = a.D - node_level(x);
-  const unsigned long long v = ((unsigned long long)(1u + height) << 32) | x;
+// phase-1 parent insert, priority 1 + height (:133, :390)
+__device__ __forceinline__ void insert_first_parent(const ForestArgs& a, uint32_t x, const Digest& d) {
   if (digest_zero(d)) *a.zero_exists = 1;
+  const unsigned long long v = ((unsigned long long)(1u + a.D - node_level(x)) << 32) | x;
   const MapRef ref = map_insert(a.map, d, v, a.cur, a.st);
   if (ref.found && !ref.inserted) map_merge_current(a.map, ref.slot, v, a.cur);
 }
 
-// Phase-1 parents are inserted together at the end of a band (or warp task), up to FF_GROUP
-// per thread at once.  B2D_FF_GROUPED 1: map_insert_group (all home reads, then all claims in
-// flight together); 0: one insert after another, each waiting for a DRAM read of its home slot
-// and then its atomics.  Measured with groups of 2: forest 0.173 against 0.176 ms per 4 GiB
-// step, batched step 12.67 against 12.87 ms; groups of 4 spill registers.  Prefetching each
-// group's home slots into L2 before inserting them one at a time was slower (0.185 ms and 13.30
-// ms; on the MD5 series 1.68 against 1.44 ms of forest per step).
-#ifndef B2D_FF_GROUPED
-#define B2D_FF_GROUPED 1
-#endif
-constexpr int FF_GROUP = 2;
-__device__ __forceinline__ void insert_first_parents(const ForestArgs& a, const uint32_t (&x)[FF_GROUP],
-                                                     const Digest (&d)[FF_GROUP], uint32_t cnt) {
-#pragma unroll
-  for (int j = 0; j < FF_GROUP; j++)
-    if ((uint32_t)j < cnt && digest_zero(d[j])) *a.zero_exists = 1;
-#if B2D_FF_GROUPED
-  Key128 k[FF_GROUP];
-  unsigned long long pv[FF_GROUP];
-  MapRef r[FF_GROUP];
-#pragma unroll
-  for (int j = 0; j < FF_GROUP; j++) {
-    k[j] = digest_key(d[j]);
-    pv[j] = map_pack(((unsigned long long)(1u + a.D - node_level(x[j])) << 32) | x[j], a.cur);
-  }
-  map_insert_group<FF_GROUP>(a.map, k, pv, cnt, r, a.st);
-#pragma unroll
-  for (int j = 0; j < FF_GROUP; j++)
-    if ((uint32_t)j < cnt && r[j].found && !r[j].inserted)
-      map_merge_current(a.map, r[j].slot, ((unsigned long long)(1u + a.D - node_level(x[j])) << 32) | x[j], a.cur);
-#else
-#pragma unroll
-  for (int j = 0; j < FF_GROUP; j++)
-    if ((uint32_t)j < cnt) insert_first_parent(a.self, x[j], d[j]);
-#endif
-}
-
+// The rare heavy paths (hashing, map probes) are kept out of line so the label folds stay small in
+// the instruction cache.
 __device__ __noinline__ void hash_first_parent(const ForestArgs* self, uint32_t x) {
   const ForestArgs a = with_round(*self);
   const Digest d = hash_pair(a.kind, a.tree[2u * x + 1u], a.tree[2u * x + 2u]);
   a.tree[x] = d;
-  insert_first_parent(self, x, d);
+  insert_first_parent(a, x, d);
 }
 
 // two shifted children: the parent is a shifted duplicate only if its digest is already known;
@@ -414,31 +376,20 @@ __device__ __forceinline__ void forest_first_body(const ForestArgs& a, uint32_t 
   }
   __syncthreads();
   const uint32_t total = wpre[FF_WORDS];
-  for (uint32_t r0 = t; r0 < total; r0 += FAST_THREADS * FF_GROUP) {
-    uint32_t xs[FF_GROUP], c = 0;
-    Digest ds[FF_GROUP];
-#pragma unroll
-    for (int j = 0; j < FF_GROUP; j++) {
-      const uint32_t r = r0 + FAST_THREADS * j;
-      xs[j] = 0;
-      ds[j].w[0] = ds[j].w[1] = ds[j].w[2] = ds[j].w[3] = 0u;
-      if (r >= total) continue;
-      uint32_t lo = 0, hi = FF_WORDS;   // word with wpre[w] <= r < wpre[w+1]
-      while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (wpre[mid] <= r) lo = mid; else hi = mid;
-      }
-      uint32_t word = ff[lo], skip = r - wpre[lo];
-      while (skip--) word &= word - 1u;   // drop the lower set bits
-      const uint32_t bit = lo * 32u + (__ffs(word) - 1u);
-      uint32_t k = 1;                     // band height of this bit
-      while (k < FF_LEVELS && bit >= ff_base(k + 1)) k++;
-      const uint64_t first = (root << (FF_LEVELS - k)) + (1ull << (FF_LEVELS - k)) - 1ull;
-      xs[j] = (uint32_t)(first + (bit - ff_base(k)));
-      ds[j] = a.tree[xs[j]];
-      c = j + 1;
+  for (uint32_t r = t; r < total; r += FAST_THREADS) {
+    uint32_t lo = 0, hi = FF_WORDS;   // word with wpre[w] <= r < wpre[w+1]
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (wpre[mid] <= r) lo = mid; else hi = mid;
     }
-    insert_first_parents(a, xs, ds, c);
+    uint32_t word = ff[lo], skip = r - wpre[lo];
+    while (skip--) word &= word - 1u;   // drop the lower set bits
+    const uint32_t bit = lo * 32u + (__ffs(word) - 1u);
+    uint32_t k = 1;                     // band height of this bit
+    while (k < FF_LEVELS && bit >= ff_base(k + 1)) k++;
+    const uint64_t first = (root << (FF_LEVELS - k)) + (1ull << (FF_LEVELS - k)) - 1ull;
+    const uint32_t x = (uint32_t)(first + (bit - ff_base(k)));
+    insert_first_parent(a, x, a.tree[x]);
   }
 }
 // The first band of a phase has one band per 1024 (phase 1) or 4096 (phase 2) leaves, most of
@@ -514,7 +465,7 @@ __device__ __forceinline__ void forest_fast_body(const ForestArgs& a, uint32_t b
       first = (first - 1ull) >> 1;
 #pragma unroll
       for (int j = 0; j < width; j++) {
-        // two FIXED children: an inner node, FIXED in an incremental checkpoint (fixed_or_node)
+        // two FIXED children: an inner node, FIXED in an incremental checkpoint
         if (PHASE == 2 && !a.baseline && v[2 * j] == FIXED_DUPL && v[2 * j + 1] == FIXED_DUPL) v[j] = FIXED_DUPL;
         else v[j] = combine<PHASE>(a, first + j, v[2 * j], v[2 * j + 1]);
       }
@@ -587,10 +538,10 @@ __global__ void __launch_bounds__(FAST_THREADS, B2D_FAST_MINB) forest_fast_seg(F
 constexpr uint32_t WB1_LEVELS = 7;
 constexpr uint32_t WB2_LEVELS = 9;
 constexpr uint32_t WB_THREADS = 256;
-// resident CTAs per SM the warp bands are compiled for (phase 1: 5, 48 registers; phase 2: 4,
-// 64 registers)
+// resident CTAs per SM the warp bands are compiled for (64 registers; phase 1 at 5 CTAs spilled:
+// MD5 floats 213 against 199 us)
 #ifndef B2D_WB1_MINB
-#define B2D_WB1_MINB 5
+#define B2D_WB1_MINB 4
 #endif
 #ifndef B2D_WB2_MINB
 #define B2D_WB2_MINB 4
@@ -630,37 +581,28 @@ __device__ __forceinline__ uint4 slot_labels16(const ForestArgs& a, const LeafSl
 
 // Parents a phase-1 warp task created, inserted into the map together once the task's hashing is
 // done (spread over the lanes): inserting each where it is hashed put a chain of dependent map
-// round trips on the lanes that carry the upper levels.  At most 127 per task of 128 leaves.
+// round trips on the lanes that carry the upper levels.  At most 127 per task of 128 leaves.  Each
+// parent's home slot is prefetched into L2 as it is recorded, so its insert waits for L2 and not
+// for memory, and one insert per lane at a time is enough: two in flight together, without the
+// prefetch, were slower (phase times of increments: 400 MB at 10 % 115 and 96 us, 1 GiB MD5 floats
+// 233 and 199 us), as was a CAS at every probe instead of a read first (MD5 floats 308 us: the
+// zero pages' parents share slots).
 struct WarpInserts {
   uint32_t* node;   // 128 entries of this warp's buffer in shared memory
   Digest* dig;
   uint32_t* count;
+  MapView map;
 };
 __device__ __forceinline__ void wi_add(const WarpInserts& wi, uint32_t x, const Digest& d) {
   const uint32_t pos = atomicAdd(wi.count, 1u);
   wi.node[pos] = x;
   wi.dig[pos] = d;
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(map_key(wi.map, map_home(digest_key(d), wi.map.cap))));
 }
 __device__ __forceinline__ void wi_flush(const ForestArgs& a, const WarpInserts& wi, uint32_t lane) {
   __syncwarp();
   const uint32_t cnt = *wi.count;
-  // lane takes entries lane, lane + 32, ... in groups of FF_GROUP
-  for (uint32_t r0 = lane; r0 < cnt; r0 += 32u * FF_GROUP) {
-    uint32_t x[FF_GROUP], c = 0;
-    Digest d[FF_GROUP];
-#pragma unroll
-    for (int j = 0; j < FF_GROUP; j++) {
-      const uint32_t r = r0 + 32u * j;
-      x[j] = 0;
-      d[j].w[0] = d[j].w[1] = d[j].w[2] = d[j].w[3] = 0u;
-      if (r < cnt) {
-        x[j] = wi.node[r];
-        d[j] = wi.dig[r];
-        c = j + 1;
-      }
-    }
-    insert_first_parents(a, x, d, c);
-  }
+  for (uint32_t r = lane; r < cnt; r += 32u) insert_first_parent(a, wi.node[r], wi.dig[r]);
   __syncwarp();
   if (lane == 0) *wi.count = 0;
   __syncwarp();
@@ -737,7 +679,7 @@ __device__ __forceinline__ void warp1_task(const ForestArgs& a, uint32_t task, u
   }
   // heights 3..7: shuffles; lane 0 ends at the task root
   if (__any_sync(0xffffffffu, b)) {
-#pragma unroll
+#pragma unroll 1   // one copy of the hash: unrolled, the task outgrew the instruction caches
     for (int s = 0; s < 5; s++) {
       const uint32_t rb = __shfl_down_sync(0xffffffffu, b, 1u << s);
       const Digest rd = shfl_down_digest(dg, 1u << s);
@@ -758,49 +700,114 @@ __device__ __forceinline__ void warp1_task(const ForestArgs& a, uint32_t task, u
   wi_flush(a, wi, lane);
 }
 
-// Phase-2 parent of two FIXED children in an incremental checkpoint: FIXED, with nothing pushed
-// or looked up, so the call is skipped.  A task of 512 leaves almost always holds a few scattered
-// shifted copies (0.5 % of the plain series' chunks), so most tasks take the slow path, and most
-// of their nodes are still FIXED pairs.
-__device__ __forceinline__ uint8_t fixed_or_node(const ForestArgs& a, uint32_t x, uint8_t ll, uint8_t rl) {
-  if (!a.baseline && ll == FIXED_DUPL && rl == FIXED_DUPL) return FIXED_DUPL;
-  return forest_node<2>(a, x, ll, rl);
+// one bit per byte of w that equals the byte `v` (0 .. 4): bits 0 .. 3
+__device__ __forceinline__ uint32_t bytes_equal(uint32_t w, uint32_t v) {
+  const uint32_t eq = __vcmpeq4(w, v * 0x01010101u) & 0x08040201u;
+  return (eq * 0x01010101u) >> 24;
+}
+// bits 0 .. 15 to the even bits
+__device__ __forceinline__ uint32_t spread16(uint32_t v) {
+  v = (v | v << 8) & 0x00ff00ffu;
+  v = (v | v << 4) & 0x0f0f0f0fu;
+  v = (v | v << 2) & 0x33333333u;
+  return (v | v << 1) & 0x55555555u;
+}
+// what a baseline does at a parent besides its label
+__device__ __forceinline__ void baseline_node(const ForestArgs& a, uint32_t x, bool first) {
+  if (!first) {
+    if (a.lost) bulk_settle(a.self, x, false);
+    else baseline_parent(a.self, x);
+  } else if (a.lost_seen && ((a.lost[x >> 5] >> (x & 31u)) & 1u)) {
+    bulk_settle(a.self, x, true);
+  }
+}
+
+// The phase-2 rules (forest_node<2>) over a lane's 16 leaves, as bit sets: bit i of `fixed`, `first`
+// and `shift` is the label of slot i (none: DONE), and at height h the nodes sit at the multiples
+// of 2^h.  Whole levels are decided by a few logic operations, and only shifted pairs, a baseline's
+// parents and region roots are gone through one by one, in loops that are not unrolled: written out
+// node by node the fold was 15 copies of the rule, and its warps spent two thirds of their time
+// waiting for instructions (26 us of a 400 MB increment).
+__device__ __forceinline__ uint8_t fold16(const ForestArgs& a, uint64_t x0, const uint4& w) {
+  uint32_t fixed = bytes_equal(w.x, FIXED_DUPL) | bytes_equal(w.y, FIXED_DUPL) << 4 |
+                   bytes_equal(w.z, FIXED_DUPL) << 8 | bytes_equal(w.w, FIXED_DUPL) << 12;
+  uint32_t first = bytes_equal(w.x, FIRST_OCUR) | bytes_equal(w.y, FIRST_OCUR) << 4 |
+                   bytes_equal(w.z, FIRST_OCUR) << 8 | bytes_equal(w.w, FIRST_OCUR) << 12;
+  uint32_t shift = bytes_equal(w.x, SHIFT_DUPL) | bytes_equal(w.y, SHIFT_DUPL) << 4 |
+                   bytes_equal(w.z, SHIFT_DUPL) << 8 | bytes_equal(w.w, SHIFT_DUPL) << 12;
+  uint64_t base = x0;            // node of bit 0 at this height
+  uint32_t grid = 0x5555u;       // bits of this height's nodes: multiples of 2^h
+#pragma unroll 1
+  for (uint32_t h = 1; h <= 4; h++) {
+    const uint32_t d = 1u << (h - 1u);   // distance of a pair's halves
+    const uint64_t child = base;
+    base = (base - 1ull) >> 1;
+    // nodes of this height that are leaves themselves (level D-1 of a tree whose chunk count is not
+    // a power of two): both halves carry their label, which passes on
+    uint32_t leaf = 0;
+    if (h == 1u && base + 7ull >= a.n - 1u) {
+      const uint32_t inner = base >= a.n - 1u ? 0u : (uint32_t)(a.n - 1u - base);   // of the 8 nodes
+      leaf = grid & ~((1u << (2u * inner)) - 1u);
+    }
+    const uint32_t done = ~(fixed | first | shift);
+    uint32_t xf = fixed & (fixed >> d) & grid, ff = first & (first >> d) & grid;
+    uint32_t ss = shift & (shift >> d) & grid;
+    const uint32_t dd = done & (done >> d) & grid;
+    const uint32_t mixed = grid & ~(xf | ff | ss | dd);
+    uint32_t sout = ss & leaf;
+    ss &= ~leaf;
+    // differing children become region roots
+    const uint32_t both = mixed | mixed << d;
+    uint32_t pf = both & first, ps = both & shift;
+    if (pf | ps) {
+      if (h == 1u) {   // 16 leaves are one word of flags
+        atomicOr(reinterpret_cast<uint32_t*>(a.push) + ((x0 + 1ull) >> 4), spread16(pf) * PUSH_FIRST | spread16(ps) * PUSH_SHIFT);
+      } else {
+        for (uint32_t m = pf | ps; m; m &= m - 1u) {
+          const uint32_t b = __ffs(m) - 1u;
+          push_set(a.push, child + (b >> (h - 1u)), (pf >> b) & 1u ? PUSH_FIRST : PUSH_SHIFT);
+        }
+      }
+    }
+    for (; ss; ss &= ss - 1u) {
+      const uint32_t b = __ffs(ss) - 1u;
+      if (shift_pair(a.self, (uint32_t)(base + (b >> h))) == SHIFT_DUPL) sout |= 1u << b;
+    }
+    if (a.baseline) {
+      uint32_t m = grid & ~leaf;
+      if (!a.lost_seen) m &= ~ff;   // nothing to settle at first occurrences
+      for (; m; m &= m - 1u) {
+        const uint32_t b = __ffs(m) - 1u;
+        baseline_node(a, (uint32_t)(base + (b >> h)), (ff >> b) & 1u);
+      }
+    }
+    fixed = xf;
+    first = ff;
+    shift = sout;
+    grid &= h == 1u ? 0x1111u : h == 2u ? 0x0101u : 0x0001u;
+  }
+  return fixed & 1u ? FIXED_DUPL : first & 1u ? FIRST_OCUR : shift & 1u ? SHIFT_DUPL : DONE;
 }
 
 __device__ __forceinline__ void warp2_task(const ForestArgs& a, uint32_t task, uint32_t lane, const uint4& w) {
   const uint64_t root = ((1ull << (a.D - WB2_LEVELS)) - 1ull) + task;
   const uint64_t x0 = (1ull << a.D) - 1ull + task * 512u + 16u * lane;
-  bool fast = !a.baseline && w.x == 0x01010101u && w.y == 0x01010101u && w.z == 0x01010101u &&
-              w.w == 0x01010101u;   // all 16 leaves FIXED
+  const bool fast = !a.baseline && w.x == 0x01010101u && w.y == 0x01010101u && w.z == 0x01010101u &&
+                    w.w == 0x01010101u;   // all 16 leaves FIXED
   if (__all_sync(0xffffffffu, fast)) {
     if (lane == 0) band_output<2>(a, root, FIXED_DUPL);
     return;
   }
   uint8_t lab = FIXED_DUPL;
-  if (!fast) {
-    uint8_t v[16];
-    const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-    for (int j = 0; j < 16; j++) v[j] = (uint8_t)(ws[j >> 2] >> (8 * (j & 3)));
-    uint64_t first = x0;
-#pragma unroll
-    for (int width = 8; width >= 1; width >>= 1) {
-      first = (first - 1ull) >> 1;
-#pragma unroll
-      for (int j = 0; j < width; j++) {
-        if (width == 8 && first + j >= a.n - 1u) v[j] = v[2 * j];   // a leaf of level D-1
-        else v[j] = fixed_or_node(a, (uint32_t)(first + j), v[2 * j], v[2 * j + 1]);
-      }
-    }
-    lab = v[0];
-  }
+  if (!fast) lab = fold16(a, x0, w);
   uint64_t y = ((x0 + 1ull) >> 4) - 1ull;   // the lane's 16-leaf subtree root
-#pragma unroll
+#pragma unroll 1
   for (int s = 0; s < 5; s++) {
     __syncwarp();   // digests written by the partner lane at the previous level are visible
     const uint8_t rl = (uint8_t)__shfl_down_sync(0xffffffffu, (uint32_t)lab, 1u << s);
     if ((lane & ((2u << s) - 1u)) == 0) {
       y = (y - 1ull) >> 1;
+      // two FIXED children in an incremental checkpoint: FIXED, with nothing pushed or looked up
       if (a.baseline || lab != FIXED_DUPL || rl != FIXED_DUPL) lab = forest_node<2>(a, (uint32_t)y, lab, rl);
     }
   }
@@ -830,7 +837,7 @@ constexpr uint32_t WB_FULL = 0xffffffffu;
   __shared__ uint32_t wi_node_[WB_THREADS / 32u][128];                                          \
   __shared__ Digest wi_dig_[WB_THREADS / 32u][128];                                             \
   __shared__ uint32_t wi_count_[WB_THREADS / 32u];                                              \
-  const WarpInserts wi{wi_node_[threadIdx.x >> 5], wi_dig_[threadIdx.x >> 5], &wi_count_[threadIdx.x >> 5]}; \
+  const WarpInserts wi{wi_node_[threadIdx.x >> 5], wi_dig_[threadIdx.x >> 5], &wi_count_[threadIdx.x >> 5], wi_map_}; \
   if ((threadIdx.x & 31u) == 0) *wi.count = 0;                                                  \
   __syncwarp();
 
@@ -871,12 +878,13 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB1_MINB)
     forest_warp1_kernel(const __grid_constant__ ForestArgs a0, uint32_t ntasks, uint32_t queue) {
   griddep_enter();
   stamp_start(a0);
+  const ForestArgs a = with_round(a0);
+  const MapView wi_map_ = a.map;
   B2D_WARP_INSERT_BUFFERS
   B2D_WARP_QUEUE_BUFFERS
-  const ForestArgs a = with_round(a0);
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t G = (gridDim.x * WB_THREADS) >> 5;
-  const uint32_t w0 = (blockIdx.x * WB_THREADS + threadIdx.x) >> 5;
+  const uint32_t w0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;   // neighbouring tasks go to different CTAs
   const LeafSlots q = leaf_slots(a);
   auto labels = [&](uint32_t task) { return slot_labels4(a, q, task * 128u + 4u * lane); };
   if (!queue) {
@@ -926,7 +934,7 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB2_MINB)
   const ForestArgs a = with_round(a0);
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t G = (gridDim.x * WB_THREADS) >> 5;
-  const uint32_t w0 = (blockIdx.x * WB_THREADS + threadIdx.x) >> 5;
+  const uint32_t w0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;   // neighbouring tasks go to different CTAs
   const LeafSlots q = leaf_slots(a);
   auto labels = [&](uint32_t task) { return slot_labels16(a, q, task * 512u + 16u * lane); };
   if (!queue) {
@@ -977,10 +985,11 @@ __global__ void __launch_bounds__(WB_THREADS, B2D_WB2_MINB)
 // Segmented warp bands (batched form): CTA b of a handle's range holds its tasks 8b .. 8b+7,
 // one per warp.
 __global__ void __launch_bounds__(WB_THREADS) forest_warp1_seg(ForestSeg s) {
-  B2D_WARP_INSERT_BUFFERS
   uint32_t bid, nb;
   const uint32_t h = seg_find(s.beg, s.n, bid, nb);
   const ForestArgs a = with_round(s.args[h]);
+  const MapView wi_map_ = a.map;
+  B2D_WARP_INSERT_BUFFERS
   const uint32_t task = bid * (WB_THREADS / 32u) + (threadIdx.x >> 5);
   if (task >= (1u << (a.D - WB1_LEVELS))) return;
   const uint32_t lane = threadIdx.x & 31u;

@@ -273,15 +273,18 @@ __host__ __device__ __forceinline__ Digest hash_bytes(int kind, const uint8_t* p
 
 // Inner node digest: hash of the 32 bytes left-child digest || right-child digest
 // (src/tree_approach.cpp:131,221,389,459 of the reference).
+// MD5's is out of line: its 64 steps in each of a kernel's hashes made the kernels outgrow the
+// instruction caches, whichever hash they ran.
+static __device__ __noinline__ Digest hash_pair_md5(Digest l, Digest r) {
+  uint32_t st[4];
+  md5_init(st);
+  uint32_t m[16] = {l.w[0], l.w[1], l.w[2], l.w[3], r.w[0], r.w[1], r.w[2], r.w[3],
+                    0x80u, 0u, 0u, 0u, 0u, 0u, 256u, 0u};
+  md5_compress(st, m);
+  return md5_digest(st);
+}
 __device__ __forceinline__ Digest hash_pair(int kind, const Digest& l, const Digest& r) {
-  if (kind == HASH_MD5) {
-    uint32_t st[4];
-    md5_init(st);
-    uint32_t m[16] = {l.w[0], l.w[1], l.w[2], l.w[3], r.w[0], r.w[1], r.w[2], r.w[3],
-                      0x80u, 0u, 0u, 0u, 0u, 0u, 256u, 0u};
-    md5_compress(st, m);
-    return md5_digest(st);
-  }
+  if (kind == HASH_MD5) return hash_pair_md5(l, r);
   Murmur3 h;
   h.init();
   h.block_words(l.w[0], l.w[1], l.w[2], l.w[3]);
