@@ -39,4 +39,19 @@ __device__ __forceinline__ uint4 load_unit(const uint8_t* data, uint64_t len, ui
   return r;
 }
 
+// an asynchronous copy of a 16-byte piece to shared memory (`bytes` of it, the rest zeros)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// 16 bytes from byte m (< 16) of a piece on, the rest from the next piece
+__device__ __forceinline__ uint4 shift_piece(const uint4& lo, const uint4& hi, uint32_t m) {
+  uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+  for (int i = 0; i < 6; i++) w[i] = m & 8u ? w[i + 2] : w[i];
+#pragma unroll
+  for (int i = 0; i < 5; i++) w[i] = m & 4u ? w[i + 1] : w[i];
+  const uint32_t s = 8u * (m & 3u);
+  return make_uint4(__funnelshift_r(w[0], w[1], s), __funnelshift_r(w[1], w[2], s), __funnelshift_r(w[2], w[3], s),
+                    __funnelshift_r(w[3], w[4], s));
+}
 }  // namespace b2d

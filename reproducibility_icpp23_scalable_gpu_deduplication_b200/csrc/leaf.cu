@@ -11,6 +11,7 @@
 //   * leaf_any_kernel: any chunk size or alignment, one chunk per lane streamed through shared
 //     memory in aligned pieces.
 #include <cuda.h>
+#include "copy.cuh"
 #include "dedup_kernels.cuh"
 #include "hash.cuh"
 #include "map.cuh"
@@ -297,20 +298,6 @@ __device__ __forceinline__ uint32_t swz(uint32_t o) {
 constexpr uint32_t ANY_WARPS = 8;
 constexpr uint32_t ANY_STAGES = 3;
 constexpr uint32_t ANY_STAGE_BYTES = 32u * 128u;
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-// 16 bytes from byte m (< 16) of a piece on, the rest from the next piece
-__device__ __forceinline__ uint4 shift_piece(const uint4& lo, const uint4& hi, uint32_t m) {
-  uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-  for (int i = 0; i < 6; i++) w[i] = m & 8u ? w[i + 2] : w[i];
-#pragma unroll
-  for (int i = 0; i < 5; i++) w[i] = m & 4u ? w[i + 1] : w[i];
-  const uint32_t s = 8u * (m & 3u);
-  return make_uint4(__funnelshift_r(w[0], w[1], s), __funnelshift_r(w[1], w[2], s), __funnelshift_r(w[2], w[3], s),
-                    __funnelshift_r(w[3], w[4], s));
-}
 // the low `n` bytes of a word (all for n >= 4)
 __device__ __forceinline__ uint32_t low_bytes(uint32_t v, uint32_t n) {
   return n >= 4u ? v : v & ((1u << (8u * n)) - 1u);

@@ -25,6 +25,7 @@
 // the stores stay 16 bytes wide) and every load and store instruction covers whole sectors.
 // Every index and copy is bounds-checked: a diff that would make the reference read or write
 // outside a buffer sets DERR_RESTART_RANGE and the access is skipped.
+#include "copy.cuh"
 #include "restart.cuh"
 #include "scan.cuh"
 
@@ -481,72 +482,159 @@ __global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_expand_shift_se
 // (their leaf, main id - 1), as the reference's node_list does (:933-939).  A chunk's NodeID
 // usually stays its own leaf all the way down, so that leaf's flags in every slot are loaded up
 // front, side by side; another leaf's flags are loaded when the walk reaches it.
+// Returns the source of chunk c (null: nothing to copy), its bytes in *nb_out and the end of the
+// data section it lies in in *end_out.
+__device__ __forceinline__ const uint8_t* walk_source(const RestartWalk& w, uint64_t c, uint64_t* nb_out,
+                                                      const uint8_t** end_out) {
+  const uint64_t dst = c * w.cs;
+  uint64_t nb = 0;
+  const uint8_t* src = nullptr;
+  const uint8_t* end = nullptr;
+  if (c < w.n) {
+    const uint32_t own = (uint32_t)c + w.n - 1u;   // heap index of chunk c's leaf
+    uint32_t pf = 0;                                // 2 flag bits per slot for leaf `own`
+#pragma unroll
+    for (uint32_t k = 0; k < RESTART_WINDOW; k++)
+      if (k < w.count) pf |= (uint32_t)w.slot[k].flag[c] << (2u * k);
+    uint2 id;
+    if (w.dense) {
+      id = w.node_list[c];
+    } else {
+      id = make_uint2(own, w.main_cur - 1u);
+      if (w.mflag[c]) {
+        const uint2 m = w.node_list[c];
+        if (m.x != 0xffffffffu) id = m;
+      }
+    }
+    const uint2 id0 = id;
+#pragma unroll
+    for (uint32_t k = 0; k < RESTART_WINDOW; k++) {
+      if (k >= w.count) break;
+      const uint32_t cur = w.cur[k];
+      if (id.y != cur) continue;
+      const RestartSlot s = w.slot[k];
+      uint64_t ws = w.cs;
+      if (dst + ws > w.datalen[k]) ws = w.datalen[k] - dst;
+      const uint64_t lc = (uint64_t)id.x - (w.n - 1u);
+      const bool leaf = id.x >= w.n - 1u && lc < w.n;
+      const uint32_t f = !leaf ? 0u : id.x == own ? (pf >> (2u * k)) & 3u : (uint32_t)s.flag[lc];
+      if (f & R_HAS_DIST) {
+        const uint8_t* p =
+            checked_src(w.data[k], w.data_len[k], w.out_len, dst, (uint64_t)s.dist[lc] * w.cs, ws, w.st);
+        if (p) {
+          src = p;
+          nb = ws;
+          end = w.data[k] + w.data_len[k];
+        }
+      } else if ((f & R_HAS_REP) && s.rep[lc].x != 0xffffffffu) {
+        const uint2 prev = s.rep[lc];
+        if (prev.y == cur) {
+          const uint64_t pc = (uint64_t)prev.x - (w.n - 1u);
+          if (prev.x >= w.n - 1u && pc < w.n && (s.flag[pc] & R_HAS_DIST)) {
+            const uint8_t* p =
+                checked_src(w.data[k], w.data_len[k], w.out_len, dst, (uint64_t)s.dist[pc] * w.cs, ws, w.st);
+            if (p) {
+              src = p;
+              nb = ws;
+              end = w.data[k] + w.data_len[k];
+            }
+          } else {
+            set_error(w.st, DERR_RESTART_RANGE, 4);
+          }
+        } else {
+          id = prev;
+        }
+      } else {
+        id = make_uint2(id.x, cur - 1u);
+      }
+    }
+    if (!w.last && (!w.dense || id.x != id0.x || id.y != id0.y)) w.node_list[c] = id;
+  }
+  *nb_out = nb;
+  *end_out = end;
+  return src;
+}
+
 __global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_walk_kernel(const __grid_constant__ RestartWalk w) {
   griddep_enter();
   R_WARP_LOOP(cb, w.n) {
-    const uint64_t c = cb + lane;
-    const uint64_t dst = c * w.cs;
-    uint64_t nb = 0;
-    const uint8_t* src = nullptr;
-    if (c < w.n) {
-      const uint32_t own = (uint32_t)c + w.n - 1u;   // heap index of chunk c's leaf
-      uint32_t pf = 0;                                // 2 flag bits per slot for leaf `own`
-#pragma unroll
-      for (uint32_t k = 0; k < RESTART_WINDOW; k++)
-        if (k < w.count) pf |= (uint32_t)w.slot[k].flag[c] << (2u * k);
-      uint2 id;
-      if (w.dense) {
-        id = w.node_list[c];
-      } else {
-        id = make_uint2(own, w.main_cur - 1u);
-        if (w.mflag[c]) {
-          const uint2 m = w.node_list[c];
-          if (m.x != 0xffffffffu) id = m;
-        }
-      }
-      const uint2 id0 = id;
-#pragma unroll
-      for (uint32_t k = 0; k < RESTART_WINDOW; k++) {
-        if (k >= w.count) break;
-        const uint32_t cur = w.cur[k];
-        if (id.y != cur) continue;
-        const RestartSlot s = w.slot[k];
-        uint64_t ws = w.cs;
-        if (dst + ws > w.datalen[k]) ws = w.datalen[k] - dst;
-        const uint64_t lc = (uint64_t)id.x - (w.n - 1u);
-        const bool leaf = id.x >= w.n - 1u && lc < w.n;
-        const uint32_t f = !leaf ? 0u : id.x == own ? (pf >> (2u * k)) & 3u : (uint32_t)s.flag[lc];
-        if (f & R_HAS_DIST) {
-          const uint8_t* p =
-              checked_src(w.data[k], w.data_len[k], w.out_len, dst, (uint64_t)s.dist[lc] * w.cs, ws, w.st);
-          if (p) {
-            src = p;
-            nb = ws;
-          }
-        } else if ((f & R_HAS_REP) && s.rep[lc].x != 0xffffffffu) {
-          const uint2 prev = s.rep[lc];
-          if (prev.y == cur) {
-            const uint64_t pc = (uint64_t)prev.x - (w.n - 1u);
-            if (prev.x >= w.n - 1u && pc < w.n && (s.flag[pc] & R_HAS_DIST)) {
-              const uint8_t* p =
-                  checked_src(w.data[k], w.data_len[k], w.out_len, dst, (uint64_t)s.dist[pc] * w.cs, ws, w.st);
-              if (p) {
-                src = p;
-                nb = ws;
-              }
-            } else {
-              set_error(w.st, DERR_RESTART_RANGE, 4);
-            }
-          } else {
-            id = prev;
-          }
-        } else {
-          id = make_uint2(id.x, cur - 1u);
-        }
-      }
-      if (!w.last && (!w.dense || id.x != id0.x || id.y != id0.y)) w.node_list[c] = id;
+    uint64_t nb;
+    const uint8_t* end;
+    const uint8_t* src = walk_source(w, cb + lane, &nb, &end);
+    warp_copy(w.out, w.cs, w.width, w.per, w.per_log2, (cb + lane) * w.cs, src, nb);
+  }
+}
+
+// The walk with its copies staged through shared memory: each warp resolves 32 chunks, issues their
+// bytes as asynchronous 16-byte pieces (cp.async) and, while they are on their way, writes out the
+// 32 chunks before.  A warp's loads so overlap the next group's lookups, and none of them holds a
+// register: a restart of 1 GiB from five device diffs takes 640 us, through registers, four pieces a
+// lane at a time, 668 us.  A source is fetched from the 16-byte boundary before it on, one piece
+// more than the chunk has, and shifted into place when it is written, so sources of any alignment
+// move in whole pieces.  For 16-byte aligned outputs and chunk sizes that are multiples of 16 up to
+// STAGE_CHUNK (larger ones have enough in flight as it is).
+constexpr uint32_t WALK_WARPS = 4;
+constexpr uint32_t STAGE_CHUNK = 128;
+constexpr uint32_t STAGE_BYTES = 32u * (STAGE_CHUNK + 16u);
+__device__ __forceinline__ void stage_write(const RestartWalk& w, const uint8_t* stage, uint64_t cb, uint32_t mis,
+                                            bool staged) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t per = w.per, row = per + 1u;
+  uint4* out = reinterpret_cast<uint4*>(w.out + cb * w.cs);
+  const uint32_t state = mis | (staged ? 16u : 0u);
+#pragma unroll 4
+  for (uint32_t u = lane; u < 32u * per; u += 32u) {
+    const uint32_t j = w.per_log2 != 0xffu ? u >> w.per_log2 : u / per;
+    const uint32_t st = __shfl_sync(R_FULL, state, j);
+    const uint4* p = reinterpret_cast<const uint4*>(stage) + j * row + (u - j * per);
+    if (st & 16u) out[u] = shift_piece(p[0], p[1], st & 15u);
+  }
+}
+__global__ void __launch_bounds__(WALK_WARPS * 32, 6) r_walk_staged_kernel(const __grid_constant__ RestartWalk w) {
+  extern __shared__ __align__(16) uint8_t walk_smem[];
+  griddep_enter();
+  uint8_t* ring = walk_smem + (threadIdx.x >> 5) * (2u * STAGE_BYTES);
+  const uint32_t ring32 = (uint32_t)__cvta_generic_to_shared(ring);
+  const uint32_t row = w.per + 1u;
+  const uint32_t magic = 65536u / row + 1u;   // i / row for i < 32 * 9: exact
+  uint64_t prev_cb = 0;
+  uint32_t prev_mis = 0, k = 0;
+  bool prev_staged = false;
+  R_WARP_LOOP(cb, w.n) {
+    uint64_t nb;
+    const uint8_t* end;
+    const uint8_t* src = walk_source(w, cb + lane, &nb, &end);
+    const uint32_t mis = (uint32_t)(uintptr_t)src & 15u;
+    // the last piece must not leave the data section; a short chunk and one at the section's very
+    // end are copied by their lane
+    const bool staged = src && nb == w.cs && (mis == 0u || src + nb + (16u - mis) <= end);
+    const uint64_t first = reinterpret_cast<uint64_t>(src) - mis;
+    const uint32_t slot = (k & 1u) * STAGE_BYTES;
+#pragma unroll 3
+    for (uint32_t i = lane; i < 32u * row; i += 32u) {
+      const uint32_t j = (i * magic) >> 16, q = i - j * row;
+      const uint64_t s = __shfl_sync(R_FULL, first, j);
+      const uint32_t st = __shfl_sync(R_FULL, mis | (staged ? 16u : 0u), j);
+      if ((st & 16u) && (q < w.per || (st & 15u)))
+        cp_async16(ring32 + slot + 16u * i, reinterpret_cast<const void*>(s + 16u * q), 16u);
     }
-    warp_copy(w.out, w.cs, w.width, w.per, w.per_log2, dst, src, nb);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (src && !staged) copy_bytes(w.out + (cb + lane) * w.cs, src, nb);
+    if (k > 0u) {
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncwarp();
+      stage_write(w, ring + (STAGE_BYTES - slot), prev_cb, prev_mis, prev_staged);
+      __syncwarp();   // read before the next group's pieces land in it
+    }
+    prev_cb = cb;
+    prev_mis = mis;
+    prev_staged = staged;
+    k++;
+  }
+  if (k > 0u) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+    stage_write(w, ring + ((k - 1u) & 1u) * STAGE_BYTES, prev_cb, prev_mis, prev_staged);
   }
 }
 
@@ -713,6 +801,14 @@ cudaError_t launch_restart_walk(const RestartWalk& walk, int sm_count, cudaStrea
   uint64_t src_al = 0;
   for (uint32_t k = 0; k < w.count; k++) src_al |= (uint64_t)(uintptr_t)w.data[k];
   copy_width((uint64_t)(uintptr_t)w.out, src_al, w.cs, w.width, w.per, w.per_log2);
+  if (w.width == 16u && w.cs <= STAGE_CHUNK) {
+    constexpr size_t smem = WALK_WARPS * 2u * STAGE_BYTES;
+    const cudaError_t e =
+        cudaFuncSetAttribute(r_walk_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const uint64_t want = ceil_div_u64(w.n, 32u * WALK_WARPS), cap = (uint64_t)sm_count * 24u;   // four waves even out the ends
+    return launch_dependent(r_walk_staged_kernel, (uint32_t)(want < cap ? want : cap), WALK_WARPS * 32u, smem, s, w);
+  }
   return launch_dependent(r_walk_kernel, grid_for(w.n, sm_count), R_THREADS, 0, s, w);
 }
 
