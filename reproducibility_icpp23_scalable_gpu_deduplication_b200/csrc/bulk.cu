@@ -11,9 +11,9 @@
 //   build       makes each range of the table in shared memory and writes it out once, empty slots
 //               included (the table is not cleared before).
 // All of it streams: per node 16 bytes read twice, 20 written and read once per scatter pass, and
-// the table written once.  Whole baselines at 128 B chunks: 4 GiB 11.1, now 7.3 ms; 64 MiB 380, now
-// 230 us.  Of the 4 GiB's 5.0 ms here the writing of the 8.6 GB table takes 2.7 and the scatter
-// passes 1.5.
+// the table written once.  Whole baselines at 128 B chunks: 4 GiB 11.1, now 6.4 ms; 64 MiB 380, now
+// 220 us.  Of the 4 GiB's 4.2 ms here the writing of the 8.6 GB table takes 2.2 and the scatter
+// passes 1.35.
 //
 // The result is the map the one-by-one inserts leave (src/tree_approach.cpp:54-94, 116-145,
 // 218-224 in sequential order): an entry is owned by its lowest leaf, else by its lowest
@@ -509,8 +509,13 @@ cudaError_t launch_bulk(const BulkArgs& args, int sm_count, cudaStream_t stream,
   BulkArgs a = args;
   cudaError_t e = cudaSuccess;
   uint32_t c = 0;
+  // Large builds' kernels are launched the ordinary way: with the next kernel's CTAs let in while the
+  // one before drains, its resident grid fills the SMs unevenly and late, and as each CTA has its
+  // fixed share, all wait for the last (4 GiB: scatter passes 750 and 750 against 720 and 620 us,
+  // build 2.75 against 2.16 ms).  Small ones are bound by the launches themselves.
+  const bool early = a.n < (1u << 20);
 #define B2D_LD(...)                                              \
-  if ((e = launch_dependent(__VA_ARGS__)) != cudaSuccess) return e; \
+  if ((e = launch_early(early, __VA_ARGS__)) != cudaSuccess) return e; \
   c++;
   if (!a.list) {
     uint32_t in = a.D;   // >= 15
