@@ -1018,22 +1018,33 @@ int do_restart(b2d_dedup* d, void* d_out, uint64_t len, const uint8_t* const* di
       k = q.end;
     }
   };
+  auto reserve = [&]() {
+    cudaError_t e = ddiffs ? cudaSuccess : d->r_diff.reserve(max_bytes);
+    if (e == cudaSuccess) e = d->r_node_list.reserve(n);
+    if (e == cudaSuccess) e = d->r_mflag.reserve(n);
+    if (e == cudaSuccess) e = d->r_dist.reserve((uint64_t)n * max_count);
+    if (e == cudaSuccess) e = d->r_rep.reserve((uint64_t)n * max_count);
+    if (e == cudaSuccess) e = d->r_flag.reserve((uint64_t)n * max_count);
+    if (e == cudaSuccess) e = d->r_offs.reserve(std::max<uint64_t>(max_lists, 1));
+    if (e == cudaSuccess) e = d->r_partial.reserve(2 * SCAN_GRID * max_count);
+    if (e == cudaSuccess) e = d->r_cum.reserve(max_cum);
+    if (e == cudaSuccess) e = d->r_total.reserve(2 * max_count);
+    if (e == cudaSuccess) e = d->r_straddle.reserve(max_count);
+    return e;
+  };
   plan(window, ddiffs ? ~0ull : RESTART_SLOT_BYTES);
-  if (!ddiffs && d->r_diff.reserve(max_bytes) != cudaSuccess) {
+  cudaError_t re = reserve();
+  if (re == cudaErrorMemoryAllocation) {   // too little device memory for a window: one diff at a time
     (void)cudaGetLastError();
-    plan(1, 0);   // one diff at a time
-    B2D_CU(d->r_diff.reserve(max_bytes));
+    d->r_diff.release();
+    d->r_dist.release();
+    d->r_rep.release();
+    d->r_flag.release();
+    d->r_offs.release();
+    plan(1, 0);
+    re = reserve();
   }
-  B2D_CU(d->r_node_list.reserve(n));
-  B2D_CU(d->r_mflag.reserve(n));
-  B2D_CU(d->r_dist.reserve((uint64_t)n * max_count));
-  B2D_CU(d->r_rep.reserve((uint64_t)n * max_count));
-  B2D_CU(d->r_flag.reserve((uint64_t)n * max_count));
-  B2D_CU(d->r_offs.reserve(std::max<uint64_t>(max_lists, 1)));
-  B2D_CU(d->r_partial.reserve(2 * SCAN_GRID * max_count));
-  B2D_CU(d->r_cum.reserve(max_cum));
-  B2D_CU(d->r_total.reserve(2 * max_count));
-  B2D_CU(d->r_straddle.reserve(max_count));
+  B2D_CU(re);
   B2D_CU(d->state.reserve(1));
   B2D_CU(d->state_h.reserve(1));
   B2D_CU(cudaMemsetAsync(d->state.p, 0, sizeof(DevState), d->stream));
@@ -1827,7 +1838,10 @@ int b2d_create(uint32_t chunk_size, int hash_kind, b2d_dedup** out) {
     d->kind = hash_kind;
     cudaError_t e = cudaGetDevice(&d->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&d->sm_count, cudaDevAttrMultiProcessorCount, d->device);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&d->own_stream, cudaStreamNonBlocking);
+    // a blocking stream: the handle's work follows the legacy default stream's.  A cudaMemcpy from
+    // pageable memory may return while its last piece is still on its way to the device, and a
+    // checkpoint's hashing starts within microseconds of the call.
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&d->own_stream, cudaStreamDefault);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&d->cap_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
       delete d;
@@ -2196,7 +2210,7 @@ int b2d_batch_create(b2d_batch** out) {
     b2d_batch* b = new b2d_batch();
     cudaError_t e = cudaGetDevice(&b->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&b->sm_count, cudaDevAttrMultiProcessorCount, b->device);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->own_stream, cudaStreamDefault);   // as a handle's
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming);
     for (auto& ev : b->ev)
