@@ -375,7 +375,8 @@ __global__ void __launch_bounds__(ANY_WARPS * 32, 2) leaf_any_kernel(LeafArgs a0
     const uint64_t p0 = addr - mis;                                 // the chunk's first aligned piece
     const uint64_t pieces = valid ? (mis + nb + 15u) / 16u : 0ull;
     // segment s of a chunk: its pieces 8 s + 1 .. 8 s + 8 (piece 0 is read directly)
-    const uint64_t segs = (a.cs + 15u) / 16u / 8u + 1u;             // enough for every chunk of the warp
+    const uint64_t most = a.len < a.cs ? a.len : a.cs;              // bytes of the longest chunk there is
+    const uint64_t segs = most / 128u + 1u;                         // whole segments, and one with the end
     Digest old;
     old.w[0] = old.w[1] = old.w[2] = old.w[3] = 0u;
     if (valid) old = prior_digest(a, c);
