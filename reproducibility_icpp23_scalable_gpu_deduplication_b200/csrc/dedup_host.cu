@@ -854,6 +854,16 @@ bool parse_hdr(const uint8_t* b, uint64_t size, HostHdr& h) {
   return h.data_off <= size && h.cs > 0 && h.datalen > 0;
 }
 
+// A diff that kernels may read where it lies: memory that is not the device's, managed or page-locked
+// is refused here, as a copy from the device would refuse it, before a kernel follows the pointer.
+int device_diff(const void* p, uint64_t size) {
+  if (!p || size < 32) return B2D_ERR_FORMAT;
+  cudaPointerAttributes pa;
+  const cudaError_t e = cudaPointerGetAttributes(&pa, p);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e == cudaSuccess && pa.type != cudaMemoryTypeUnregistered ? B2D_OK : B2D_ERR_CUDA;
+}
+
 // Headers of device-resident diffs idx .. idx - count + 1, into hdr[0 .. count): one small kernel and
 // one wait for up to RESTART_HEADERS of them.
 int read_device_headers(b2d_dedup* d, const void* const* ddiffs, const uint64_t* sizes, int idx, int count,
@@ -863,7 +873,8 @@ int read_device_headers(b2d_dedup* d, const void* const* ddiffs, const uint64_t*
     RestartHeaders q{};
     for (; q.count < RESTART_HEADERS && k + (int)q.count < count; q.count++) {
       const int i = idx - k - (int)q.count;
-      if (!ddiffs[i] || sizes[i] < 32) return B2D_ERR_FORMAT;
+      const int drc = device_diff(ddiffs[i], sizes[i]);
+      if (drc) return drc;
       q.diff[q.count] = static_cast<const uint8_t*>(ddiffs[i]);
     }
     B2D_CU(launch_restart_headers(q, d->r_hdr.p, d->stream));

@@ -1,0 +1,70 @@
+"""Restarts from lists of device diffs: what is read of the list, and when.
+
+A restart follows the chain from the selected diff down to its baseline (src/tree_approach.cpp:966-1128)
+and reads the headers of the diffs on it, after the work that made them.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+from reproducibility_icpp23_scalable_gpu_deduplication_b200 import TreeDeduplicator
+from reproducibility_icpp23_scalable_gpu_deduplication_b200._lib import lib
+
+pytestmark = pytest.mark.gpu
+
+CS, N = 128, 4096
+B2D_ERR_CUDA, B2D_ERR_FORMAT = -2, -4
+
+
+def to_dev(a):
+    import torch
+
+    return torch.from_numpy(np.frombuffer(a, np.uint8).copy()).cuda()
+
+
+def states(count):
+    rng = np.random.default_rng(3)
+    out = [rng.integers(0, 256, (N, CS), dtype=np.uint8)]
+    for k in range(1, count):
+        x = out[-1].copy()
+        x[20 * k:20 * k + 30] = rng.integers(0, 256, (30, CS), dtype=np.uint8)
+        out.append(x)
+    return [x.reshape(-1) for x in out]
+
+
+def diffs_of(bufs, baselines=(0,)):
+    g = TreeDeduplicator(CS)
+    out = [g.checkpoint(to_dev(b), k in baselines) for k, b in enumerate(bufs)]
+    g.close()
+    return out
+
+
+def restart(g, out, entries, last):
+    """b2d_restart_device with (address, size) entries, on the handle's stream"""
+    ptrs = (ctypes.c_void_p * len(entries))(*[a for a, _ in entries])
+    sizes = (ctypes.c_uint64 * len(entries))(*[n for _, n in entries])
+    return lib().b2d_restart_device(g._h, ctypes.c_void_p(out.data_ptr()), out.numel(), ptrs, sizes, len(entries), last)
+
+
+def entries_of(tensors):
+    return [(t.data_ptr(), t.numel()) for t in tensors]
+
+
+@pytest.mark.parametrize("at", [3, 1, 0])
+def test_pageable_entry_is_refused(cuda, at):
+    """a diff in memory that is not the device's: an error, and the handle goes on"""
+    import torch
+
+    bufs = states(4)
+    diffs = diffs_of(bufs)
+    dev = [to_dev(d) for d in diffs]
+    host = np.frombuffer(diffs[at], np.uint8).copy()
+    entries = entries_of(dev)
+    entries[at] = (host.ctypes.data, host.size)
+    g = TreeDeduplicator(CS)
+    out = torch.zeros(N * CS, dtype=torch.uint8, device="cuda")
+    assert restart(g, out, entries, 3) == B2D_ERR_CUDA
+    assert restart(g, out, entries_of(dev), 3) == 0
+    assert np.array_equal(out.cpu().numpy(), bufs[3])
+    g.close()
