@@ -831,27 +831,12 @@ int write_restart_log(b2d_dedup* d, uint32_t id, const std::string& logname) {
   return B2D_OK;
 }
 
-struct HostHdr {
-  uint32_t ref_id, chkpt_id;
-  uint64_t datalen;
-  uint32_t cs, F, P, S;
-  uint64_t first_off, count_off, shift_off, data_off;
-};
-
-bool parse_hdr(const uint8_t* b, uint64_t size, HostHdr& h) {
-  if (!b || size < 32) return false;
-  memcpy(&h.ref_id, b, 4);
-  memcpy(&h.chkpt_id, b + 4, 4);
-  memcpy(&h.datalen, b + 8, 8);
-  memcpy(&h.cs, b + 16, 4);
-  memcpy(&h.F, b + 20, 4);
-  memcpy(&h.P, b + 24, 4);
-  memcpy(&h.S, b + 28, 4);
-  h.first_off = 32;
-  h.count_off = h.first_off + 4ull * h.F;
-  h.shift_off = h.count_off + 8ull * h.P;
-  h.data_off = h.shift_off + 8ull * h.S;
-  return h.data_off <= size && h.cs > 0 && h.datalen > 0;
+// header of a diff in host memory
+bool parse_host_header(const uint8_t* b, uint64_t size, DiffHeader& h) {
+  uint32_t w[8];
+  if (!b || size < sizeof(w)) return false;
+  memcpy(w, b, sizeof(w));
+  return parse_header(w, size, h);
 }
 
 // A diff that kernels may read where it lies: memory that is not the device's, managed or page-locked
@@ -864,25 +849,36 @@ int device_diff(const void* p, uint64_t size) {
   return e == cudaSuccess && pa.type != cudaMemoryTypeUnregistered ? B2D_OK : B2D_ERR_CUDA;
 }
 
-// Headers of device-resident diffs idx .. idx - count + 1, into hdr[0 .. count): one small kernel and
-// one wait for up to RESTART_HEADERS of them.
-int read_device_headers(b2d_dedup* d, const void* const* ddiffs, const uint64_t* sizes, int idx, int count,
-                        HostHdr* hdr) {
-  B2D_CU(d->r_hdr.reserve(32 * RESTART_HEADERS));
-  for (int k = 0; k < count;) {
+// The headers of a chain of device-resident diffs, newest first from diff `id`: down while the index is
+// not below the last header's ref_id.  A kernel follows the chain, RESTART_HEADERS entries at most per
+// launch, and reads no diff that is not on it: the list may hold anything there.
+int read_device_chain(b2d_dedup* d, const void* const* ddiffs, const uint64_t* sizes, uint32_t id,
+                      std::vector<DiffHeader>& hdrs) {
+  B2D_CU(d->r_hdr.reserve(sizeof(uint32_t) * RESTART_HEADERS * 8 + sizeof(uint32_t)));
+  uint32_t* raw = reinterpret_cast<uint32_t*>(d->r_hdr.p);
+  // most chains are short: few pointers are looked up for the first launch
+  uint32_t most = 8;
+  for (int idx = (int)id;; most = RESTART_HEADERS) {
     RestartHeaders q{};
-    for (; q.count < RESTART_HEADERS && k + (int)q.count < count; q.count++) {
-      const int i = idx - k - (int)q.count;
-      const int drc = device_diff(ddiffs[i], sizes[i]);
-      if (drc) return drc;
+    q.idx = idx;
+    int rc = B2D_OK;   // of the entry that ends the launch's part of the chain
+    for (; q.count < most && idx - (int)q.count >= 0; q.count++) {
+      const int i = idx - (int)q.count;
+      if ((rc = device_diff(ddiffs[i], sizes[i]))) break;
       q.diff[q.count] = static_cast<const uint8_t*>(ddiffs[i]);
+      q.size[q.count] = sizes[i];
     }
-    B2D_CU(launch_restart_headers(q, d->r_hdr.p, d->stream));
+    if (q.count == 0) return rc ? rc : B2D_ERR_FORMAT;
+    B2D_CU(launch_restart_headers(q, raw, raw + 8 * RESTART_HEADERS, d->stream));
     B2D_CU(cudaStreamSynchronize(d->stream));
-    for (uint32_t j = 0; j < q.count; j++, k++)
-      if (!parse_hdr(d->r_hdr.p + 32 * j, sizes[idx - k], hdr[k])) return B2D_ERR_FORMAT;
+    const uint32_t seen = raw[8 * RESTART_HEADERS];
+    for (uint32_t j = 0; j < seen; j++, idx--) {
+      DiffHeader h;
+      if (!parse_header(raw + 8 * j, sizes[idx], h)) return B2D_ERR_FORMAT;
+      hdrs.push_back(h);
+    }
+    if (idx < 0 || idx < (int)hdrs.back().ref_id) return B2D_OK;
   }
-  return B2D_OK;
 }
 
 // Copies host memory to the device on the handle's stream.  Page-locked memory goes straight;
@@ -957,13 +953,16 @@ int do_restart(b2d_dedup* d, void* d_out, uint64_t len, const uint8_t* const* di
   using clk = std::chrono::high_resolution_clock;
   const auto t0 = clk::now();
   if (!d_out || (!diffs && !ddiffs) || !sizes || id >= count) return B2D_ERR_ARG;
-  HostHdr h;
+  // the chain, newest first: from `id` down while the index is not below the last ref_id
+  std::vector<DiffHeader> hdrs;
   if (ddiffs) {
-    const int hrc = read_device_headers(d, ddiffs, sizes, (int)id, 1, &h);
+    const int hrc = read_device_chain(d, ddiffs, sizes, id, hdrs);
     if (hrc) return hrc;
-  } else if (!parse_hdr(diffs[id], sizes[id], h)) {
-    return B2D_ERR_FORMAT;
+  } else {
+    hdrs.emplace_back();
+    if (!parse_host_header(diffs[id], sizes[id], hdrs[0])) return B2D_ERR_FORMAT;
   }
+  const DiffHeader h = hdrs[0];
   // every diff the checkpoint path writes has ref_id <= chkpt_id == its position in the list;
   // a list that breaks this names no chain to walk, so it is rejected before any device work
   if (h.ref_id > h.chkpt_id || h.chkpt_id != id) return B2D_ERR_FORMAT;
@@ -971,29 +970,12 @@ int do_restart(b2d_dedup* d, void* d_out, uint64_t len, const uint8_t* const* di
   uint64_t nc = (h.datalen + h.cs - 1) / h.cs;
   if (nc > 0x7fffffffull) return B2D_ERR_FORMAT;
   const uint32_t n = (uint32_t)nc, N = 2u * n - 1u;
-  // the chain, newest first: from `id` down while the index is not below the last ref_id
-  std::vector<HostHdr> hdrs{h};   // of diffs id, id - 1, ...
-  {
-    std::vector<HostHdr> ahead;   // device headers read together, of diffs id - hdrs.size() on down
-    size_t used = 0;
-    uint32_t ref = h.ref_id;
-    for (int idx = (int)id - 1; idx >= 0 && idx >= (int)ref; idx--) {
-      HostHdr hh;
-      if (ddiffs) {
-        if (used == ahead.size()) {
-          ahead.resize((size_t)(idx - (int)ref + 1));
-          used = 0;
-          const int hrc = read_device_headers(d, ddiffs, sizes, idx, idx - (int)ref + 1, ahead.data());
-          if (hrc) return hrc;
-        }
-        hh = ahead[used++];
-      } else if (!parse_hdr(diffs[idx], sizes[idx], hh)) {
-        return B2D_ERR_FORMAT;
-      }
-      ref = hh.ref_id;
+  if (!ddiffs)
+    for (int idx = (int)id - 1; idx >= 0 && idx >= (int)hdrs.back().ref_id; idx--) {
+      DiffHeader hh;
+      if (!parse_host_header(diffs[idx], sizes[idx], hh)) return B2D_ERR_FORMAT;
       hdrs.push_back(hh);
     }
-  }
   // Sets of diffs expanded together: the main diff with a window of older ones, then windows.  A
   // window's diffs share a chunk size (the walk copies from all of them); its slots' memory and, for
   // host diffs, their copies are bounded.
@@ -1082,7 +1064,7 @@ int do_restart(b2d_dedup* d, void* d_out, uint64_t len, const uint8_t* const* di
     const auto c0 = clk::now();
     std::vector<Upload> copies;
     for (uint32_t m = 0; m < members; m++) {
-      const HostHdr& hh = hdrs[q.beg + m];
+      const DiffHeader& hh = hdrs[q.beg + m];
       const size_t idx = id - (q.beg + m);
       RestartArgs& a = rs.a[m];
       if (ddiffs) {

@@ -682,12 +682,24 @@ __global__ void __launch_bounds__(256) r_cum_set(const __grid_constant__ Restart
   cum_body(s.a[blockIdx.x]);
 }
 
-__global__ void __launch_bounds__(32) r_headers_kernel(const __grid_constant__ RestartHeaders h, uint8_t* out) {
-  out[32u * blockIdx.x + threadIdx.x] = h.diff[blockIdx.x][threadIdx.x];
+// one warp, one diff after another: a header says whether the next diff is read at all
+__global__ void __launch_bounds__(32) r_headers_kernel(const __grid_constant__ RestartHeaders h, uint32_t* out,
+                                                       uint32_t* seen) {
+  __shared__ uint32_t w[8];
+  uint32_t k = 0;
+  for (bool more = true; more && k < h.count; k++) {
+    reinterpret_cast<uint8_t*>(w)[threadIdx.x] = h.diff[k][threadIdx.x];
+    __syncwarp();
+    DiffHeader d;
+    more = parse_header(w, h.size[k], d) && h.idx - (int)k - 1 >= (int)d.ref_id;
+    if (threadIdx.x < 8u) out[8u * k + threadIdx.x] = w[threadIdx.x];
+    __syncwarp();
+  }
+  if (threadIdx.x == 0) *seen = k;
 }
-cudaError_t launch_restart_headers(const RestartHeaders& h, uint8_t* out, cudaStream_t s) {
+cudaError_t launch_restart_headers(const RestartHeaders& h, uint32_t* out, uint32_t* seen, cudaStream_t s) {
   if (h.count == 0 || h.count > RESTART_HEADERS) return cudaErrorInvalidValue;
-  r_headers_kernel<<<h.count, 32, 0, s>>>(h, out);
+  r_headers_kernel<<<1, 32, 0, s>>>(h, out, seen);
   return cudaGetLastError();
 }
 

@@ -109,13 +109,38 @@ cudaError_t launch_restart_diff(const RestartArgs& a, StraddleInfo* sd, int sm_c
 // caller.  `sd` has one record per diff.
 cudaError_t launch_restart_diffs(const RestartSet& set, StraddleInfo* sd, int sm_count, cudaStream_t s);
 int restart_diffs_launches(uint32_t n, bool list);
-// the first 32 bytes of up to RESTART_HEADERS diffs, written to `out` (pinned host memory)
+// header_t of a diff (include/utils.hpp:29-37) from its eight words, and the offsets that follow from
+// it; false where it does not fit a diff of `size` bytes
+struct DiffHeader {
+  uint32_t ref_id, chkpt_id;
+  uint64_t datalen;
+  uint32_t cs, F, P, S;
+  uint64_t first_off, count_off, shift_off, data_off;
+};
+__host__ __device__ inline bool parse_header(const uint32_t* w, uint64_t size, DiffHeader& h) {
+  h.ref_id = w[0];
+  h.chkpt_id = w[1];
+  h.datalen = (uint64_t)w[2] | ((uint64_t)w[3] << 32);
+  h.cs = w[4];
+  h.F = w[5];
+  h.P = w[6];
+  h.S = w[7];
+  h.first_off = 32;
+  h.count_off = h.first_off + 4ull * h.F;
+  h.shift_off = h.count_off + 8ull * h.P;
+  h.data_off = h.shift_off + 8ull * h.S;
+  return h.data_off <= size && h.cs > 0 && h.datalen > 0;
+}
+// The chain of diffs idx, idx - 1, ... (at most `count`, of 32 bytes and more) as far as their headers
+// carry it: the headers' words to `out`, 8 each, how many to `seen` (pinned host memory).
 constexpr uint32_t RESTART_HEADERS = 64;
 struct RestartHeaders {
   uint32_t count;
+  int idx;
   const uint8_t* diff[RESTART_HEADERS];
+  uint64_t size[RESTART_HEADERS];
 };
-cudaError_t launch_restart_headers(const RestartHeaders& h, uint8_t* out, cudaStream_t s);
+cudaError_t launch_restart_headers(const RestartHeaders& h, uint32_t* out, uint32_t* seen, cudaStream_t s);
 // resolves the chunks owed by the window's diffs and copies them
 cudaError_t launch_restart_walk(const RestartWalk& w, int sm_count, cudaStream_t s);
 // kernel launches made by one launch_restart_diff call (a walk is one launch)

@@ -68,3 +68,41 @@ def test_pageable_entry_is_refused(cuda, at):
     assert restart(g, out, entries_of(dev), 3) == 0
     assert np.array_equal(out.cpu().numpy(), bufs[3])
     g.close()
+
+
+@pytest.mark.parametrize("entry", ["null", "short"])
+def test_entries_off_the_chain_are_not_read(cuda, entry):
+    """a chain that an older diff ends early (a baseline that stands for those before it): what the
+    list holds below it does not matter"""
+    import torch
+
+    bufs = states(4)
+    mixed = diffs_of(bufs)[:2] + [diffs_of(bufs[:3], (0, 2))[2], diffs_of(bufs)[3]]
+    dev = [to_dev(d) for d in mixed]
+    entries = entries_of(dev)
+    for k in (0, 1):
+        entries[k] = (None, 4096) if entry == "null" else (dev[k].data_ptr(), 31)
+    g = TreeDeduplicator(CS)
+    out = torch.zeros(N * CS, dtype=torch.uint8, device="cuda")
+    assert restart(g, out, entries, 3) == 0
+    assert np.array_equal(out.cpu().numpy(), bufs[3])
+    # on the chain they do
+    entries = entries_of([to_dev(d) for d in diffs_of(bufs)])
+    entries[1] = (None, 4096) if entry == "null" else (dev[1].data_ptr(), 31)
+    assert restart(g, out, entries, 3) == B2D_ERR_FORMAT
+    g.close()
+
+
+@pytest.mark.parametrize("count", [8, 9, 64, 65, 73, 140])
+def test_long_chains(cuda, count):
+    """chains of one and of several header reads"""
+    import torch
+
+    bufs = states(count)
+    dev = [to_dev(d) for d in diffs_of(bufs)]
+    g = TreeDeduplicator(CS)
+    for last in (count - 1, count - 2):
+        out = torch.zeros(N * CS, dtype=torch.uint8, device="cuda")
+        assert restart(g, out, entries_of(dev), last) == 0
+        assert np.array_equal(out.cpu().numpy(), bufs[last]), last
+    g.close()
