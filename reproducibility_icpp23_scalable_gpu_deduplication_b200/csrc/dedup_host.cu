@@ -224,6 +224,7 @@ struct b2d_dedup {
   DevBuf<uint8_t> r_diff;
   DevBuf<StraddleInfo> r_straddle;
   PinnedBuf<uint8_t> r_hdr;                // headers of device diffs
+  cudaEvent_t order_ev = nullptr;          // the legacy default stream's work before a restart
   PinnedBuf<uint8_t> r_stage;              // upload()'s ring, and when each piece's copy is done
   cudaEvent_t stage_ev[STAGE_PIECES] = {};
 
@@ -277,6 +278,7 @@ b2d_dedup::~b2d_dedup() {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     for (auto& e : stage_ev)
       if (e) cudaEventDestroy(e);
+    if (order_ev) cudaEventDestroy(order_ev);
     if (own_stream) cudaStreamDestroy(own_stream);
     if (cap_stream) cudaStreamDestroy(cap_stream);
   }
@@ -849,6 +851,16 @@ int device_diff(const void* p, uint64_t size) {
   return e == cudaSuccess && pa.type != cudaMemoryTypeUnregistered ? B2D_OK : B2D_ERR_CUDA;
 }
 
+// The handle's stream goes on after what the legacy default stream, and the blocking streams it waits
+// for, hold now.
+int follow_default_stream(b2d_dedup* d) {
+  if (d->stream == cudaStreamLegacy) return B2D_OK;
+  if (!d->order_ev) B2D_CU(cudaEventCreateWithFlags(&d->order_ev, cudaEventDisableTiming));
+  B2D_CU(cudaEventRecord(d->order_ev, cudaStreamLegacy));
+  B2D_CU(cudaStreamWaitEvent(d->stream, d->order_ev, 0));
+  return B2D_OK;
+}
+
 // The headers of a chain of device-resident diffs, newest first from diff `id`: down while the index is
 // not below the last header's ref_id.  A kernel follows the chain, RESTART_HEADERS entries at most per
 // launch, and reads no diff that is not on it: the list may hold anything there.
@@ -956,7 +968,10 @@ int do_restart(b2d_dedup* d, void* d_out, uint64_t len, const uint8_t* const* di
   // the chain, newest first: from `id` down while the index is not below the last ref_id
   std::vector<DiffHeader> hdrs;
   if (ddiffs) {
-    const int hrc = read_device_chain(d, ddiffs, sizes, id, hdrs);
+    // diffs put in place on the default stream are there, whatever stream the handle was given: a
+    // copy from pageable memory may still be on its way when its call returns
+    int hrc = follow_default_stream(d);
+    if (hrc == B2D_OK) hrc = read_device_chain(d, ddiffs, sizes, id, hdrs);
     if (hrc) return hrc;
   } else {
     hdrs.emplace_back();

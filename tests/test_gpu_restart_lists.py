@@ -106,3 +106,25 @@ def test_long_chains(cuda, count):
         assert restart(g, out, entries_of(dev), last) == 0
         assert np.array_equal(out.cpu().numpy(), bufs[last]), last
     g.close()
+
+
+@pytest.mark.parametrize("stream", ["other", "own"])
+def test_follows_the_default_stream(cuda, stream):
+    """diffs that the default stream is still copying when the restart is called"""
+    import torch
+
+    bufs = states(4)
+    src = [to_dev(d) for d in diffs_of(bufs)]
+    g = TreeDeduplicator(CS)
+    other = torch.cuda.Stream()
+    assert lib().b2d_set_stream(g._h, ctypes.c_void_p(other.cuda_stream if stream == "other" else None)) == 0
+    for _ in range(3):
+        dst = [torch.zeros_like(x) for x in src]
+        out = torch.zeros(N * CS, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        torch.cuda._sleep(20_000_000)   # about 10 ms before the copies start
+        for x, y in zip(dst, src):
+            x.copy_(y)
+        assert restart(g, out, entries_of(dst), 3) == 0
+        assert np.array_equal(out.cpu().numpy(), bufs[3])
+    g.close()
