@@ -931,8 +931,7 @@ int upload(b2d_dedup* d, const std::vector<Upload>& copies) {
   uint32_t T = 1;
   while (2 * T <= std::min<uint64_t>(most, pieces.size())) T *= 2;
   std::atomic<int> err{0};
-  auto work = [&](uint32_t t) {
-    cudaError_t e = cudaSetDevice(d->device);
+  auto work = [&](uint32_t t, cudaError_t e) {
     for (size_t p = t; p < pieces.size() && e == cudaSuccess && err.load() == 0; p += T) {
       const uint32_t slot = (uint32_t)(p % STAGE_PIECES);
       uint8_t* s = d->r_stage.p + STAGE_PIECE * slot;
@@ -948,11 +947,13 @@ int upload(b2d_dedup* d, const std::vector<Upload>& copies) {
   uint32_t started = 1;
   try {
     threads.reserve(T);
-    for (; started < T; started++) threads.emplace_back(work, started);
+    // the caller's own thread keeps the device it has
+    for (; started < T; started++)
+      threads.emplace_back([&work, d, t = started] { work(t, cudaSetDevice(d->device)); });
   } catch (...) {   // no more threads: their pieces are filled here
   }
-  work(0);
-  for (uint32_t t = started; t < T; t++) work(t);
+  work(0, cudaSuccess);
+  for (uint32_t t = started; t < T; t++) work(t, cudaSuccess);
   for (auto& t : threads) t.join();
   return err.load();
 }
