@@ -91,6 +91,9 @@ int b2d_set_stream(b2d_dedup* d, void* cuda_stream);
  *   "warp_bands"        forest phases whose lowest levels run as warp tasks (7 levels per task
  *                       in phase 1, 9 in phase 2) instead of CTA bands (10 and 12 levels): bit 0
  *                       phase 1, bit 1 phase 2, 0..3 (default 3)
+ *   "restart_window"    older diffs that a restart resolves together, at most, 1..8 (0 = as many as
+ *                       its memory bounds allow, the default); 1 = one diff at a time, with the
+ *                       least memory.  A restart that runs out of device memory sets it to 1
  *   "graph"             0 = launch a checkpoint's kernels one by one on the handle's stream
  *                       (default; measured faster), 1 = replay them as one CUDA graph, 2 = graph
  *                       that reports no phase times (b2d_phase_times then reads 0) */

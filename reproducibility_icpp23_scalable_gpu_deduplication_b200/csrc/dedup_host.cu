@@ -216,6 +216,7 @@ struct b2d_dedup {
   bool diff_valid = false;
 
   // restart scratch
+  int restart_window = 0;                  // most older diffs resolved together (0: as many as fit)
   DevBuf<uint2> r_node_list, r_rep;      // restart: NodeIDs of the main diff's chunks; slots' rep
   DevBuf<uint32_t> r_dist;                 // slots' data offsets
   DevBuf<uint8_t> r_mflag, r_flag;
@@ -994,16 +995,21 @@ int do_restart(b2d_dedup* d, void* d_out, uint64_t len, const uint8_t* const* di
     }
   // Sets of diffs expanded together: the main diff with a window of older ones, then windows.  A
   // window's diffs share a chunk size (the walk copies from all of them); its slots' memory and, for
-  // host diffs, their copies are bounded.
+  // host diffs, their copies are bounded.  Windows of host diffs are kept small: the copies take far
+  // longer than a walk, and the handle keeps the memory.
   const uint64_t per_slot = 13ull * n;   // dist u32 + rep uint2 + a flag byte per chunk
-  const uint64_t window = std::min<uint64_t>(RESTART_WINDOW, std::max<uint64_t>(1, RESTART_SLOT_BYTES / per_slot));
+  const uint64_t slot_bytes = ddiffs ? RESTART_SLOT_BYTES : RESTART_HOST_BYTES;
+  const uint64_t window = std::min<uint64_t>(RESTART_WINDOW, std::max<uint64_t>(1, slot_bytes / per_slot));
   struct Set {
     size_t beg, end;   // of hdrs
   };
   std::vector<Set> sets;
   uint64_t max_bytes = 0, max_lists = 0, max_cum = 0, max_count = 0;
   auto room = [&](size_t k) { return (sizes[id - k] + 31u) / 16u * 16u; };   // a diff's device copy
-  auto plan = [&](uint64_t win, uint64_t byte_limit) {
+  auto plan = [&]() {
+    const uint64_t win = d->restart_window ? std::min<uint64_t>(window, d->restart_window) : window;
+    // a window of one: one diff at a time, the main diff by itself too
+    const uint64_t byte_limit = d->restart_window == 1 ? 0 : ddiffs ? ~0ull : RESTART_HOST_BYTES;
     sets.clear();
     max_bytes = max_lists = max_cum = max_count = 0;
     for (size_t k = 0; k < hdrs.size();) {
@@ -1041,16 +1047,18 @@ int do_restart(b2d_dedup* d, void* d_out, uint64_t len, const uint8_t* const* di
     if (e == cudaSuccess) e = d->r_straddle.reserve(max_count);
     return e;
   };
-  plan(window, ddiffs ? ~0ull : RESTART_SLOT_BYTES);
+  plan();
   cudaError_t re = reserve();
-  if (re == cudaErrorMemoryAllocation) {   // too little device memory for a window: one diff at a time
+  if (re == cudaErrorMemoryAllocation && d->restart_window != 1) {
+    // too little device memory for a window: one diff at a time, from now on
     (void)cudaGetLastError();
+    d->restart_window = 1;
     d->r_diff.release();
     d->r_dist.release();
     d->r_rep.release();
     d->r_flag.release();
     d->r_offs.release();
-    plan(1, 0);
+    plan();
     re = reserve();
   }
   B2D_CU(re);
@@ -2061,6 +2069,7 @@ int b2d_set_param(b2d_dedup* d, const char* name, int64_t value) {
   else if (k == "map_max_load_pct" && value >= 10 && value <= 90) d->map_max_load = value / 100.0;
   else if (k == "map_headroom_pct" && value >= 100 && value <= 1000) d->map_headroom = value / 100.0;
   else if (k == "warp_bands" && value >= 0 && value <= 3) d->warp_bands = (int)value;
+  else if (k == "restart_window" && value >= 0 && value <= (int64_t)RESTART_WINDOW) d->restart_window = (int)value;
   else if (k == "graph" && value >= 0 && value <= 2) {
     d->use_graph = value != 0;
     d->graph_timing = value != 2;

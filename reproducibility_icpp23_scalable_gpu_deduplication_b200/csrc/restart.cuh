@@ -58,6 +58,7 @@ struct RestartArgs {
 // Older diffs resolved by one walk over the chunks, newest first.
 constexpr uint32_t RESTART_WINDOW = 8;
 constexpr uint64_t RESTART_SLOT_BYTES = 8ull << 30;   // memory for the window slots of one restart
+constexpr uint64_t RESTART_HOST_BYTES = 256ull << 20; // the same, and for the copies, of host diffs
 struct RestartWalk {
   uint32_t count;          // diffs in this window
   int dense;               // node_list holds every chunk's NodeID (an earlier window wrote it)
