@@ -238,9 +238,15 @@ constexpr uint32_t FF_WORDS = 32;          // 1023 bits: band heights 1..10
 __device__ __forceinline__ uint32_t ff_base(uint32_t k) {   // first bit of band height k
   return 1024u - (2048u >> k);
 }
-__device__ __forceinline__ void ff_set(uint32_t* ff, uint32_t k, uint32_t i) {
+// a first-occurrence parent's home slot, on its way to L2 before the parent is inserted
+__device__ __forceinline__ void prefetch_home(const MapView& m, const Digest& d) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(map_key(m, map_home(digest_key(d), m.cap))));
+}
+// records parent i of band height k, whose digest is d, for the inserts at the band's end
+__device__ __forceinline__ void ff_add(const ForestArgs& a, uint32_t* ff, uint32_t k, uint32_t i, const Digest& d) {
   const uint32_t bit = ff_base(k) + i;
   atomicOr(&ff[bit >> 5], 1u << (bit & 31u));
+  prefetch_home(a.map, d);
 }
 __device__ __forceinline__ Digest shfl_down_digest(const Digest& d, uint32_t delta) {
   Digest r;
@@ -302,7 +308,7 @@ __device__ __forceinline__ void forest_first_body(const ForestArgs& a, uint32_t 
       d1[j] = hash_pair(a.kind, a.tree[x0 + 2 * j], a.tree[x0 + 2 * j + 1]);
       a.tree[p] = d1[j];
       m1 |= 1u << j;
-      ff_set(ff, 1, 2u * t + j);
+      ff_add(a, ff, 1, 2u * t + j, d1[j]);
     }
   }
   // band height 2: node (root << 8) + 255 + t
@@ -314,7 +320,7 @@ __device__ __forceinline__ void forest_first_body(const ForestArgs& a, uint32_t 
     dg = hash_pair(a.kind, d1[0], d1[1]);
     a.tree[y] = dg;
     b = 1;
-    ff_set(ff, 2, t);
+    ff_add(a, ff, 2, t, dg);
   }
   // band heights 3..7: warp shuffles
   if (__any_sync(0xffffffffu, b)) {
@@ -328,7 +334,7 @@ __device__ __forceinline__ void forest_first_body(const ForestArgs& a, uint32_t 
         if (b) {
           dg = hash_pair(a.kind, dg, rd);
           a.tree[y] = dg;
-          ff_set(ff, 3 + s, t >> (s + 1));
+          ff_add(a, ff, 3 + s, t >> (s + 1), dg);
         }
       }
     }
@@ -355,7 +361,7 @@ __device__ __forceinline__ void forest_first_body(const ForestArgs& a, uint32_t 
         if (b) {
           dg = hash_pair(a.kind, dg, rd);
           a.tree[y] = dg;
-          ff_set(ff, 8 + s, lane >> (s + 1));
+          ff_add(a, ff, 8 + s, lane >> (s + 1), dg);
         }
       }
     }
@@ -583,10 +589,13 @@ __device__ __forceinline__ uint4 slot_labels16(const ForestArgs& a, const LeafSl
 // done (spread over the lanes): inserting each where it is hashed put a chain of dependent map
 // round trips on the lanes that carry the upper levels.  At most 127 per task of 128 leaves.  Each
 // parent's home slot is prefetched into L2 as it is recorded, so its insert waits for L2 and not
-// for memory, and one insert per lane at a time is enough: two in flight together, without the
-// prefetch, were slower (phase times of increments: 400 MB at 10 % 115 and 96 us, 1 GiB MD5 floats
-// 233 and 199 us), as was a CAS at every probe instead of a read first (MD5 floats 308 us: the
-// zero pages' parents share slots).
+// for memory, and one insert per lane at a time is enough.  Two in flight together, without and with
+// the prefetch, against one with it: increment's forest 104 and 98 against 91 us (400 MB at 10 %), 212
+// and 214 against 197 us (1 GiB MD5 floats), 173 and 176 against 161 us (4 GiB); a batch's increment
+// (256 buffers, 13 GB) 8.00 and 7.99 against 7.75 ms.  One without the prefetch is as fast there; in
+// the CTA bands, which insert their parents after the band too, it took 109 against 100 us (400 MB).
+// A CAS at every probe instead of a read first took 308 us (MD5 floats: the zero pages' parents share
+// slots).
 struct WarpInserts {
   uint32_t* node;   // 128 entries of this warp's buffer in shared memory
   Digest* dig;
@@ -597,7 +606,7 @@ __device__ __forceinline__ void wi_add(const WarpInserts& wi, uint32_t x, const 
   const uint32_t pos = atomicAdd(wi.count, 1u);
   wi.node[pos] = x;
   wi.dig[pos] = d;
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(map_key(wi.map, map_home(digest_key(d), wi.map.cap))));
+  prefetch_home(wi.map, d);
 }
 __device__ __forceinline__ void wi_flush(const ForestArgs& a, const WarpInserts& wi, uint32_t lane) {
   __syncwarp();
