@@ -717,8 +717,10 @@ DiffGrids diff_grids(const DiffArgs& a, uint32_t bcap, int sm_count) {
   // longer ranges (<= 296) keep it short; the scatter walks each range with one warp
   r.gs = grid_for(a.n, 8192, SHIFT_GRID);
   r.gc = r.gs + grid_for(a.n, 4096, (uint32_t)sm_count * 8u);
-  // two waves of resident CTAs for the gather, four from 2 GiB on: with four, an increment's emit
-  // pass took 37 against 29 us (64 MiB); with two, the 4 GiB baseline's 1.54 against 1.45 ms
+  // two waves of resident CTAs for the gather, four from 2 GiB on, where the one run of a baseline gains
+  // what increments lose.  Diff assembly with two and four, baselines and increments (5 % in runs of
+  // 32 chunks of 128 B), us: 32 MiB 31 and 36, 22 and 29; 128 MiB 63 and 67, 25 and 32; 512 MiB 195 and
+  // 189, 35 and 44; 2 GiB 734 and 697, 87 and 96; 4 GiB baseline 1540 and 1450
   const uint64_t bytes = (uint64_t)a.n * a.cs;
   r.ge = shift_ctas(r.gs, bcap) + grid_for(bytes, 32768, (uint32_t)sm_count * (bytes >> 31 ? 8u : 4u));
   // 16-byte aligned source units; both kinds write a 16-byte aligned data section
