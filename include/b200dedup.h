@@ -17,8 +17,12 @@
  * only permute them).
  *
  * Threading: one handle per host thread; a handle is not thread-safe.  All device work of a
- * handle runs on one CUDA stream (its own, or the one given to b2d_set_stream).  Device
- * pointers passed in must belong to the current device.
+ * handle runs on one CUDA stream (its own, or the one given to b2d_set_stream).  A handle's and a
+ * batch's own stream is a blocking one: its work follows what the legacy default stream holds when
+ * a call is made, and the default stream's later work follows it, so the two do not overlap.  A
+ * caller that wants them to gives a non-blocking stream, and then has its buffers in place before
+ * it calls (a cudaMemcpy from pageable memory may return while its last piece is on its way).
+ * Device pointers passed in must belong to the current device.
  */
 #ifndef B200DEDUP_H
 #define B200DEDUP_H
@@ -95,8 +99,9 @@ int b2d_set_stream(b2d_dedup* d, void* cuda_stream);
  *                       its memory bounds allow, the default); 1 = one diff at a time, with the
  *                       least memory.  A restart that runs out of device memory sets it to 1
  *   "graph"             0 = launch a checkpoint's kernels one by one on the handle's stream
- *                       (default; measured faster), 1 = replay them as one CUDA graph, 2 = graph
- *                       that reports no phase times (b2d_phase_times then reads 0) */
+ *                       (default), 1 = replay them as one CUDA graph, 2 = graph that reports no
+ *                       phase times (b2d_phase_times then reads 0).  A graph costs the host less
+ *                       per increment; baselines of large buffers are faster without it */
 int b2d_set_param(b2d_dedup* d, const char* name, int64_t value);
 
 /* checkpoint(header_t&, uint8_t* data_ptr, size_t len, HostMirror& diff_h, bool make_baseline)
@@ -204,7 +209,7 @@ int b2d_restart_timers(b2d_dedup* d, double out[2]);
 int b2d_datasizes(b2d_dedup* d, uint64_t out[2]);
 /* Device time (seconds, read from the global timer by its kernels) of the last checkpoint's three
  * stages: chunk hashing + labelling, Merkle forest, diff assembly.  *leaf_path (nullable) is 1
- * when the TMA-staged hashing kernel ran, 0 for the byte-granular one.  No reference
+ * when the TMA-staged hashing kernel ran, 0 for the one that takes any size and alignment.  No reference
  * counterpart (the reference times whole phases on the host, src/tree_approach.cpp:1640-1688). */
 int b2d_phase_times(b2d_dedup* d, double out[3], int* leaf_path);
 /* device kernels launched by the last checkpoint/restart call on this handle */

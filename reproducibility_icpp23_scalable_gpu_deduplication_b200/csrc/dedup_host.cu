@@ -176,8 +176,10 @@ struct b2d_dedup {
   bool have_tree = false;
   LeafTuning tune;
   double map_max_load = 0.75;
-  // replay each checkpoint's launches as one CUDA graph (off by default: on the 4 GiB series
-  // the graph launch measured 0.15-0.2 ms slower per checkpoint than the 22 stream launches)
+  // Replay each checkpoint's launches as one CUDA graph.  Off by default: one graph serves baselines
+  // and increments, so a graph handle's baselines are not built in bulk (4 GiB 11.6 against 6.4 ms).
+  // An increment's launches cost the host less as one graph: an unchanged 1 MiB 40 against 56 us, 64 MiB
+  // 59 and 67, 1 GiB 252 and 258, 4 GiB 836 and 839.
   bool use_graph = false;
   bool graph_timing = true;       // phase times are reported for graph replays
   double map_headroom = MAP_HEADROOM;   // baseline table size over its minimum (entries + N at max load)
@@ -192,7 +194,7 @@ struct b2d_dedup {
 
   DevBuf<Digest> tree;
   DevBuf<uint8_t> lab, leaflab, push, dupflag;
-  void* map_mem = nullptr;        // map_cap + 1 keys, then their values (map_at), from the library's map pool
+  void* map_mem = nullptr;        // map_cap + 1 slots (map_at), from the library's map pool
   uint64_t map_cap = 0;
   double map_grow_s = 0;          // host seconds spent growing the map (all checkpoints)
   double map_alloc_s = 0;         // host seconds in the map allocation calls (all tables)

@@ -1,6 +1,7 @@
-// Block-level scan helpers for the reduce-then-scan passes (no cross-CTA waiting: every
-// multi-CTA scan here is three launches -- per-CTA reduce, one-CTA scan of the partials,
-// per-CTA rescan + scatter -- so no kernel ever spins on another CTA).
+// Block-level scan helpers for the reduce-then-scan passes.  No kernel ever spins on another CTA: a
+// scan over several CTAs is a launch that counts per CTA and one that rescans from the counts before
+// its own, which it adds up itself (gather.cu) or finds scanned by a launch of one CTA in between
+// (restart.cu, bulk.cu), or by the last CTA of the counting launch to finish (gather.cu's layout).
 #pragma once
 #include "common.cuh"
 
