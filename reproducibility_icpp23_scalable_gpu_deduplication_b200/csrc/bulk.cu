@@ -479,7 +479,6 @@ __global__ void __launch_bounds__(256) overflow_kernel(BulkArgs a) {
 
 // ------------------------------------------------------------------ host side
 bool bulk_plan(uint32_t n, uint64_t cap, int list, uint64_t diff_bytes, BulkPlan& p) {
-  if (B2D_MAP_SPLIT) return false;   // build writes interleaved slots
   p.count = list ? n : 2ull * n - 1ull;
   const uint64_t ranges = (cap + BULK_RANGE - 1u) / BULK_RANGE;
   if (n < (list ? BULK_MIN_LIST : BULK_MIN_TREE) || ranges > BULK_MAX_RANGES) return false;

@@ -8,8 +8,7 @@
 //   push   : 2 bits per node region-root flags set by each node's parent: 1 first-occurrence
 //                            root, 2 shifted-duplicate root (16 nodes per 32-bit word; node x at
 //                            position x + 1, so every level starts on its own power of two)
-//   map    : cap+1 keys (16 B) then cap+1 values (8 B): open-addressing digest -> NodeID
-//            table, 24 B per slot (map.cuh)
+//   map    : open-addressing digest -> NodeID table of cap + 1 slots, 32 B each (map.cuh)
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -68,11 +67,6 @@ __host__ __device__ __forceinline__ void leaf_range(uint32_t node, uint32_t num_
   if (r > num_nodes) r = num_nodes - 1u;
   lo = l;
   hi = r;
-}
-__host__ __device__ __forceinline__ uint32_t num_leaf_descendents(uint32_t node, uint32_t num_nodes) {
-  uint32_t lo, hi;
-  leaf_range(node, num_nodes, lo, hi);
-  return hi - lo + 1u;
 }
 __host__ __device__ __forceinline__ uint32_t leftmost_leaf(uint32_t node, uint32_t num_nodes) {
   uint32_t lo, hi;

@@ -421,8 +421,7 @@ __global__ void __launch_bounds__(FAST_THREADS, B2D_FF_MINB) forest_first_seg(Fo
   forest_first_body(with_round(s.args[h]), bid, s.p0[h]);
 }
 
-// Fast band: inputs at level `in`, outputs at level in - 12.
-template <int PHASE>
+// Fast band of phase 2: inputs at level `in`, outputs at level in - 12.
 __device__ __forceinline__ void forest_fast_body(const ForestArgs& a, uint32_t bid, uint32_t in) {
   __shared__ uint8_t wlab[FAST_THREADS / 32];
   const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
@@ -432,38 +431,28 @@ __device__ __forceinline__ void forest_fast_body(const ForestArgs& a, uint32_t b
   bool fast = !a.baseline;
   if (in == a.D && (a.n & (a.n - 1u)) == 0) {
     // power-of-two leaf count, leaf band: the 16 inputs are chunks 16t.. of this CTA's 4096,
-    // one aligned 16-byte load; FIXED = 0x01 bytes, FIRST = 0x00 bytes
+    // one aligned 16-byte load; FIXED = 0x01 bytes
     const uint4 w = *reinterpret_cast<const uint4*>(a.leaflab + (x0 - (a.n - 1u)));
-    if (PHASE == 2) {
-      fast = fast && w.x == 0x01010101u && w.y == 0x01010101u && w.z == 0x01010101u && w.w == 0x01010101u;
-    } else {
-      const uint32_t zx = (w.x - 0x01010101u) & ~w.x, zy = (w.y - 0x01010101u) & ~w.y;
-      const uint32_t zz = (w.z - 0x01010101u) & ~w.z, zw = (w.w - 0x01010101u) & ~w.w;
-      fast = fast && (((zx | zy | zz | zw) & 0x80808080u) == 0);   // no zero byte at all: no FIRST
-    }
+    fast = fast && w.x == 0x01010101u && w.y == 0x01010101u && w.z == 0x01010101u && w.w == 0x01010101u;
     if (!fast) {
       const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-      for (int j = 0; j < 16; j++) v[j] = leaf_view<PHASE>(a, (uint32_t)(x0 + j), (uint8_t)(ws[j >> 2] >> (8 * (j & 3))));
+      for (int j = 0; j < 16; j++) v[j] = leaf_view<2>(a, (uint32_t)(x0 + j), (uint8_t)(ws[j >> 2] >> (8 * (j & 3))));
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 16; j++) v[j] = input_label<PHASE>(a, x0 + j);
+    for (int j = 0; j < 16; j++) v[j] = input_label<2>(a, x0 + j);
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
-      if (PHASE == 2) fast = fast && v[j] == FIXED_DUPL;
-      else fast = fast && v[j] != FIRST_OCUR && v[j] != NONE_LABEL;
-    }
+    for (int j = 0; j < 16; j++) fast = fast && v[j] == FIXED_DUPL;
   }
-  // every input of the band unchanged (phase 2: all FIXED; phase 1: no first occurrence): the
-  // whole subtree folds to one label without further work
+  // every input of the band unchanged: the whole subtree folds to one label without further work
   if (!__syncthreads_or(!fast)) {
-    if (t == 0) band_output<PHASE>(a, root, PHASE == 2 ? FIXED_DUPL : DONE);
+    if (t == 0) band_output<2>(a, root, FIXED_DUPL);
     return;
   }
   uint8_t lab;
   if (fast) {
-    lab = PHASE == 2 ? FIXED_DUPL : DONE;
+    lab = FIXED_DUPL;
   } else {
     uint64_t first = x0;
 #pragma unroll
@@ -472,8 +461,8 @@ __device__ __forceinline__ void forest_fast_body(const ForestArgs& a, uint32_t b
 #pragma unroll
       for (int j = 0; j < width; j++) {
         // two FIXED children: an inner node, FIXED in an incremental checkpoint
-        if (PHASE == 2 && !a.baseline && v[2 * j] == FIXED_DUPL && v[2 * j + 1] == FIXED_DUPL) v[j] = FIXED_DUPL;
-        else v[j] = combine<PHASE>(a, first + j, v[2 * j], v[2 * j + 1]);
+        if (!a.baseline && v[2 * j] == FIXED_DUPL && v[2 * j + 1] == FIXED_DUPL) v[j] = FIXED_DUPL;
+        else v[j] = combine<2>(a, first + j, v[2 * j], v[2 * j + 1]);
       }
     }
     lab = v[0];
@@ -486,11 +475,7 @@ __device__ __forceinline__ void forest_fast_body(const ForestArgs& a, uint32_t b
     const uint8_t rl = (uint8_t)__shfl_down_sync(0xffffffffu, (uint32_t)lab, 1u << s);
     if ((lane & ((2u << s) - 1u)) == 0) {
       y = (y - 1ull) >> 1;
-      if (!(PHASE == 2 && !a.baseline && lab == FIXED_DUPL && rl == FIXED_DUPL) &&
-          !(PHASE == 1 && !a.baseline && lab != FIRST_OCUR && lab != NONE_LABEL && rl != NONE_LABEL))
-        lab = combine<PHASE>(a, y, lab, rl);
-      else if (PHASE == 1)
-        lab = DONE;
+      if (a.baseline || lab != FIXED_DUPL || rl != FIXED_DUPL) lab = combine<2>(a, y, lab, rl);
     }
   }
   if (lane == 0) wlab[warp] = lab;
@@ -504,27 +489,25 @@ __device__ __forceinline__ void forest_fast_body(const ForestArgs& a, uint32_t b
       const uint8_t rl = (uint8_t)__shfl_down_sync(0xffffffffu, (uint32_t)lab, 1u << s);
       if ((lane & ((2u << s) - 1u)) == 0 && lane < FAST_THREADS / 32) {
         y = (y - 1ull) >> 1;
-        lab = combine<PHASE>(a, y, lab, rl);
+        lab = combine<2>(a, y, lab, rl);
       }
     }
-    if (lane == 0) band_output<PHASE>(a, root, lab);
+    if (lane == 0) band_output<2>(a, root, lab);
   }
 }
-template <int PHASE>
 __global__ void __launch_bounds__(FAST_THREADS, B2D_FAST_MINB) forest_fast_kernel(const __grid_constant__ ForestArgs a0, uint32_t in,
                                                                                   uint32_t nbands) {
   griddep_enter();
   const ForestArgs a = with_round(a0);
   for (uint32_t bid = blockIdx.x; bid < nbands; bid += gridDim.x) {
-    forest_fast_body<PHASE>(a, bid, in);
+    forest_fast_body(a, bid, in);
     __syncthreads();
   }
 }
-template <int PHASE>
 __global__ void __launch_bounds__(FAST_THREADS, B2D_FAST_MINB) forest_fast_seg(ForestSeg s) {
   uint32_t bid, nb;
   const uint32_t h = seg_find(s.beg, s.n, bid, nb);
-  forest_fast_body<PHASE>(with_round(s.args[h]), bid, s.p0[h]);
+  forest_fast_body(with_round(s.args[h]), bid, s.p0[h]);
 }
 
 // Warp bands: the first band of each phase, as
@@ -1111,7 +1094,7 @@ static uint32_t resident_ctas(K kernel) {
 
 cudaError_t launch_forest(const ForestArgs& args, int phase, cudaStream_t stream, int sm_count, int warp_mask) {
   static const uint32_t res_first = resident_ctas(forest_first_kernel);
-  static const uint32_t res_fast = resident_ctas(forest_fast_kernel<2>);
+  static const uint32_t res_fast = resident_ctas(forest_fast_kernel);
   std::vector<ForestStep> steps;
   ForestArgs a = args;
   if (warp_bands(a.n, a.D, phase, warp_mask)) {
@@ -1139,7 +1122,7 @@ cudaError_t launch_forest(const ForestArgs& args, int phase, cudaStream_t stream
       const uint32_t cap = (phase == 1 ? res_first : res_fast) * (uint32_t)(sm_count > 0 ? sm_count : 0);
       if (B2D_FOREST_PERSIST && cap && grid > cap) grid = cap;
       e = phase == 1 ? launch_dependent(forest_first_kernel, grid, FAST_THREADS, 0, stream, a, st.p0, st.ctas)
-                     : launch_dependent(forest_fast_kernel<2>, grid, FAST_THREADS, 0, stream, a, st.p0, st.ctas);
+                     : launch_dependent(forest_fast_kernel, grid, FAST_THREADS, 0, stream, a, st.p0, st.ctas);
     } else {
       e = phase == 1 ? launch_dependent(forest_band_kernel<1>, st.ctas, FOREST_THREADS, 0, stream, a, st.p0, st.p1)
                      : launch_dependent(forest_band_kernel<2>, st.ctas, FOREST_THREADS, 0, stream, a, st.p0, st.p1);
@@ -1167,7 +1150,7 @@ cudaError_t launch_forest_seg(const ForestSeg& s, int phase, int kind, uint32_t 
     else forest_warp2_seg<<<ctas, WB_THREADS, 0, stream>>>(s);
   } else if (kind == 0) {
     if (phase == 1) forest_first_seg<<<ctas, FAST_THREADS, 0, stream>>>(s);
-    else forest_fast_seg<2><<<ctas, FAST_THREADS, 0, stream>>>(s);
+    else forest_fast_seg<<<ctas, FAST_THREADS, 0, stream>>>(s);
   } else {
     if (phase == 1) forest_band_seg<1><<<ctas, FOREST_THREADS, 0, stream>>>(s);
     else forest_band_seg<2><<<ctas, FOREST_THREADS, 0, stream>>>(s);

@@ -5,12 +5,8 @@
 //   insert(key, value): insert-if-absent; reports inserted vs existing plus the slot;
 //   the slot's value stays mutable for the lowest-index update (tree_approach.cpp:85,339).
 //
-// Table layout (cap + 1 slots in one allocation), one of two, chosen at build time:
-//   B2D_MAP_SPLIT 0 (default): a 32-byte slot per entry, the 128-bit key then its u64 value, so
-//     an insert's value update lands in the sector its key claim already brought in;
-//   B2D_MAP_SPLIT 1: all keys, then all values (24 bytes per slot): a probe reads only keys,
-//     eight to a line, but every value update is a second DRAM access (measured slower on the
-//     checkpoint path, which inserts or looks up every changed chunk).
+// Table layout: cap + 1 slots of 32 bytes in one allocation, the 128-bit key then its u64 value, so an
+// insert's value update lands in the sector its key claim already brought in.
 // keys: the 128-bit digest, claimed with one 128-bit atomicCAS (EMPTY = all ones).
 // values: u64 = priority << 45 | checkpoint << 32 | node.  Every insert of the current
 //   checkpoint applies atomicMin to it; within one checkpoint the checkpoint field is the same,
@@ -25,17 +21,13 @@
 #pragma once
 #include "common.cuh"
 
-#ifndef B2D_MAP_SPLIT
-#define B2D_MAP_SPLIT 0
-#endif
-
 namespace b2d {
 
 struct __align__(16) Key128 {
   unsigned long long lo, hi;
 };
-constexpr uint64_t MAP_SLOT_BYTES = B2D_MAP_SPLIT ? sizeof(Key128) + sizeof(unsigned long long) : 32;
-constexpr uint64_t MAP_STRIDE = B2D_MAP_SPLIT ? 1 : 2;   // Key128 units from one slot's key to the next
+constexpr uint64_t MAP_SLOT_BYTES = 32;
+constexpr uint64_t MAP_STRIDE = 2;   // Key128 units from one slot's key to the next
 
 constexpr unsigned long long MAP_EMPTY = ~0ull;
 constexpr uint32_t MAP_TREE_BITS = 13;
@@ -61,15 +53,14 @@ struct MapView {
 __host__ __device__ __forceinline__ MapView map_at(void* mem, uint64_t cap, unsigned long long* size) {
   MapView m;
   m.keys = static_cast<Key128*>(mem);
-  m.vals = B2D_MAP_SPLIT ? reinterpret_cast<unsigned long long*>(m.keys + cap + 1)
-                         : reinterpret_cast<unsigned long long*>(m.keys) + 2;
+  m.vals = reinterpret_cast<unsigned long long*>(m.keys) + 2;
   m.cap = cap;
   m.size = size;
   return m;
 }
 __host__ __device__ __forceinline__ Key128* map_key(const MapView& m, uint64_t i) { return m.keys + i * MAP_STRIDE; }
 __host__ __device__ __forceinline__ unsigned long long* map_val(const MapView& m, uint64_t i) {
-  return m.vals + (B2D_MAP_SPLIT ? i : 4 * i);
+  return m.vals + 4 * i;
 }
 
 struct MapRef {

@@ -729,8 +729,6 @@ static void copy_width(uint64_t dst_al, uint64_t src_al, uint32_t cs, uint32_t& 
   if (per && (per & (per - 1u)) == 0) per_log2 = (uint32_t)__builtin_ctz(per);
 }
 
-int restart_diff_launches(uint32_t n, bool list) { return list ? 2 : 8 + (straddle_query(n).count ? 2 : 0); }
-
 cudaError_t launch_restart_diff(const RestartArgs& args, StraddleInfo* sd, int sm_count, cudaStream_t s) {
   RestartArgs a = args;
   copy_width((uint64_t)(uintptr_t)a.out, (uint64_t)(uintptr_t)(a.diff + a.data_off), a.cs, a.width, a.per,

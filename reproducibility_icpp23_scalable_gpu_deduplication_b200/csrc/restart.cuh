@@ -109,7 +109,7 @@ cudaError_t launch_restart_diff(const RestartArgs& a, StraddleInfo* sd, int sm_c
 // between 45 small launches.  Fills every a.cum itself; the flags of all slots are cleared by the
 // caller.  `sd` has one record per diff.
 cudaError_t launch_restart_diffs(const RestartSet& set, StraddleInfo* sd, int sm_count, cudaStream_t s);
-int restart_diffs_launches(uint32_t n, bool list);
+int restart_diffs_launches(uint32_t n, bool list);   // kernels of one call
 // header_t of a diff (include/utils.hpp:29-37) from its eight words, and the offsets that follow from
 // it; false where it does not fit a diff of `size` bytes
 struct DiffHeader {
@@ -144,7 +144,5 @@ struct RestartHeaders {
 cudaError_t launch_restart_headers(const RestartHeaders& h, uint32_t* out, uint32_t* seen, cudaStream_t s);
 // resolves the chunks owed by the window's diffs and copies them
 cudaError_t launch_restart_walk(const RestartWalk& w, int sm_count, cudaStream_t s);
-// kernel launches made by one launch_restart_diff call (a walk is one launch)
-int restart_diff_launches(uint32_t n, bool list);
 
 }  // namespace b2d

@@ -58,32 +58,13 @@ int scratch_for_current_device(unsigned char** out) {
   return B2D_OK;
 }
 
-struct NaHdr {
-  uint32_t ref_id, chkpt_id;
-  uint64_t datalen;
-  uint32_t cs, F, P, S;
-  uint64_t first_off, count_off, shift_off, data_off;
-};
-
 // header of a device-resident diff, read into host stack memory
-int read_hdr(const void* d_diff, uint64_t size, cudaStream_t s, NaHdr& h) {
+int read_hdr(const void* d_diff, uint64_t size, cudaStream_t s, DiffHeader& h) {
   if (!d_diff || size < 32) return B2D_ERR_FORMAT;
   uint32_t w[8];
   if (cudaMemcpyAsync(w, d_diff, 32, cudaMemcpyDeviceToHost, s) != cudaSuccess) return B2D_ERR_CUDA;
   if (cudaStreamSynchronize(s) != cudaSuccess) return B2D_ERR_CUDA;
-  h.ref_id = w[0];
-  h.chkpt_id = w[1];
-  h.datalen = (uint64_t)w[2] | ((uint64_t)w[3] << 32);
-  h.cs = w[4];
-  h.F = w[5];
-  h.P = w[6];
-  h.S = w[7];
-  h.first_off = 32;
-  h.count_off = h.first_off + 4ull * h.F;
-  h.shift_off = h.count_off + 8ull * h.P;
-  h.data_off = h.shift_off + 8ull * h.S;
-  if (h.data_off > size || h.cs == 0 || h.datalen == 0) return B2D_ERR_FORMAT;
-  return B2D_OK;
+  return parse_header(w, size, h) ? B2D_OK : B2D_ERR_FORMAT;
 }
 
 }  // namespace
@@ -98,7 +79,7 @@ extern "C" int b2d_restart_noalloc(void* d_out, uint64_t len, const void* const*
   unsigned char* base = nullptr;
   int rc = scratch_for_current_device(&base);
   if (rc) return rc;
-  NaHdr h;
+  DiffHeader h;
   if ((rc = read_hdr(d_diffs[chkpt_id], sizes[chkpt_id], s, h))) return rc;
   // diffs[i] must be checkpoint i, whose baseline is not after it (as b2d_restart checks)
   if (h.ref_id > h.chkpt_id || h.chkpt_id != chkpt_id) return B2D_ERR_FORMAT;
@@ -111,7 +92,7 @@ extern "C" int b2d_restart_noalloc(void* d_out, uint64_t len, const void* const*
   {
     uint32_t ref = h.ref_id;
     for (int idx = (int)chkpt_id; idx >= 0 && idx >= (int)ref; idx--) {
-      NaHdr hh;
+      DiffHeader hh;
       if ((rc = read_hdr(d_diffs[idx], sizes[idx], s, hh))) return rc;
       if (idx != (int)chkpt_id) ref = hh.ref_id;
       if (hh.F > NOALLOC_MAX_CHUNKS || hh.S > NOALLOC_MAX_CHUNKS || (uint64_t)hh.chkpt_id + 1 > NOALLOC_MAX_IDS)
@@ -156,7 +137,7 @@ extern "C" int b2d_restart_noalloc(void* d_out, uint64_t len, const void* const*
 
   uint32_t ref = h.ref_id;
   for (int idx = (int)chkpt_id; idx >= 0 && idx >= (int)ref; idx--) {
-    NaHdr hh;
+    DiffHeader hh;
     if ((rc = read_hdr(d_diffs[idx], sizes[idx], s, hh))) return rc;
     if (idx != (int)chkpt_id) ref = hh.ref_id;
     if (hh.F > NOALLOC_MAX_CHUNKS || hh.S > NOALLOC_MAX_CHUNKS || (uint64_t)hh.chkpt_id + 1 > NOALLOC_MAX_IDS)
