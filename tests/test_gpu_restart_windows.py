@@ -61,3 +61,66 @@ def test_memory_of_a_host_restart(cuda):
     assert held[0] < 256 * MIB + (n // 128) * (13 * 5 + 9) + 8 * MIB
     # one diff at a time: the largest of them and one slot
     assert held[1] < len(max(diffs, key=len)) + (n // 128) * (13 + 9) + 8 * MIB
+
+
+def plain_chain(nbytes, cs, count):
+    """states that only rewrite chunks (no moves): restarts are whole for any chunk count"""
+    import torch
+
+    rng = np.random.default_rng(cs)
+    x = rng.integers(0, 256, nbytes, dtype=np.uint8)
+    states, diffs = [], []
+    with ListDeduplicator(cs) as g:
+        for k in range(count):
+            x = x.copy()
+            x[k * 5000 * cs:(k * 5000 + 3000) * cs] = rng.integers(0, 256, 3000 * cs, dtype=np.uint8)
+            states.append(x)
+            diffs.append(np.frombuffer(g.checkpoint(torch.from_numpy(x).cuda(), k == 0), np.uint8))
+    return states, diffs
+
+
+@pytest.mark.parametrize("kind", ["pageable", "page-locked", "mixed"])
+@pytest.mark.parametrize("stream", [None, 1, 2])
+def test_uploads(cuda, kind, stream):
+    """host diffs of several upload pieces, in pageable and page-locked memory, on the handle's own, the
+    legacy default and the per-thread default stream"""
+    import ctypes
+
+    import torch
+
+    from reproducibility_icpp23_scalable_gpu_deduplication_b200._lib import lib
+
+    states, diffs = plain_chain(40 * MIB + 77, 128, 4)
+    keep = []
+    for k, d in enumerate(diffs):
+        if kind == "page-locked" or (kind == "mixed" and k % 2):
+            t = torch.empty(d.size, dtype=torch.uint8, pin_memory=True)
+            t.copy_(torch.from_numpy(d.copy()))
+            keep.append(t)
+            diffs[k] = t.numpy()
+    ptrs = (ctypes.c_void_p * 4)(*[d.ctypes.data for d in diffs])
+    sizes = (ctypes.c_uint64 * 4)(*[d.size for d in diffs])
+    with ListDeduplicator(128) as g:
+        assert lib().b2d_set_stream(g._h, ctypes.c_void_p(stream)) == 0
+        for last in (3, 0, 2):
+            out = torch.zeros(states[0].size, dtype=torch.uint8, device="cuda")
+            torch.cuda.synchronize()
+            assert lib().b2d_restart(g._h, ctypes.c_void_p(out.data_ptr()), out.numel(), ptrs, sizes, 4, last, None) == 0
+            assert np.array_equal(out.cpu().numpy(), states[last]), last
+
+
+@pytest.mark.parametrize("cs", [64, 100, 128, 256])
+@pytest.mark.parametrize("offset", [0, 1, 4, 8])
+def test_output_alignments(cuda, cs, offset):
+    """outputs of 2^15 chunks and more that do not start on 16 bytes"""
+    import torch
+
+    nbytes = cs * 33333 - 9
+    states, diffs = plain_chain(nbytes, cs, 4)
+    dev = [to_dev(d) for d in diffs]
+    with ListDeduplicator(cs) as g:
+        for run, chain in ((g.restart, diffs), (g.restart_device, dev)):
+            mem = torch.full((nbytes + 64,), 7, dtype=torch.uint8, device="cuda")
+            run(mem[offset:offset + nbytes], chain, 3)
+            assert np.array_equal(mem[offset:offset + nbytes].cpu().numpy(), states[3])
+            assert bool((mem[:offset] == 7).all()) and bool((mem[offset + nbytes:] == 7).all())
