@@ -476,26 +476,38 @@ __device__ __forceinline__ void shift_write_range(const DiffArgs& a, uint32_t ra
   }
 }
 // ---------------------------------------------------------------- data gather
+// A 16-byte unit of the data section whose source reaches past the buffer's end (zeros, :643-645), where
+// chunks and buffer are 16-byte aligned: a unit then lies within one region.  One byte after another: a
+// kernel has the registers of what it calls, 124 with the routine below.
+__device__ __noinline__ void gather_end_unit(const uint8_t* data, uint64_t len, uint64_t s, uint4* dst) {
+  uint64_t lo = 0, hi = 0;
+#pragma unroll 1
+  for (uint32_t b = 0; b < 16u && s + b < len; b++) {
+    const uint64_t v = (uint64_t)data[s + b] << (8u * (b & 7u));
+    if (b < 8u) lo |= v;
+    else hi |= v;
+  }
+  *dst = make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
+}
 // a 16-byte unit of the data section that a region ends in, or whose source reaches past the
-// buffer's end (zeros, :643-645): byte by byte, region r holding its first byte.  Where chunks and
-// buffer are 16-byte aligned only the units at the buffer's end are, and one byte after another:
-// a kernel has the registers of what it calls, and with 16 loads side by side here it had 124.
-template <bool ALIGNED>
-__device__ __noinline__ void gather_unit_bytes(const DiffArgs* args, uint64_t unit, uint32_t r) {
-  const DiffArgs& a = *args;
-  const uint32_t F = a.meta->F;
-  const uint64_t total = a.meta->T * a.cs;
-  uint8_t* dst = a.diff + a.meta->data_off;
+// buffer's end: byte by byte, region r holding its first byte
+struct GatherBytes {
+  const uint8_t* data;
+  uint64_t len, cs, total;   // buffer length, chunk size, bytes of the data section
+  const uint32_t *region_off, *first_list;
+  uint32_t F, n, N, D;
+};
+__device__ __noinline__ void gather_unit_bytes(GatherBytes a, uint8_t* dst, uint64_t unit, uint32_t r) {
   const uint64_t pos0 = 16ull * unit;
-  auto start_of = [&](uint32_t i) { return i < F ? (uint64_t)a.region_off[i] * a.cs : ~0ull; };
+  auto start_of = [&](uint32_t i) { return i < a.F ? (uint64_t)a.region_off[i] * a.cs : ~0ull; };
   // source byte minus data-section byte, within region r
   auto shift_of = [&](uint32_t i) {
-    return (uint64_t)(node_span(a.first_list[i], a.N, a.D).first - (a.n - 1u)) * a.cs - start_of(i);
+    return (node_span(a.first_list[i], a.N, a.D).first - (a.n - 1u)) * a.cs - start_of(i);
   };
   uint64_t shift = shift_of(r), next = start_of(r + 1u);
   uint8_t t[16];
   // the bytes' loads do not wait for one another (one at a time, a unit took 16 memory round trips)
-#pragma unroll (ALIGNED ? 1 : 16)
+#pragma unroll
   for (uint32_t b = 0; b < 16u; b++) {
     const uint64_t pos = pos0 + b;
     while (pos >= next) {
@@ -504,16 +516,16 @@ __device__ __noinline__ void gather_unit_bytes(const DiffArgs* args, uint64_t un
       next = start_of(r + 1u);
     }
     const uint64_t s = pos + shift;
-    t[b] = pos < total && s < a.len ? __ldg(a.data + s) : 0u;
+    t[b] = pos < a.total && s < a.len ? __ldg(a.data + s) : 0u;
   }
-  if (pos0 + 16u <= total) {
+  if (pos0 + 16u <= a.total) {
     uint4 v;
     memcpy(&v, t, 16);
     *reinterpret_cast<uint4*>(dst + pos0) = v;
   } else {
 #pragma unroll
     for (uint32_t b = 0; b < 16u; b++)
-      if (pos0 + b < total) dst[pos0 + b] = t[b];
+      if (pos0 + b < a.total) dst[pos0 + b] = t[b];
   }
 }
 
@@ -628,8 +640,11 @@ __device__ __forceinline__ void gather_body(const DiffArgs& a, uint32_t bid, uin
         if (pos + 16u <= end && s < a.len && a.len - s >= 16u) {
           st |= 1u << i;
           v[i] = ALIGNED ? __ldg(reinterpret_cast<const uint4*>(a.data + s)) : load_unit(a.data, a.len, s);
+        } else if (ALIGNED) {
+          gather_end_unit(a.data, a.len, s, dst + u + g);
         } else {
-          gather_unit_bytes<ALIGNED>(&a, u + g, r + j);
+          gather_unit_bytes(GatherBytes{a.data, a.len, a.cs, total, a.region_off, a.first_list, F, a.n, a.N, a.D},
+                            dst_base, u + g, r + j);
         }
       }
 #pragma unroll
@@ -667,10 +682,9 @@ __device__ __forceinline__ void diff_emit_body(const DiffArgs& a, uint32_t bid, 
   if (warp < warps && range < ranges) shift_write_range(a, range, ranges, bucket_count(a, bcap), run + warp * bcap);
 }
 template <bool ALIGNED>
-__global__ void __launch_bounds__(EMIT_THREADS, 2) diff_emit_kernel(const __grid_constant__ DiffArgs a0, uint32_t bcap,
-                                                                   uint32_t ranges) {
+__global__ void __launch_bounds__(EMIT_THREADS, 2) diff_emit_kernel(DiffArgs a0, uint32_t bcap, uint32_t ranges) {
   griddep_enter();
-  diff_emit_body<ALIGNED>(a0, blockIdx.x, gridDim.x, bcap, ranges);
+  diff_emit_body<ALIGNED>(with_round(a0), blockIdx.x, gridDim.x, bcap, ranges);
   // the last CTA hands the checkpoint's state to the host: a copy enqueued behind this kernel
   // took 10 us of a small checkpoint
   if (a0.state_host == nullptr) return;
