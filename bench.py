@@ -760,7 +760,7 @@ def main():
     alg_leaf = nbytes + 32 * n_chunks              # read the buffer, read + write a digest per chunk
     achieved = alg_leaf / (leaf_ms * 1e-3) / GB if leaf_ms > 0 else 0.0
     tb = leaf_traffic(cs)
-    roofline = {"bound": "hbm", "kernel": f"leaf_tma_kernel (chunk {cs} B)" if path else "leaf_any_kernel",
+    roofline = {"bound": "hbm", "kernel": f"leaf_tma_kernel (chunk {cs} B)" if path else "leaf_any_kernel or leaf_short_kernel",
                 "achieved": round(achieved, 1), "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": round(tb * nbytes) if tb else None,
                 "algorithmic_bytes": alg_leaf, "launch_ms": round(leaf_ms, 4),

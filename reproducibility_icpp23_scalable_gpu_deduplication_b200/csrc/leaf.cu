@@ -9,7 +9,7 @@
 //     ring; eight consumer warps hash one chunk per lane.  Used when the chunk size is a
 //     multiple of 16 bytes (MD5: 64) and the buffer is 16-byte aligned.
 //   * leaf_any_kernel: any chunk size or alignment, one chunk per lane streamed through shared
-//     memory in aligned pieces.
+//     memory in aligned pieces; leaf_short_kernel: the same for short chunks, read directly.
 #include <cuda.h>
 #include "copy.cuh"
 #include "dedup_kernels.cuh"
@@ -448,6 +448,30 @@ __global__ void __launch_bounds__(ANY_WARPS * 32, 2) leaf_any_kernel(LeafArgs a0
   }
 }
 
+// Short chunks on the same terms: one thread per chunk, read where it lies.  A warp's 32 chunks are a few
+// kilobytes side by side, which the L1 serves, and the staging above costs a chunk three quarters of a
+// segment at least.  launch_leaves has the line between the two.
+template <int KIND>
+__global__ void __launch_bounds__(256) leaf_short_kernel(LeafArgs a0) {
+  griddep_enter();
+  const LeafArgs a = with_round(a0);
+  const uint64_t groups = ((uint64_t)a.n + 31u) / 32u, warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t g = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; g < groups; g += warps) {
+    const uint64_t c = 32u * g + (threadIdx.x & 31u);
+    const bool valid = c < a.n;
+    const uint64_t off = c * a.cs;
+    Digest old, d;
+    old.w[0] = old.w[1] = old.w[2] = old.w[3] = 0u;
+    d = old;
+    if (valid) {
+      old = prior_digest(a, c);
+      d = hash_bytes(KIND, a.data + off, c == a.n - 1u ? a.len - off : a.cs);
+    }
+    if (a.bulk) bulk_finish(a, (uint32_t)c, valid, d);
+    else if (valid) leaf_finish(a, (uint32_t)c, d, old);
+  }
+}
+
 // fold the U-byte segment of row `row` of a staged tile into a lane's running digest state
 template <int U, int KIND>
 __device__ __forceinline__ void hash_segment(const uint8_t* stage, uint32_t row, Murmur3& mm, uint32_t md[4],
@@ -853,6 +877,17 @@ int launch_leaves(const LeafArgs& a, int sm_count, const LeafTuning& tune, cudaS
       }
       return e == cudaSuccess ? 1 : -1;
     }
+  }
+  // Chunks that are read faster where they lie than through shared memory.  Hashing of 2^21 chunks (64 MiB
+  // at most), directly and staged, us: Murmur3 with chunks and buffer 4-byte aligned, 4 B 25 and 63, 32 B
+  // 33 and 66, 64 B 39 and 40, 100 B 25 and 30, 120 B 29 and 27, 200 B 34 and 28; otherwise, byte by byte,
+  // 5 B 26 and 61, 33 B 48 and 67, 44 B 43 and 53, 56 B 46 and 43, 64 B 132 and 39; MD5, always byte by
+  // byte, 4 B 74 and 90, 33 B 74 and 94, 60 B 62 and 69, 63 B 65 and 65, 72 B 70 and 58.
+  const bool words = ((reinterpret_cast<uintptr_t>(a.data) | a.cs) & 3u) == 0;
+  if (a.cs < (a.kind == HASH_MD5 ? 64u : words ? 112u : 48u)) {
+    auto kern = a.kind == HASH_MD5 ? leaf_short_kernel<HASH_MD5> : leaf_short_kernel<HASH_MURMUR3>;
+    const uint64_t want = ceil_div_u64(a.n, 256u), cap = (uint64_t)sm_count * 16u;
+    return launch_dependent(kern, (uint32_t)(want < cap ? want : cap), 256, 0, stream, a) == cudaSuccess ? 0 : -1;
   }
   constexpr size_t smem = ANY_WARPS * ANY_STAGES * ANY_STAGE_BYTES;
   auto kern = a.kind == HASH_MD5 ? leaf_any_kernel<HASH_MD5> : leaf_any_kernel<HASH_MURMUR3>;
