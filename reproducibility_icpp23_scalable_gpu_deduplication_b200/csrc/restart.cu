@@ -571,8 +571,8 @@ __global__ void __launch_bounds__(R_THREADS, B2D_RESTART_MINB) r_walk_kernel(con
 // register: a restart of 1 GiB from five device diffs takes 640 us, through registers, four pieces a
 // lane at a time, 668 us.  A source is fetched from the 16-byte boundary before it on, one piece
 // more than the chunk has, and shifted into place when it is written, so sources of any alignment
-// move in whole pieces.  For 16-byte aligned outputs and chunk sizes that are multiples of 16 up to
-// STAGE_CHUNK (larger ones have enough in flight as it is).
+// move in whole pieces.  For chunk sizes that are multiples of 16 up to STAGE_CHUNK (larger ones have
+// enough in flight as it is); launch_restart_walk says when.
 constexpr uint32_t WALK_WARPS = 4;
 constexpr uint32_t STAGE_CHUNK = 128;
 constexpr uint32_t STAGE_BYTES = 32u * (STAGE_CHUNK + 16u);
@@ -644,6 +644,26 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, 6) r_walk_staged_kernel(const
 __device__ __forceinline__ void cum_body(const RestartArgs& a) {
   __shared__ uint32_t sh[33];
   unsigned long long* cum = const_cast<unsigned long long*>(a.cum);
+  if (a.P <= 32u && a.ncum <= 32u) {   // one warp holds the rows and the counts
+    const uint32_t lane = threadIdx.x;
+    if (lane >= 32u) return;
+    const bool row = lane < a.P;
+    const uint32_t ck = row ? rd_u32(a.diff + a.count_off + 8ull * lane) : 0u;
+    const uint32_t n = row ? rd_u32(a.diff + a.count_off + 8ull * lane + 4) : 0u;
+    if (row && ck >= a.ncum) set_error(a.st, DERR_RESTART_RANGE, 5);
+    unsigned long long v = 0;
+    for (uint32_t i = 0; i < a.P; i++) {
+      const uint32_t t = __shfl_sync(R_FULL, ck, i), c = __shfl_sync(R_FULL, n, i);
+      if (t == lane) v = c;
+    }
+#pragma unroll
+    for (uint32_t d = 1; d < 32u; d <<= 1) {
+      const unsigned long long below = __shfl_up_sync(R_FULL, v, d);
+      if (lane >= d) v += below;
+    }
+    if (lane < a.ncum) cum[lane] = v;
+    return;
+  }
   for (uint32_t t = threadIdx.x; t < a.ncum; t += blockDim.x) cum[t] = 0;
   auto id = [&](uint32_t i) { return rd_u32(a.diff + a.count_off + 8ull * i); };
   auto cnt = [&](uint32_t i) { return rd_u32(a.diff + a.count_off + 8ull * i + 4); };
@@ -811,7 +831,16 @@ cudaError_t launch_restart_walk(const RestartWalk& walk, int sm_count, cudaStrea
   uint64_t src_al = 0;
   for (uint32_t k = 0; k < w.count; k++) src_al |= (uint64_t)(uintptr_t)w.data[k];
   copy_width((uint64_t)(uintptr_t)w.out, src_al, w.cs, w.width, w.per, w.per_log2);
-  if (w.width == 16u && w.cs <= STAGE_CHUNK) {
+  // Staged where most chunks are copied and there are groups enough to overlap, for chunks of more than
+  // 64 bytes; the walk through registers costs a group less that has little or nothing to copy.  Through
+  // registers and staged, us.  512 MiB from a baseline and four increments: chunks of 16 B 859 and 992,
+  // 64 B 313 and 322, 80 B 310 and 295, 128 B 244 and 228; 64 MiB: 64 B 44.7 and 45.1, 128 B 37 and 33;
+  // 4 MiB: 128 B 6.4 and 8.8.  By the share of 2^23 chunks of 128 B that one diff holds: 1 % 85 and 181,
+  // 20 % 188 and 216 (scattered 248 and 270), 40 % 275 and 243 (310 and 300), 80 % 413 and 349.
+  uint64_t data = 0;
+  for (uint32_t k = 0; k < w.count; k++) data += w.data_len[k];
+  if (w.width == 16u && w.cs > 64u && w.cs <= STAGE_CHUNK && w.out_len >= (32ull << 20) &&
+      data >= w.out_len / 8u * 3u) {
     constexpr size_t smem = WALK_WARPS * 2u * STAGE_BYTES;
     const cudaError_t e =
         cudaFuncSetAttribute(r_walk_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -124,3 +124,29 @@ def test_output_alignments(cuda, cs, offset):
             run(mem[offset:offset + nbytes], chain, 3)
             assert np.array_equal(mem[offset:offset + nbytes].cpu().numpy(), states[3])
             assert bool((mem[:offset] == 7).all()) and bool((mem[offset + nbytes:] == 7).all())
+
+
+@pytest.mark.parametrize("cs", [64, 80, 96, 112, 128, 144])
+@pytest.mark.parametrize("nbytes", [32 * MIB - 5, 33 * MIB + 5])
+def test_large_walks(cuda, cs, nbytes):
+    """outputs on both sides of the size and the chunk sizes from which copies are staged, from diffs at
+    several alignments, in one window and in several"""
+    import torch
+
+    states, diffs = plain_chain(nbytes, cs, 4)
+    with ListDeduplicator(cs) as g:
+        for window in (0, 1):
+            g.set_param("restart_window", window)
+            for shift in (0, 1, 4, 8):
+                mems = [torch.zeros(d.size + 16, dtype=torch.uint8, device="cuda") for d in diffs]
+                dev = []
+                for m, d in zip(mems, diffs):
+                    v = m[shift:shift + d.size]
+                    v.copy_(torch.from_numpy(d.copy()))
+                    dev.append(v)
+                out = torch.zeros(nbytes, dtype=torch.uint8, device="cuda")
+                g.restart_device(out, dev, 3)
+                assert np.array_equal(out.cpu().numpy(), states[3]), (window, shift)
+            out.zero_()
+            g.restart(out, diffs, 3)
+            assert np.array_equal(out.cpu().numpy(), states[3]), window
