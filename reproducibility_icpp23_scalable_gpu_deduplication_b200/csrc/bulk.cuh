@@ -46,7 +46,9 @@ struct BulkPlan {
   uint64_t key1, key2, id1, id2;
   uint64_t zeroed_bytes, start, over_count, lost, alloc, alloc1, tile_beg;
 };
-// false: this tree and table are not built in bulk
+// false: this tree and table are not built in bulk: too few chunks, more than BULK_MAX_RANGES table
+// ranges, or entries that do not fit the diff buffer (40 bytes per chunk of a tree in one scatter pass,
+// 80 in two, of the buffer's 16 + chunk size: from 24 and from 64 byte chunks on; lists half of that)
 bool bulk_plan(uint32_t n, uint64_t cap, int list, uint64_t diff_bytes, BulkPlan& p);
 cudaError_t launch_bulk(const BulkArgs& a, int sm_count, cudaStream_t stream, uint32_t* launches);
 
