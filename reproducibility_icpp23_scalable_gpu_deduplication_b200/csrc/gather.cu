@@ -536,7 +536,7 @@ __device__ __noinline__ void gather_unit_bytes(GatherBytes a, uint8_t* dst, uint
 // are held one per lane, and each unit finds its region among them by a five-step shuffle search,
 // so no load waits on another.  Where one region covers a whole step of the warp the search is
 // left out and the warp streams to the region's end: a 4 GiB baseline, one region, was bound by
-// the search's instructions (2.40 ms, now 1.41 ms; a plain copy of the same bytes takes 1.35 ms).
+// the search's instructions (2.40 ms, now 1.36 ms; a plain copy of the same bytes takes 1.35 ms).
 // Chunk sizes or buffers that are not 16-byte aligned take the same path with shifted loads
 // (load_unit): with one thread per chunk and byte copies, 1000 B chunks of a 150 MB buffer at an
 // 8-byte offset took 331 us per increment of 5 % and the whole series 2.40 ms, now 0.94 ms.
